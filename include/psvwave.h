@@ -259,16 +259,20 @@ const char *psv_step_kernel_name(const psv_model *m, int k);
  * ping-pong buffers; FP32 only), PSV_VARIANT_TWO_KERNEL (separate stress and
  * velocity launches, as the reference's two loop nests; the only FP64
  * variant), PSV_VARIANT_FUSED_TMA (the fused step with TMA tile loads, one
- * launch per step; FP32, the default) or PSV_VARIANT_FUSED_TMA_PERSISTENT
- * (the same step, every time step of a simulation in one persistent launch
- * whose tiles start a step as soon as their neighbours have finished the
- * previous one). Results of the FP32 variants agree to FP32 rounding. No
+ * launch per step; FP32), PSV_VARIANT_FUSED_TMA_PERSISTENT (the same step,
+ * every time step of a simulation in one persistent launch whose tiles start
+ * a step as soon as their neighbours have finished the previous one; the
+ * default on large grids) or PSV_VARIANT_FUSED_CLUSTER (every time step in
+ * one launch that keeps the grid on chip; the default on small grids). Until
+ * a variant or tile shape is set, larger grids that fit on the chip run
+ * resident as well. Results of the FP32 variants agree to FP32 rounding. No
  * counterpart in the reference. */
 enum psv_variant {
   PSV_VARIANT_FUSED = 0,
   PSV_VARIANT_TWO_KERNEL = 1,
   PSV_VARIANT_FUSED_TMA = 2,
-  PSV_VARIANT_FUSED_TMA_PERSISTENT = 3
+  PSV_VARIANT_FUSED_TMA_PERSISTENT = 3,
+  PSV_VARIANT_FUSED_CLUSTER = 4
 };
 int psv_set_kernel_variant(psv_model *m, int variant);
 int psv_get_kernel_variant(const psv_model *m, int *variant);
@@ -355,11 +359,11 @@ int psv_batch_set_parameter_fields_device(psv_batch *b, const double *fields,
  * previous one. Results are identical. */
 int psv_batch_set_persistent(psv_batch *b, int persistent);
 int psv_batch_get_persistent(const psv_batch *b, int *persistent);
-/* Cluster-resident scheme: cluster != 0 runs every member in its own
- * thread-block cluster that keeps the member's whole grid in shared memory
- * for every time step, all members in one launch (the batched form of the
- * model variant fused_cluster, whose results it equals bit for bit).
- * PSV_ERR_INVALID_ARGUMENT when a member does not fit a cluster; *fits
+/* Resident scheme: cluster != 0 keeps every member's whole grid on chip for
+ * every time step, each member on its own team of CTAs (one thread-block
+ * cluster where that holds it); the batched form of the model variant
+ * fused_cluster, whose results it equals bit for bit.
+ * PSV_ERR_INVALID_ARGUMENT when a member does not fit on the chip; *fits
  * (psv_batch_cluster_fits) tells beforehand. psv_batch_set_persistent
  * switches it off; psv_batch_autotune also times it when the members fit. */
 int psv_batch_set_cluster(psv_batch *b, int cluster);

@@ -1,8 +1,8 @@
 """Batched forward simulation: shots of many fdModels, of uneven grid sizes,
 advanced together (C ABI psv_batch_*): one TMA-step launch per time step
 with the whole time loop replayed as one CUDA graph (the default), every
-step in one persistent launch, or every member in its own cluster-resident
-launch; the autotuner picks. Media updates and misfits of many members go
+step in one persistent launch, or every member's grid resident on chip;
+the autotuner picks. Media updates and misfits of many members go
 through one call each."""
 import ctypes
 
@@ -62,11 +62,10 @@ class Batch:
 
     @cluster.setter
     def cluster(self, on):
-        """Cluster-resident scheme (True): every member in its own
-        thread-block cluster holding its whole grid in shared memory for
-        every step, all members in one launch; results equal each model's
-        own `fused_cluster` run bit for bit. ValueError when a member does
-        not fit (`cluster_fits`). Setting `persistent` switches it off."""
+        """Resident scheme (True): every member's grid held on chip for every
+        step by its own team of CTAs (one thread-block cluster where that
+        holds it); results equal each model's own `fused_cluster` run bit
+        for bit. ValueError when a member does not fit (`cluster_fits`). Setting `persistent` switches it off."""
         _capi.check(self._lib.psv_batch_set_cluster(self._h, int(bool(on))))
 
     @property
@@ -142,7 +141,7 @@ class Batch:
 
     def autotune(self, n_steps=50):
         """Times every tile shape with both tile launch schemes, and the
-        cluster-resident scheme when the members fit, on n_steps steps of
+        resident scheme when the members fit, on n_steps steps of
         the active members and keeps the fastest; returns the tile shape
         (the scheme is `cluster`, else `persistent`)."""
         v = ctypes.c_int()

@@ -2,10 +2,10 @@
 #include "psv_batch.hpp"
 
 #include <algorithm>
+#include <tuple>
 #include <limits>
 
 #include "../../include/psvwave.h"
-#include "psv_cluster.hpp"
 
 namespace psv {
 
@@ -54,34 +54,176 @@ void Batch::add(Model *m, int shot) {
   members_.emplace_back(m, shot);
   active_h_.push_back(1);
   built_ = false;
-  cluster_nc_ = -1;
+  fits_ = -1;
+  grids_.clear();
+  packed_.clear();
   cluster_ = false;
   clear_graphs();
 }
 
-bool Batch::cluster_fits() {
-  if (cluster_nc_ < 0) {
-    std::vector<int> nx, nz, np;
-    for (const auto &mb : members_) {
-      nx.push_back(mb.first->geometry().nx);
-      nz.push_back(mb.first->geometry().nz);
-      np.push_back(mb.first->config().np_boundary);
-    }
-    int prev = 0;
+namespace {
+struct OnDevice {
+  int prev = 0;
+  explicit OnDevice(int device) {
     cudaGetDevice(&prev);
-    cuda_check(cudaSetDevice(device_), "cudaSetDevice");
-    cluster_nc_ = cluster::plan_batch(nx.data(), nz.data(), np.data(), static_cast<int>(nx.size()),
-                                      &cluster_smem_);
-    cudaSetDevice(prev);
+    cuda_check(cudaSetDevice(device), "cudaSetDevice");
   }
-  return cluster_nc_ > 0;
+  ~OnDevice() { cudaSetDevice(prev); }
+};
+
+// A member's plan under a layout; no CTAs: it does not fit.
+resident::Plan member_plan(const resident::Grid &g, int nc, int per_sm) {
+  if (nc > 0) {
+    const resident::Plan p = resident::plan_cluster(g, nc);
+    if (p.ctas() > 0) return p;
+  }
+  return resident::plan_smallest(g, per_sm);
+}
+}  // namespace
+
+bool Batch::layout_holds(const Layout &l) {
+  if (grids_.empty())
+    for (const auto &mb : members_) grids_.push_back(mb.first->resident_grid());
+  for (const auto &g : grids_)
+    if (member_plan(g, l.nc, l.per_sm).ctas() == 0) return false;
+  return true;
+}
+
+bool Batch::cluster_fits() {
+  if (fits_ < 0) {
+    OnDevice on(device_);
+    // Fewest CTAs that hold every member: clusters, else mailbox teams.
+    fits_ = 0;
+    std::vector<Layout> tries;
+    for (int nc : {4, 5, 6, 8, 9, 10, 12, 16}) {
+      bool all = true;
+      if (grids_.empty())
+        for (const auto &mb : members_) grids_.push_back(mb.first->resident_grid());
+      for (const auto &g : grids_) all = all && resident::plan_cluster(g, nc).ctas() > 0;
+      if (all) {
+        tries.push_back(Layout{nc, 2});
+        break;
+      }
+    }
+    tries.push_back(Layout{0, 2});
+    tries.push_back(Layout{0, 1});
+    for (const Layout &l : tries)
+      if (!members_.empty() && layout_holds(l)) {
+        layout_ = l;
+        fits_ = 1;
+        break;
+      }
+  }
+  return fits_ > 0;
+}
+
+// The launches of the active members: cluster members by kernel instance,
+// mailbox teams first-fit by decreasing size into cooperative launches, whose
+// spare CTAs then go to the team with the tallest tiles.
+void Batch::pack() {
+  if (packed_ == active_h_ && !launches_.empty()) return;
+  clear_graphs();
+  launches_.clear();
+  std::vector<resident::Member> members;
+  std::vector<int> ctas;
+  struct Team {
+    int k;
+    resident::Plan p;
+  };
+  std::vector<Team> clusters, teams;
+  for (int k = 0; k < size(); ++k) {
+    if (!active_h_[k]) continue;
+    const resident::Plan p = member_plan(grids_[k], layout_.nc, layout_.per_sm);
+    (p.cluster ? clusters : teams).push_back(Team{k, p});
+  }
+  auto emit = [&](const std::vector<Team> &set, bool cluster) {
+    resident::Launch l;
+    l.first_member = static_cast<int>(members.size());
+    l.first_cta = static_cast<int>(ctas.size());
+    l.rows = set[0].p.rows;
+    l.stride = set[0].p.stride;
+    for (size_t i = 0; i < set.size(); ++i) {
+      const resident::Plan &p = set[i].p;
+      members.push_back(resident::Member{set[i].k, l.ctas, p.tiles_x, p.tiles_z, p.groups, p.n_rec,
+                                         p.n_inj});
+      ctas.insert(ctas.end(), p.ctas(), static_cast<int>(i));
+      l.ctas += p.ctas();
+      l.rows = std::max(l.rows, p.rows);
+      l.threads = std::max(l.threads, p.threads);
+      l.smem = std::max(l.smem, p.smem);
+      if (cluster) l.team = p.ctas();
+    }
+    launches_.push_back(l);
+  };
+  std::stable_sort(clusters.begin(), clusters.end(), [](const Team &a, const Team &b) {
+    return std::make_tuple(a.p.ctas(), a.p.rows, a.p.stride) <
+           std::make_tuple(b.p.ctas(), b.p.rows, b.p.stride);
+  });
+  for (size_t i = 0; i < clusters.size();) {
+    size_t j = i;
+    while (j < clusters.size() && clusters[j].p.ctas() == clusters[i].p.ctas() &&
+           clusters[j].p.rows == clusters[i].p.rows && clusters[j].p.stride == clusters[i].p.stride)
+      ++j;
+    emit(std::vector<Team>(clusters.begin() + i, clusters.begin() + j), true);
+    i = j;
+  }
+  std::stable_sort(teams.begin(), teams.end(),
+                   [](const Team &a, const Team &b) { return a.p.ctas() > b.p.ctas(); });
+  const int slots = resident::resident_slots(layout_.per_sm);
+  std::vector<std::vector<Team>> bins;
+  std::vector<int> used;
+  for (const Team &t : teams) {
+    size_t b = 0;
+    while (b < bins.size() && used[b] + t.p.ctas() > slots) ++b;
+    if (b == bins.size()) {
+      bins.emplace_back();
+      used.push_back(0);
+    }
+    bins[b].push_back(t);
+    used[b] += t.p.ctas();
+  }
+  for (size_t b = 0; b < bins.size(); ++b) {
+    for (;;) {
+      Team *tall = nullptr;
+      int rows = 0;
+      for (Team &t : bins[b]) {
+        const int r = (grids_[t.k].nx + t.p.tiles_x - 1) / t.p.tiles_x;
+        if (r > rows) {
+          rows = r;
+          tall = &t;
+        }
+      }
+      if (!tall || used[b] + tall->p.tiles_z > slots ||
+          !resident::set_tiles_x(tall->p, grids_[tall->k], tall->p.tiles_x + 1, layout_.per_sm))
+        break;
+      used[b] += tall->p.tiles_z;
+    }
+    emit(bins[b], false);
+  }
+  size_t mail = 0;
+  for (const auto &l : launches_) mail = std::max(mail, resident::launch_mailbox_bytes(l));
+  if (mail_.bytes() < mail) mail_.allocate(mail);
+  if (res_members_.bytes() < members.size() * sizeof(members[0]))
+    res_members_.allocate(members.size() * sizeof(members[0]));
+  if (res_ctas_.bytes() < ctas.size() * sizeof(int)) res_ctas_.allocate(ctas.size() * sizeof(int));
+  if (!members.empty()) {
+    cuda_check(cudaMemcpyAsync(res_members_.get(), members.data(),
+                               members.size() * sizeof(members[0]), cudaMemcpyHostToDevice, stream_),
+               "upload batch teams");
+    cuda_check(cudaMemcpyAsync(res_ctas_.get(), ctas.data(), ctas.size() * sizeof(int),
+                               cudaMemcpyHostToDevice, stream_),
+               "upload batch teams");
+    cuda_check(cudaStreamSynchronize(stream_), "upload batch teams");
+  }
+  packed_ = active_h_;
 }
 
 void Batch::set_cluster(bool on) {
   if (on && !cluster_fits())
-    throw Error(PSV_ERR_INVALID_ARGUMENT, "a batch member does not fit a thread-block cluster");
+    throw Error(PSV_ERR_INVALID_ARGUMENT, "a batch member does not fit on the chip");
   if (on == cluster_) return;
   cluster_ = on;
+  packed_.clear();
   clear_graphs();
 }
 
@@ -126,10 +268,7 @@ void Batch::build() {
     d.nt = c.nt;
     d.nr = c.nr;
     d.si = c.snapshot_interval;
-    d.dt = static_cast<float>(c.dt);
-    d.idx = static_cast<float>(1.0 / c.dx);
-    d.idz = static_cast<float>(1.0 / c.dz);
-    d.dt_d = c.dt;
+    d.set_steps(c.dt, c.dx, c.dz);
     d.lm = m.lm_.as<float>();
     d.mu = m.mu_.as<float>();
     d.b = m.b_.as<float>();
@@ -194,6 +333,8 @@ void Batch::build() {
                           cudaMemcpyHostToDevice),
                "upload batch tiles");
   }
+  // (The uploads ran on the legacy stream, for which stream_ does not wait.)
+  cuda_check(cudaStreamSynchronize(cudaStreamLegacy), "batch build");
   built_ = true;
 }
 
@@ -243,6 +384,7 @@ void Batch::forward(bool store, int n_steps) {
   // Members' own streams may still be updating their media.
   for (auto &mb : members_) mb.first->synchronize();
   if (!built_) build();
+  if (cluster_) pack();
   // The flags live in device memory that the (captured) step launches read.
   cuda_check(cudaMemcpyAsync(active_.get(), active_h_.data(), active_h_.size() * sizeof(int),
                              cudaMemcpyHostToDevice, stream_),
@@ -250,11 +392,15 @@ void Batch::forward(bool store, int n_steps) {
   const int steps = (n_steps <= 0 || n_steps > nt_) ? nt_ : n_steps;
   const int cfg = tile_cfg_;
   auto enqueue = [&]() {
-    cuda_check(cudaMemsetAsync(arena_.get(), 0, arena_.bytes(), stream_), "batch zero");
+    if (!cluster_)
+      cuda_check(cudaMemsetAsync(arena_.get(), 0, arena_.bytes(), stream_), "batch zero");
     if (cluster_) {
-      cuda_check(cluster::steps_batch(descs_d_.as<tma::SimDesc>(), active_.as<int>(), size(),
-                                      cluster_nc_, cluster_smem_, steps, store, stream_),
-                 "batch cluster steps");
+      for (const auto &l : launches_)
+        cuda_check(resident::steps_batch(descs_d_.as<tma::SimDesc>(),
+                                         res_members_.as<resident::Member>(), res_ctas_.as<int>(),
+                                         l, steps, store, mail_.get(), err_flag_.as<int>(),
+                                         stream_),
+                   "batch resident steps");
     } else if (persistent_) {
       cuda_check(cudaMemsetAsync(sched_.get(), 0, sched_.bytes(), stream_), "batch schedule");
       cuda_check(tma::steps_persistent_batch(descs_d_.as<tma::SimDesc>(),
@@ -411,18 +557,42 @@ int Batch::autotune(int n_steps) {
       }
     }
   }
+  // The resident scheme, in clusters and in mailbox teams with one or two
+  // CTAs per SM (few launches: timed on the second run).
   bool best_cluster = false;
+  Layout best_layout;
   if (cluster_fits()) {
-    set_cluster(true);
-    forward(false, n_steps);
-    forward(false, n_steps);
-    cudaEventRecord(a, stream_);
-    forward(false, n_steps);
-    cudaEventRecord(b, stream_);
-    cudaEventSynchronize(b);
-    float ms = 0;
-    cudaEventElapsedTime(&ms, a, b);
-    if (ms < best) best_cluster = true;
+    // (The smallest clusters that hold a member fill the device best, the
+    // largest are the quickest each.)
+    std::vector<Layout> tries;
+    for (int nc : {4, 5, 6, 8, 9, 10, 12, 16}) {
+      if (!tries.empty() && nc < 16) continue;
+      bool any = false;
+      for (const auto &g : grids_) any = any || resident::plan_cluster(g, nc).ctas() > 0;
+      if (any) tries.push_back(Layout{nc, 2});
+    }
+    tries.push_back(Layout{0, 2});
+    tries.push_back(Layout{0, 1});
+    for (const Layout &l : tries) {
+      if (!layout_holds(l)) continue;
+      layout_ = l;
+      packed_.clear();
+      set_cluster(true);
+      forward(false, n_steps);
+      cudaEventRecord(a, stream_);
+      forward(false, n_steps);
+      cudaEventRecord(b, stream_);
+      cudaEventSynchronize(b);
+      float ms = 0;
+      cudaEventElapsedTime(&ms, a, b);
+      if (ms < best) {
+        best = ms;
+        best_cluster = true;
+        best_layout = l;
+      }
+    }
+    layout_ = best_cluster ? best_layout : layout_;
+    packed_.clear();
   }
   cudaEventDestroy(a);
   cudaEventDestroy(b);

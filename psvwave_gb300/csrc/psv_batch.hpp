@@ -11,6 +11,7 @@
 #include <vector>
 
 #include "psv_model.hpp"
+#include "psv_resident.hpp"
 #include "psv_tma.hpp"
 
 namespace psv {
@@ -52,12 +53,11 @@ class Batch {
   // so the per-item scheduling of the persistent scheme is measured slower.
   void set_persistent(bool on);
   bool persistent() const { return persistent_; }
-  // Cluster-resident scheme: every member in its own thread-block cluster
-  // that holds its whole grid in shared memory for every step, all members
-  // in one launch (members must fit: cluster_fits()). Takes precedence over
-  // the tile schemes while on; set_persistent() switches it off. Results
-  // equal each model's own cluster-resident run (variant fused_cluster) bit
-  // for bit.
+  // Resident scheme (psv_resident.hpp): every member's grid on chip for every
+  // step, each on its own team of CTAs (members must fit: cluster_fits()).
+  // Takes precedence over the tile schemes while on; set_persistent()
+  // switches it off. Results equal each model's own resident run (variant
+  // fused_cluster) bit for bit.
   bool cluster_fits();
   void set_cluster(bool on);
   bool cluster() const { return cluster_; }
@@ -88,8 +88,20 @@ class Batch {
   std::vector<int> active_h_;
   bool persistent_ = false;
   bool cluster_ = false;
-  int cluster_nc_ = -1;      // -1: not planned yet; 0: the members do not fit
-  size_t cluster_smem_ = 0;
+  // Resident scheme. A layout says how members become teams: clusters of nc
+  // CTAs where they hold the member (0: none), otherwise mailbox teams with
+  // per_sm CTAs sharing an SM.
+  struct Layout {
+    int nc = 0, per_sm = 2;
+  };
+  Layout layout_;
+  int fits_ = -1;  // -1: not planned yet
+  std::vector<resident::Grid> grids_;       // per member
+  std::vector<resident::Launch> launches_;  // of the active members
+  std::vector<int> packed_;                 // active flags the launches were made for
+  DeviceBuffer res_members_, res_ctas_, mail_;
+  bool layout_holds(const Layout &l);
+  void pack();
   DeviceBuffer sched_;               // persistent scheme: item counter, tile progress
   DeviceBuffer rec_start_, rec_list_;  // receivers by member tile (persistent scheme)
   std::vector<size_t> raw_off_;  // per member, floats into raw_

@@ -14,7 +14,6 @@
 #include <sstream>
 
 #include "../../include/psvwave.h"
-#include "psv_cluster.hpp"
 #include "psv_exact_tma.hpp"
 #include "psv_fast.hpp"
 
@@ -44,12 +43,16 @@ void cuda_check(cudaError_t e, const char *what) {
 
 DeviceBuffer::~DeviceBuffer() { release(); }
 
-void DeviceBuffer::allocate(size_t bytes) {
+void DeviceBuffer::allocate(size_t bytes, bool wait) {
   release();
   if (bytes == 0) bytes = 16;
   cuda_check(cudaMalloc(&ptr_, bytes), "cudaMalloc");
   bytes_ = bytes;
+  // cudaMemset is asynchronous on the legacy stream, and the streams that use
+  // the buffer do not wait for that one: a late clearing would wipe what they
+  // write first.
   cuda_check(cudaMemset(ptr_, 0, bytes), "cudaMemset");
+  if (wait) cuda_check(cudaStreamSynchronize(cudaStreamLegacy), "cudaMemset");
 }
 
 void DeviceBuffer::release() {
@@ -87,6 +90,7 @@ Model::Model(const Config &cfg, int precision, int device)
                           cudaMemcpyHostToDevice),
                "upload medium");
   }
+  cuda_check(cudaStreamSynchronize(cudaStreamLegacy), "upload medium");
   update_from_velocity();
   build_plans();
   // Tile shape. Grids with at least a full wave of 32 x 60 tiles keep them
@@ -110,10 +114,12 @@ Model::Model(const Config &cfg, int precision, int device)
     if (tile_cfg_ == tma::kTile32x60 && slots > 0 &&
         tma::tile_count(tile_cfg_, geo_.nx, geo_.nz) >= slots)
       variant_ = kFusedTmaPersistent;
-    // Grids that one thread-block cluster holds in shared memory run
-    // cluster-resident (up to kClusterCells points).
-    if (cluster_nc_ > 0 && static_cast<double>(geo_.nx) * geo_.nz <= kClusterCells)
+    // Grids that fit on the chip run resident. Up to kClusterCells points that
+    // is the variant; larger ones keep their tile variant, which takes over
+    // once a variant or tile shape is set.
+    if (resident_.ctas() > 0 && static_cast<double>(geo_.nx) * geo_.nz <= kClusterCells)
       variant_ = kFusedCluster;
+    resident_on_ = resident_.ctas() > 0;
   }
   synchronize();
 }
@@ -154,6 +160,7 @@ Model::Model(const Model &o)
     copy(kvel_[k], o.kvel_[k]);
   }
   build_descs();
+  resident_on_ = o.resident_on_;
 }
 
 Model::~Model() {
@@ -218,29 +225,29 @@ void Model::build_tables() {
 
 void Model::allocate() {
   const size_t g = grid_size(), gp = padded_size(), e = elem(), d = data_size();
-  for (auto &f : fields_) f.allocate(gp * e);
+  for (auto &f : fields_) f.allocate(gp * e, false);
   if (prec_ == PSV_FP32)
-    for (auto &f : fields2_) f.allocate(gp * e);
-  lm_.allocate(gp * e);
-  la_.allocate(gp * e);
-  mu_.allocate(gp * e);
-  b_.allocate(gp * e);
-  vp_.allocate(g * sizeof(double));
-  vs_.allocate(g * sizeof(double));
-  rho_.allocate(g * sizeof(double));
+    for (auto &f : fields2_) f.allocate(gp * e, false);
+  lm_.allocate(gp * e, false);
+  la_.allocate(gp * e, false);
+  mu_.allocate(gp * e, false);
+  b_.allocate(gp * e, false);
+  vp_.allocate(g * sizeof(double), false);
+  vs_.allocate(g * sizeof(double), false);
+  rho_.allocate(g * sizeof(double), false);
   for (int k = 0; k < 2; ++k) {
-    rtf_[k].allocate(d * sizeof(double));
-    rtf_true_[k].allocate(d * sizeof(double));
-    a_stf_[k].allocate(d * sizeof(double));
+    rtf_[k].allocate(d * sizeof(double), false);
+    rtf_true_[k].allocate(d * sizeof(double), false);
+    a_stf_[k].allocate(d * sizeof(double), false);
   }
-  rec_raw_.allocate(2 * static_cast<size_t>(cfg_.nr) * cfg_.nt * e);
-  rec_cell_.allocate(static_cast<size_t>(cfg_.nr) * sizeof(int));
-  for (auto &k : klame_) k.allocate(g * sizeof(double));
-  for (auto &k : kvel_) k.allocate(g * sizeof(double));
-  partials_.allocate(kPartials * sizeof(double));
-  err_flag_.allocate(sizeof(int));
-  scalar_.allocate(sizeof(double));
-  stf_d_.allocate(stf_.size() * sizeof(double));
+  rec_raw_.allocate(2 * static_cast<size_t>(cfg_.nr) * cfg_.nt * e, false);
+  rec_cell_.allocate(static_cast<size_t>(cfg_.nr) * sizeof(int), false);
+  for (auto &k : klame_) k.allocate(g * sizeof(double), false);
+  for (auto &k : kvel_) k.allocate(g * sizeof(double), false);
+  partials_.allocate(kPartials * sizeof(double), false);
+  err_flag_.allocate(sizeof(int), false);
+  scalar_.allocate(sizeof(double), false);
+  stf_d_.allocate(stf_.size() * sizeof(double), false);
   if (!stf_.empty())
     cuda_check(cudaMemcpy(stf_d_.get(), stf_.data(), stf_.size() * sizeof(double),
                           cudaMemcpyHostToDevice),
@@ -267,8 +274,8 @@ void Model::allocate() {
     }
     n_rec_groups_ = static_cast<int>(start.size());
     start.push_back(static_cast<int>(order.size()));
-    rec_start_.allocate(start.size() * sizeof(int));
-    rec_order_.allocate(std::max<size_t>(order.size(), 1) * sizeof(int));
+    rec_start_.allocate(start.size() * sizeof(int), false);
+    rec_order_.allocate(std::max<size_t>(order.size(), 1) * sizeof(int), false);
     cuda_check(cudaMemcpy(rec_start_.get(), start.data(), start.size() * sizeof(int),
                           cudaMemcpyHostToDevice),
                "upload receiver groups");
@@ -286,8 +293,8 @@ void Model::allocate() {
     for (int t = 0; t < n_tiles; ++t) start[t + 1] += start[t];
     std::vector<int> fill(start.begin(), start.end() - 1);
     for (int r = 0; r < cfg_.nr; ++r) list[fill[exact_tma::tile_of(geo_.nz, ix_rec_[r], iz_rec_[r])]++] = r;
-    exrec_start_.allocate(start.size() * sizeof(int));
-    exrec_list_.allocate(list.size() * sizeof(int));
+    exrec_start_.allocate(start.size() * sizeof(int), false);
+    exrec_list_.allocate(list.size() * sizeof(int), false);
     cuda_check(cudaMemcpy(exrec_start_.get(), start.data(), start.size() * sizeof(int),
                           cudaMemcpyHostToDevice),
                "upload receiver tiles");
@@ -295,7 +302,7 @@ void Model::allocate() {
                           cudaMemcpyHostToDevice),
                "upload receiver tiles");
   }
-  taper_tab_d_.allocate(taper_tab_.size() * e);
+  taper_tab_d_.allocate(taper_tab_.size() * e, false);
   if (prec_ == PSV_FP64) {
     cuda_check(cudaMemcpy(taper_tab_d_.get(), taper_tab_.data(),
                           taper_tab_.size() * sizeof(double), cudaMemcpyHostToDevice),
@@ -371,8 +378,8 @@ void Model::build_plans() {
         const int cx = terms[k].cell / nz - x0, cz = terms[k].cell % nz - z0;
         map[static_cast<size_t>(cx) * plan.h + cz] = k;
       }
-      plan_terms_[p].allocate(terms.size() * sizeof(InjTerm));
-      plan_maps_[p].allocate(map.size() * sizeof(int));
+      plan_terms_[p].allocate(terms.size() * sizeof(InjTerm), false);
+      plan_maps_[p].allocate(map.size() * sizeof(int), false);
       cuda_check(cudaMemcpy(plan_terms_[p].get(), terms.data(), terms.size() * sizeof(InjTerm),
                             cudaMemcpyHostToDevice),
                  "upload injection terms");
@@ -386,8 +393,32 @@ void Model::build_plans() {
   }
 }
 
+resident::Grid Model::resident_grid() const {
+  resident::Grid g;
+  g.nx = geo_.nx;
+  g.nz = geo_.nz;
+  for (int r = 0; r < cfg_.nr; ++r) g.receivers.push_back(ix_rec_[r] * geo_.nz + iz_rec_[r]);
+  for (const auto &shot : cfg_.shots) {
+    std::vector<int> cells;
+    for (int s : shot) {
+      // The points of a source's stencil (build_plans).
+      const int c = ix_src_[s] * geo_.nz + iz_src_[s], nz = geo_.nz;
+      for (int o : {-nz - 1, -nz, -nz + 1, -1, 0, 1, nz - 1, nz}) cells.push_back(c + o);
+    }
+    std::sort(cells.begin(), cells.end());
+    cells.erase(std::unique(cells.begin(), cells.end()), cells.end());
+    g.sources.push_back(cells);
+  }
+  return g;
+}
+
 void Model::build_descs() {
   tma_ok_ = false;
+  // The buffers were cleared and the tables uploaded on the legacy stream, for
+  // which the model's stream does not wait.
+  struct Wait {
+    ~Wait() { cudaStreamSynchronize(cudaStreamLegacy); }
+  } wait;
   if (prec_ != PSV_FP32 || !tma::supported(geo_.nx, geo_.nz, pitch_)) return;
   const int n_shots = cfg_.n_shots;
   const size_t gsz = grid_size();
@@ -408,10 +439,7 @@ void Model::build_descs() {
     d.nt = cfg_.nt;
     d.nr = cfg_.nr;
     d.si = cfg_.snapshot_interval;
-    d.dt = static_cast<float>(cfg_.dt);
-    d.idx = static_cast<float>(1.0 / cfg_.dx);
-    d.idz = static_cast<float>(1.0 / cfg_.dz);
-    d.dt_d = cfg_.dt;
+    d.set_steps(cfg_.dt, cfg_.dx, cfg_.dz);
     d.lm = lm_.as<float>();
     d.mu = mu_.as<float>();
     d.b = b_.as<float>();
@@ -451,41 +479,45 @@ void Model::build_descs() {
     std::vector<int> fill(start.begin(), start.end() - 1);
     for (int r = 0; r < cfg_.nr; ++r)
       list[fill[tma::tile_of(tile_cfg_, geo_.nz, ix_rec_[r], iz_rec_[r])]++] = r;
-    rec_tile_start_.allocate(start.size() * sizeof(int));
-    rec_tile_list_.allocate(list.size() * sizeof(int));
+    rec_tile_start_.allocate(start.size() * sizeof(int), false);
+    rec_tile_list_.allocate(list.size() * sizeof(int), false);
     cuda_check(cudaMemcpy(rec_tile_start_.get(), start.data(), start.size() * sizeof(int),
                           cudaMemcpyHostToDevice),
                "receiver tiles");
     cuda_check(cudaMemcpy(rec_tile_list_.get(), list.data(), list.size() * sizeof(int),
                           cudaMemcpyHostToDevice),
                "receiver tiles");
-    sched_.allocate(tma::sched_words(tile_cfg_, geo_.nx, geo_.nz) * sizeof(unsigned));
+    sched_.allocate(tma::sched_words(tile_cfg_, geo_.nx, geo_.nz) * sizeof(unsigned), false);
     for (int k = 0; k < n_shots; ++k) {
       descs[k].rec_start = rec_tile_start_.as<int>();
       descs[k].rec_list = rec_tile_list_.as<int>();
     }
   }
   descs_h_ = std::move(descs);
-  cluster_nc_ = cluster::plan(geo_.nx, geo_.nz, cfg_.np_boundary);
+  resident_ = resident::plan(resident_grid());
+  const size_t mail = resident::mailbox_bytes(resident_);
+  if (mail_.bytes() < mail) mail_.allocate(mail, false);
   tma_ok_ = true;
 }
 
 cudaError_t Model::tma_forward(int shot, bool store, int it0, int it1, bool zero, bool finish,
-                               cudaEvent_t *events, bool allow_cluster) {
+                               cudaEvent_t *events, bool allow_resident) {
   cudaStream_t s = stream();
-  if (zero) {
+  const tma::SimDesc &h = descs_h_[shot];
+  const int cfg = tile_cfg_;
+  const bool on_chip = use_resident() && allow_resident && it1 > it0;
+  if (zero) cur_ = 0;
+  if (zero && !on_chip) {
     const size_t bytes = padded_size() * sizeof(float);
     for (int f = 0; f < 5; ++f) {
       cudaError_t e = cudaMemsetAsync(fields_[f].get(), 0, bytes, s);
       if (e == cudaSuccess) e = cudaMemsetAsync(fields2_[f].get(), 0, bytes, s);
       if (e != cudaSuccess) return e;
     }
-    cur_ = 0;
   }
-  const tma::SimDesc &h = descs_h_[shot];
-  const int cfg = tile_cfg_;
-  if (variant_ == kFusedCluster && allow_cluster && it1 > it0) {
-    cudaError_t e = cluster::steps(h, false, it0, it1 - it0, cur_, store, cluster_nc_, s);
+  if (on_chip) {
+    cudaError_t e = resident::steps(h, resident_, false, it0, it1 - it0, cur_, zero, store,
+                                    resident::Dump(), mail_.get(), err_flag_.as<int>(), s);
     if (e != cudaSuccess) return e;
     cur_ ^= (it1 - it0) & 1;
     it0 = it1;  // done; falls through to the seismograms
@@ -520,21 +552,22 @@ cudaError_t Model::tma_forward(int shot, bool store, int it0, int it1, bool zero
 
 cudaError_t Model::tma_adjoint(int shot) {
   cudaStream_t s = stream();
+  const tma::SimDesc &h = descs_h_[cfg_.n_shots + shot];
+  cur_ = 0;
+  if (use_resident()) {
+    cudaError_t e = resident::steps(h, resident_, true, cfg_.nt - 1, cfg_.nt, 0, true, false,
+                                    resident::Dump(), mail_.get(), err_flag_.as<int>(), s);
+    if (e != cudaSuccess) return e;
+    cur_ = cfg_.nt & 1;
+    return cudaGetLastError();
+  }
   const size_t bytes = padded_size() * sizeof(float);
   for (int f = 0; f < 5; ++f) {
     cudaError_t e = cudaMemsetAsync(fields_[f].get(), 0, bytes, s);
     if (e == cudaSuccess) e = cudaMemsetAsync(fields2_[f].get(), 0, bytes, s);
     if (e != cudaSuccess) return e;
   }
-  cur_ = 0;
-  const tma::SimDesc &h = descs_h_[cfg_.n_shots + shot];
   const int cfg = tile_cfg_;
-  if (variant_ == kFusedCluster) {
-    cudaError_t e = cluster::steps(h, true, cfg_.nt - 1, cfg_.nt, 0, false, cluster_nc_, s);
-    if (e != cudaSuccess) return e;
-    cur_ = cfg_.nt & 1;
-    return cudaGetLastError();
-  }
   if (variant_ == kFusedTmaPersistent) {
     cudaError_t e = cudaMemsetAsync(sched_.get(), 0, sched_.bytes(), s);
     if (e == cudaSuccess)
@@ -707,7 +740,7 @@ double Model::exact_gradient(int C, const std::vector<int> &shot_list) {
       const int last0 = (n_ck - 1) * C;
       // The checkpoint pass runs the TMA step, as the recompute does, so that
       // every state is the same whatever the checkpoint interval (the
-      // cluster scheme agrees with it to FP32 rounding, not bit for bit).
+      // resident scheme agrees with it to FP32 rounding, not bit for bit).
       if (last0 > 0)
         cuda_check(tma_forward(shot, false, 0, 0, true, false, nullptr, false), "zero");
       for (int k = 0; k + 1 < n_ck; ++k) {
@@ -1247,7 +1280,7 @@ double Model::exact_gradient_lanes(int C, const std::vector<int> &shot_list) {
 }
 
 bool Model::run_model_lanes_ok() const {
-  return prec_ == PSV_FP32 && tma_ok_ && cfg_.n_shots > 1 &&
+  return prec_ == PSV_FP32 && tma_ok_ && cfg_.n_shots > 1 && !use_resident() &&
          (variant_ == kFusedTma || variant_ == kFusedTmaPersistent);
 }
 
@@ -1421,8 +1454,10 @@ void Model::get_exact_gradient(double *g_vp, double *g_vs, double *g_rho, bool d
 
 void Model::set_tile_cfg(int cfg) {
   if (cfg < 0 || cfg >= tma::kNumTileCfgs) throw Error(PSV_ERR_INVALID_ARGUMENT, "unknown tile shape");
-  if (cfg == tile_cfg_) return;
   DeviceGuard guard(device_);
+  if (resident_on_) clear_graphs();
+  resident_on_ = false;
+  if (cfg == tile_cfg_) return;
   clear_graphs();
   tile_cfg_ = cfg;
   if (tma_ok_) {
@@ -1445,7 +1480,7 @@ int Model::autotune(int n_steps) {
   int best_cfg = tile_cfg_, best_variant = variant_;
   bool first = true;
   std::vector<int> variants = {kFusedTma, kFusedTmaPersistent};
-  if (cluster_nc_ > 0) variants.push_back(kFusedCluster);
+  if (resident_.ctas() > 0) variants.push_back(kFusedCluster);
   for (int v : variants) {
     for (int c = 0; c < tma::kNumTileCfgs; ++c) {
       if (v == kFusedCluster && c > 0) break;  // no tiles: timed once
@@ -1698,7 +1733,7 @@ int Model::profile_forward(int shot, int n_steps, double *per_step_ms, double *k
   if (prec_ == PSV_FP64)
     err = forward_f64(a, plans_[shot], shot, false, 0, n_steps, true, false, stream());
   else if (variant_ == kFusedTma)
-    err = tma_forward(shot, false, 0, n_steps, true, false, a.events);
+    err = tma_forward(shot, false, 0, n_steps, true, false, a.events, false);
   else if (variant_ == kFused)
     err = fast::forward(a, second, &cur_, plans_[shot], shot, false, 0, n_steps, true, false,
                         stream());
@@ -1736,9 +1771,8 @@ void Model::set_variant(int v) {
     throw Error(PSV_ERR_INVALID_ARGUMENT, "the fused variants are FP32 only");
   if ((v == kFusedTma || v == kFusedTmaPersistent || v == kFusedCluster) && !tma_ok_)
     throw Error(PSV_ERR_INVALID_ARGUMENT, "the TMA variant needs driver tensor-map support");
-  if (v == kFusedCluster && cluster_nc_ == 0)
-    throw Error(PSV_ERR_INVALID_ARGUMENT,
-                "the grid does not fit in the shared memory of one thread-block cluster");
+  if (v == kFusedCluster && resident_.ctas() == 0)
+    throw Error(PSV_ERR_INVALID_ARGUMENT, "the grid does not fit on the chip");
   DeviceGuard guard(device_);
   if ((v == kTwoKernel) != (variant_ == kTwoKernel) && cur_ == 1) {
     // Bring the current state back into the primary buffers.
@@ -1749,6 +1783,7 @@ void Model::set_variant(int v) {
     cur_ = 0;
   }
   variant_ = v;
+  resident_on_ = false;
   clear_graphs();
   synchronize();
 }
@@ -1757,7 +1792,7 @@ const char *Model::step_kernel_name(int k) const {
   if (variant_ == kFused) return k == 0 ? "fused_step" : "";
   if (variant_ == kFusedTma) return k == 0 ? "fused_step_tma" : "";
   if (variant_ == kFusedTmaPersistent) return k == 0 ? "fused_steps_tma" : "";
-  if (variant_ == kFusedCluster) return k == 0 ? "cluster_steps" : "";
+  if (variant_ == kFusedCluster) return k == 0 ? "resident_steps" : "";
   return k == 0 ? "stress_step" : (k == 1 ? "velocity_step" : "");
 }
 

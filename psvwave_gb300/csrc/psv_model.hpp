@@ -15,6 +15,7 @@
 #include "psv_config.hpp"
 #include "psv_solver.hpp"
 #include "psv_exact_tma.hpp"
+#include "psv_resident.hpp"
 #include "psv_tma.hpp"
 
 namespace psv {
@@ -62,7 +63,9 @@ class DeviceBuffer {
     }
     return *this;
   }
-  void allocate(size_t bytes);  // zero-filled
+  // Zero-filled; wait = false: the clearing, and what follows it on the legacy
+  // stream, may still run (the caller waits for that stream).
+  void allocate(size_t bytes, bool wait = true);
   void release();
   void *get() const { return ptr_; }
   size_t bytes() const { return bytes_; }
@@ -165,8 +168,8 @@ class Model {
   size_t exact_bytes(int checkpoint_every) const;
   int variant() const { return variant_; }
   int kernels_per_step() const { return variant_ == kTwoKernel ? 2 : 1; }
-  // The FP32 variants built on the TMA step's descriptors (the cluster
-  // variant shares them, and the exact adjoint's recompute runs the TMA step).
+  // The FP32 variants built on the TMA step's descriptors (the resident
+  // scheme shares them, and the exact adjoint's recompute runs the TMA step).
   bool is_tma() const {
     return variant_ == kFusedTma || variant_ == kFusedTmaPersistent || variant_ == kFusedCluster;
   }
@@ -216,8 +219,17 @@ class Model {
 
   int pitch_ = 0;
   int variant_ = kTwoKernel;
-  int cluster_nc_ = 0;  // CTAs of the cluster that holds the grid, 0 if none does
-  static constexpr double kClusterCells = 1.0e5;  // default cluster-resident up to this size
+  // Grid resident on chip (psv_resident.hpp): its split (no CTAs: does
+  // not fit), and whether simulations use it beyond variant kFusedCluster: on
+  // for models whose variant and tile shape were left to the default.
+  resident::Plan resident_;
+  bool resident_on_ = false;
+  bool use_resident() const {
+    return resident_.ctas() > 0 && (variant_ == kFusedCluster || resident_on_);
+  }
+  resident::Grid resident_grid() const;
+  DeviceBuffer mail_;  // resident scheme: mailboxes between CTAs
+  static constexpr double kClusterCells = 1.0e5;  // variant kFusedCluster by default up to this size
   int cur_ = 0;  // fused variants: 0 = fields_ hold the current state, 1 = fields2_
   // TMA step: one simulation descriptor per (direction, shot) --
   // [0, n_shots) forward, [n_shots, 2 n_shots) adjoint -- on the host (their
@@ -228,7 +240,7 @@ class Model {
   void build_descs();
   cudaError_t tma_forward(int shot, bool store, int it0, int it1, bool zero, bool finish,
                           cudaEvent_t *events,
-                          bool allow_cluster = true);
+                          bool allow_resident = true);
   cudaError_t tma_adjoint(int shot);
   void check_device_error();
 

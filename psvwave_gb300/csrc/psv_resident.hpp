@@ -1,0 +1,110 @@
+// FP32 time stepping of grids held on chip for every time step of a launch
+// (psv_resident_f32.cu).
+//
+// A simulation runs on a team of CTAs, one per SM, each owning a tile of at
+// most 64 columns. Every thread keeps its points' wave fields and medium in
+// registers for all steps, and the tile's fields lie in shared memory for
+// the neighbours' stencils. After each half-step the tile's edges go to the
+// neighbouring CTAs through mailboxes in global memory (L2) whose 64-bit
+// words carry a value and the step's number, so that the receiver needs no
+// flag, fence or barrier. Global memory otherwise carries only the initial
+// and final state, receivers, snapshots, correlations and injection.
+#pragma once
+
+#include <cuda_runtime.h>
+
+#include <vector>
+
+#include "psv_tma.hpp"
+
+namespace psv {
+namespace resident {
+
+// A grid to split: its size, and the cells (ix nz + iz) of its receivers
+// and of each shot's injection points.
+struct Grid {
+  int nx = 0, nz = 0;
+  std::vector<int> receivers;
+  std::vector<std::vector<int>> sources;
+};
+
+// How one simulation is split: tiles_x x tiles_z CTAs, blocks of `threads`
+// with `groups` thread groups of at most `rows` rows each, shared rows of
+// `stride` floats; n_rec, n_inj: the most receivers and injection points of a
+// tile. cluster: the team is one thread-block cluster; otherwise its edges go
+// through mailboxes. No CTAs: the grid does not fit.
+struct Plan {
+  int tiles_x = 0, tiles_z = 0, groups = 0, rows = 0, threads = 0, stride = 0;
+  int n_rec = 0, n_inj = 0;
+  bool cluster = false;
+  size_t smem = 0;
+  int ctas() const { return tiles_x * tiles_z; }
+};
+
+// The split of a grid for one simulation at a time: the largest cluster that
+// holds it, else mailboxes over the whole device. These calls set launch
+// attributes as a side effect (call outside stream capture). Measured, one
+// simulation: 250 x 150 points in one 16-CTA cluster 1.8 us a step, by
+// mailboxes 2.6 to 3.6 us (32 to 152 CTAs); 1103 x 497 points 3.9 us by
+// mailboxes.
+Plan plan(const Grid &g);
+// A cluster of exactly nc CTAs.
+Plan plan_cluster(const Grid &g, int nc);
+// Mailboxes over at most max_ctas CTAs (0: as many as are resident at once),
+// per_sm (1 or 2) of them sharing an SM.
+Plan plan_mailbox(const Grid &g, int max_ctas, int per_sm);
+
+// States saved during a run: the state before step j of the launch goes to
+// base + (j / every) * stride when j % every == 0 (five planes of
+// nx * pitch floats). last: the final state too, where it falls on a
+// multiple of `every`.
+struct Dump {
+  float *base = nullptr;
+  size_t stride = 0;
+  int every = 1;
+  int last = 0;
+};
+
+// Mailbox bytes of a plan (0 for a cluster).
+size_t mailbox_bytes(const Plan &p);
+
+// n_steps steps of simulation d from set `parity` (forward: it0, it0 + 1,
+// ...; adjoint: it0, it0 - 1, ...), final state in set parity ^ (n_steps & 1);
+// forward snapshots when store. zero: start from zero fields instead of the
+// set's. mail: mailbox_bytes(p) of scratch (cleared here on s). One launch. *err is raised when a bounded wait for a neighbour runs
+// out.
+cudaError_t steps(const tma::SimDesc &d, const Plan &p, bool adjoint, int it0, int n_steps,
+                  int parity, bool zero, bool store, const Dump &dump, void *mail, int *err,
+                  cudaStream_t s);
+
+// ---- batches: forward steps of many simulations from zero fields ----
+
+// One member of a batched launch: its CTAs first .. first + tiles_x tiles_z - 1
+// run simulation `sim` of the table.
+struct Member {
+  int sim, first, tiles_x, tiles_z, groups, n_rec, n_inj;
+};
+// One launch: CTAs first_cta .. first_cta + ctas - 1 of the CTA table (the
+// launch's member of each), members from first_member on. team > 0: clusters
+// of `team` CTAs, one member each, as many as there are (they queue for the
+// device); team = 0: a cooperative launch whose teams exchange edges through
+// mailboxes. All members have plans of `rows` and `stride`; threads and smem
+// are their largest.
+struct Launch {
+  int first_member = 0, first_cta = 0, ctas = 0, team = 0;
+  int rows = 0, stride = 0, threads = 0;
+  size_t smem = 0;
+};
+size_t launch_mailbox_bytes(const Launch &l);
+cudaError_t steps_batch(const tma::SimDesc *sims, const Member *members, const int *cta_member,
+                        const Launch &l, int n_steps, bool store, void *mail, int *err,
+                        cudaStream_t s);
+// CTAs resident at once in a cooperative launch of per_sm CTAs per SM.
+int resident_slots(int per_sm);
+// The mailbox split with the fewest CTAs, and the same with tiles_x tiles
+// along x (false, p unchanged: does not fit).
+Plan plan_smallest(const Grid &g, int per_sm);
+bool set_tiles_x(Plan &p, const Grid &g, int tiles_x, int per_sm);
+
+}  // namespace resident
+}  // namespace psv

@@ -35,6 +35,19 @@ struct alignas(128) SimDesc {
   int nx = 0, nz = 0, pitch = 0, np = 0, nt = 0, nr = 0, si = 1;
   float dt = 0, idx = 0, idz = 0;
   double dt_d = 0;
+  // The resident step's stencil coefficients times dt / dx and dt / dz (9/8 and
+  // 1/24 along x, then z), each rounded once.
+  float coef[4] = {0, 0, 0, 0};
+  void set_steps(double dt, double dx, double dz) {
+    this->dt = static_cast<float>(dt);
+    idx = static_cast<float>(1.0 / dx);
+    idz = static_cast<float>(1.0 / dz);
+    dt_d = dt;
+    coef[0] = static_cast<float>(9.0 / 8.0 * dt / dx);
+    coef[1] = static_cast<float>(1.0 / 24.0 * dt / dx);
+    coef[2] = static_cast<float>(9.0 / 8.0 * dt / dz);
+    coef[3] = static_cast<float>(1.0 / 24.0 * dt / dz);
+  }
   const float *lm = nullptr, *b = nullptr, *taper_tab = nullptr;
   const float *mu = nullptr;  // (the TMA steps read mu through the maps)
   float *accu[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};  // this shot's snapshots

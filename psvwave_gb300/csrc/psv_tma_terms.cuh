@@ -1,5 +1,5 @@
 // Per-point terms shared by the FP32 fused steps (psv_tma_f32.cu,
-// psv_cluster_f32.cu): the adjoint's kernel correlation with a stored
+// psv_resident_f32.cu): the adjoint's kernel correlation with a stored
 // forward snapshot (src/fdModel.cpp:817-861, FP64 accumulation) and the
 // source / adjoint-source injection after the velocity update
 // (src/fdModel.cpp:681-751, 951-958), in the reference's operation order.
