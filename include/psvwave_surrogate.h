@@ -60,6 +60,12 @@ int psv_cnn_get_params(psv_cnn *n, float *params);
 /* x_dev [batch][5][200] -> misfit_dev [batch], grad_dev [batch][3][200]. */
 int psv_cnn_predict(psv_cnn *n, int batch, const float *x_dev, float *misfit_dev,
                     float *grad_dev);
+/* The same at states z_dev [batch][3][200] in physical units: the network sees
+ * z and the coordinate channels coords_dev [2][200]; misfit_dev [batch] (FP64)
+ * = m0 + ms m, grad_dev = gs_dev [3][200] times the predicted map. */
+int psv_cnn_predict_states(psv_cnn *n, int batch, const float *z_dev, const float *coords_dev,
+                           double m0, double ms, const float *gs_dev, double *misfit_dev,
+                           float *grad_dev);
 /* Loss = w_misfit mean_b (m - m_true)^2 + w_grad mean (g - g_true)^2 of a
  * batch, and its gradient with respect to the parameters (host,
  * psv_cnn_num_params floats; NULL to skip). */

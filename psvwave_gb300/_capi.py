@@ -153,6 +153,7 @@ _SIGNATURES = {
     "psv_cnn_set_params": [_vp, _vp],
     "psv_cnn_get_params": [_vp, _vp],
     "psv_cnn_predict": [_vp, _c_int, _vp, _vp, _vp],
+    "psv_cnn_predict_states": [_vp, _c_int, _vp, _vp, _c_double, _c_double, _vp, _vp, _vp],
     "psv_cnn_loss_grad": [_vp, _c_int, _vp, _vp, _vp, ctypes.c_float, ctypes.c_float, _dp, _vp],
     "psv_cnn_train_step": [_vp, _c_int, _vp, _vp, _vp, ctypes.c_float, ctypes.c_float,
                            ctypes.c_float, ctypes.c_float, ctypes.c_float, ctypes.c_float, _dp],

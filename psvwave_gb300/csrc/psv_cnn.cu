@@ -2,15 +2,15 @@
 // parameter map of the Monte Carlo workload; see psv_cnn.hpp.
 //
 // The convolutions run on the tensor cores as tcgen05 implicit GEMMs with
-// BF16 hi + lo operand splits and FP32 accumulators in TMEM: the forward
-// and the input gradient (with the ReLU mask of the layer's input fused in)
-// in conv_tc, the weight and bias gradients in conv_weight_tc as
-// fixed-order partial sums over position ranges that a second kernel adds
-// up, so every result is deterministic.
+// BF16 hi + lo operand splits and FP32 accumulators in TMEM: one kernel takes
+// an image through every layer (net_images: forward, and for training the
+// loss and the input gradients), one sums the weight and bias gradients
+// (net_weights, fixed-order partial sums), so every result is deterministic.
 #include "psv_cnn.hpp"
 
 #include <algorithm>
 #include <cmath>
+#include <cstring>
 #include <vector>
 
 #include "../../include/psvwave.h"
@@ -20,8 +20,6 @@ namespace cnn {
 
 namespace {
 
-constexpr int kThreads = 256;
-
 size_t layer_size(int l) { return (size_t)kCout[l] * kCin[l] * 9 + kCout[l]; }
 
 
@@ -30,43 +28,34 @@ __device__ __forceinline__ void tap(int k, int dil, int &dh, int &dc) {
   dc = (k % 3 - 1) * dil;
 }
 
-// ---- tensor-core convolutions (tcgen05): forward and input gradient -------
+// ---- tensor-core convolutions (tcgen05) -------------------------------------
 //
-// The forward convolution as an implicit GEMM on the 5th-generation tensor
-// cores: D[pos][co] = sum_k A[pos][k] W[co][k], with pos = b kP + p running
-// over the batch (kTcM = 128 positions per CTA, the MMA's M), co over the
-// output channels (N = cout rounded up to 16), and k = ci * 9 + tap over
-// the input channels and the 3 x 3 taps. K runs in chunks of kTcKc = 64:
-// seven input channels (63 columns) and one zero column, so that a column's
-// channel and tap are compile-time constants of the unrolled gather. Per
-// chunk each of the 128 threads gathers its position's row of the im2col
-// tile into shared memory (16-byte stores) as two BF16 matrices,
-// hi = bf16(x) and lo = bf16(x - hi), and the threads copy the chunk of
-// BF16 weights; one thread issues the tcgen05.mma instructions
-// (kind::f16, BF16 x BF16 -> FP32) for both, accumulating into a TMEM tile
-// of 128 lanes x 64 columns, and commits them to an mbarrier that every
-// thread waits on (bounded) before the next chunk overwrites the tiles.
-// Each warp then reads its 32 TMEM lanes (tcgen05.ld), adds the bias,
-// applies the ReLU and writes y[b][co][p].
+// Every convolution is an implicit GEMM in kind::f16 MMAs (BF16 x BF16 ->
+// FP32 in TMEM). FP32 operands are split into BF16 parts, hi = bf16(x) and
+// lo = bf16(x - hi), which keeps 16 significant bits (about 2^-17 relative;
+// products of BF16 values are exact in FP32). Tensors between the
+// convolutions are stored as such pairs, one 32-bit word (hi in the upper
+// half), split once by their producer, [image][channel][kPW] with kPW = 208
+// words a channel (200 positions and zeros, which taps outside the image
+// read).
 //
-// The hi + lo split keeps 16 significant bits of each activation (about
-// 2^-17 relative; the products of BF16 values are exact in FP32), so the
-// results are the FP32 convolution of the activations so rounded, up to
-// accumulation order: BF16 weights, FP32 activations and accumulation, as
-// the network is specified, to about 1e-6 relative.
-//
-// Shared-memory operands are K-major without swizzle: 8 x 16-byte core
+// A lies in TMEM: a thread owns a row (lane) and writes its columns straight
+// from registers (tcgen05.st, two BF16 a 32-bit column). Through shared memory
+// A's stores and the MMAs' reads of it took more of the shared-memory
+// bandwidth than the gather itself. B's operands are K-major in shared memory
+// without swizzle: 8 x 16-byte core
 // matrices, element (r, k) at (r / 8) * kTcSBO + (k / 8) * 128 +
 // (r % 8) * 16 + (k % 8) * 2; the descriptor's leading byte offset (between
 // K-adjacent core matrices) is 128, its stride byte offset (between 8-row
 // groups) kTcSBO.
-constexpr int kTcM = 128, kTcKc = 64, kTcCi = 7, kTcThreads = 128, kTcCols = 64;
+constexpr int kPW = 208;
+constexpr int kTcM = 128, kTcKc = 64, kTcCi = 7;
 constexpr int kTcLBO = 128, kTcSBO = (kTcKc / 8) * 128;
 
 __device__ __forceinline__ uint32_t tc_saddr(const void *p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
-__device__ __forceinline__ int tc_off(int r, int k) {
+__host__ __device__ __forceinline__ int tc_off(int r, int k) {
   return (r >> 3) * kTcSBO + (k >> 3) * kTcLBO + (r & 7) * 16 + (k & 7) * 2;
 }
 // Shared-memory matrix descriptor: start address >> 4 (bits 0-13), leading
@@ -76,431 +65,794 @@ __device__ __forceinline__ uint64_t tc_desc(uint32_t addr) {
   return (uint64_t)((addr & 0x3FFFF) >> 4) | ((uint64_t)(kTcLBO >> 4) << 16) |
          ((uint64_t)(kTcSBO >> 4) << 32) | ((uint64_t)1 << 46);
 }
-__device__ __forceinline__ void tc_mma(uint32_t tmem, uint64_t a, uint64_t b, uint32_t idesc,
+// Instruction descriptor: D FP32 (bits 4-5 = 1), A and B BF16 (7-9 = 1,
+// 10-12 = 1), both K-major, N >> 3 (17-22), M >> 4 (24-28).
+__device__ __forceinline__ uint32_t tc_idesc(int n) {
+  return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) |
+         ((uint32_t)(kTcM >> 4) << 24);
+}
+__device__ __forceinline__ void tc_mma(uint32_t tmem, uint32_t a, uint64_t b, uint32_t idesc,
                                        uint32_t accumulate) {
   asm volatile(
       "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-      " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}" ::"r"(tmem),
-      "l"(a), "l"(b), "r"(idesc), "r"(accumulate)
+      " tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}" ::"r"(tmem),
+      "r"(a), "l"(b), "r"(idesc), "r"(accumulate)
       : "memory");
 }
-__device__ __forceinline__ bool tc_wait(uint32_t bar, uint32_t parity) {
+// One lane of the calling (whole) warp.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t pred;
+  asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}" : "=r"(pred));
+  return pred != 0;
+}
+// A thread's columns of A: N registers into TMEM columns ta .. ta + N - 1 of
+// its lane.
+template <int N>
+__device__ __forceinline__ void tc_store(uint32_t ta, const uint32_t *v);
+template <>
+__device__ __forceinline__ void tc_store<8>(uint32_t ta, const uint32_t *v) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"r"(ta), "r"(v[0]),
+      "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
+      : "memory");
+}
+template <>
+__device__ __forceinline__ void tc_store<4>(uint32_t ta, const uint32_t *v) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1,%2,%3,%4};" ::"r"(ta), "r"(v[0]),
+               "r"(v[1]), "r"(v[2]), "r"(v[3])
+               : "memory");
+}
+__device__ __forceinline__ void tc_stored() {
+  asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+}
+__device__ __forceinline__ void tc_commit(uint32_t bar) {
+  asm volatile(
+      "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar)
+      : "memory");
+}
+__device__ __forceinline__ void tc_load16(uint32_t ta, uint32_t v[16]) {
+  __syncwarp();
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,"
+      "%14,%15}, [%16];"
+      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]),
+        "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]),
+        "=r"(v[14]), "=r"(v[15])
+      : "r"(ta));
+  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void tc_alloc(uint32_t *holder, int cols) {
+  asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
+                   tc_saddr(holder)),
+               "r"(cols)
+               : "memory");
+  asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void tc_dealloc(uint32_t tmem, int cols) {
+  asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(cols)
+               : "memory");
+}
+__device__ __forceinline__ void bar_init(uint64_t *bar, int count) {
+  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(tc_saddr(bar)), "r"(count)
+               : "memory");
+}
+__device__ __forceinline__ void bar_arrive(uint64_t *bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(tc_saddr(bar)) : "memory");
+}
+// Bounded wait on phase `parity` (about a second). *fail is the CTA's flag:
+// once a wait has run out no thread waits again, so that the kernel ends.
+__device__ __forceinline__ void bar_wait(uint64_t *bar, uint32_t parity, volatile int *fail) {
+  const uint32_t addr = tc_saddr(bar);
   for (uint32_t i = 0; i < (1u << 20); ++i) {
     uint32_t done;
     asm volatile(
         "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n"
         " selp.u32 %0, 1, 0, p;\n}"
         : "=r"(done)
-        : "r"(bar), "r"(parity), "r"(1000u)
+        : "r"(addr), "r"(parity), "r"(1000u)
         : "memory");
-    if (done) return true;
+    if (done || *fail) return;
   }
-  return false;
+  *fail = 1;
+}
+__device__ __forceinline__ void bulk_load(void *dst, const void *src, uint32_t bytes,
+                                          uint64_t *bar) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(tc_saddr(bar)),
+               "r"(bytes)
+               : "memory");
+  asm volatile(
+      "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::
+          "r"(tc_saddr(dst)),
+      "l"(src), "r"(bytes), "r"(tc_saddr(bar))
+      : "memory");
+}
+__device__ __forceinline__ uint32_t split_word(float x) {
+  const __nv_bfloat16 h = __float2bfloat16_rn(x);
+  const __nv_bfloat16 l = __float2bfloat16_rn(x - __bfloat162float(h));
+  return (uint32_t)__bfloat16_as_ushort(h) << 16 | __bfloat16_as_ushort(l);
+}
+// Packed weights: the B operand of every chunk of seven gathered channels (63
+// columns and a zero column), in its shared-memory layout, forward layers 0-3
+// then input gradients of layers 3, 2, 1 (rows are the layer's input channels,
+// columns its (output channel, tap)).
+constexpr int kSteps = 7;
+__host__ __device__ constexpr int step_layer(int s) { return s < kLayers ? s : 7 - s; }
+__host__ __device__ constexpr int layer_cin(int l) { return l == 0 ? 5 : l == 1 ? 32 : 64; }
+__host__ __device__ constexpr int layer_cout(int l) { return l == 0 ? 32 : l == 3 ? 4 : 64; }
+// Channels gathered, and columns of D.
+__host__ __device__ constexpr int step_k(int s) {
+  return s < kLayers ? layer_cin(step_layer(s)) : layer_cout(step_layer(s));
+}
+__host__ __device__ constexpr int step_n(int s) {
+  return s < kLayers ? (s == 3 ? 16 : layer_cout(s)) : layer_cin(step_layer(s));
+}
+static_assert(layer_cin(0) == kCin[0] && layer_cin(1) == kCin[1] && layer_cin(2) == kCin[2] &&
+                  layer_cin(3) == kCin[3] && layer_cout(0) == kCout[0] &&
+                  layer_cout(1) == kCout[1] && layer_cout(2) == kCout[2] &&
+                  layer_cout(3) == kCout[3],
+              "the layers' channels");
+__host__ __device__ constexpr int step_chunks(int s) { return (step_k(s) + kTcCi - 1) / kTcCi; }
+__host__ __device__ constexpr int step_bytes(int s) { return step_chunks(s) * step_n(s) * kTcKc * 2; }
+__host__ __device__ constexpr int step_offset(int s) {
+  int o = 0;
+  for (int i = 0; i < s; ++i) o += step_bytes(i);
+  return o;
+}
+constexpr int kPackedBytes = step_offset(kSteps);
+
+__global__ void pack_weights(const __nv_bfloat16 *__restrict__ wbf, unsigned char *__restrict__ out,
+                             const int4 offs) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;  // element of the packed operands
+  if (i >= kPackedBytes / 2) return;
+  int s = 0, base = 0;
+  while (2 * i >= base + step_bytes(s)) base += step_bytes(s++);
+  const int e = i - base / 2, per = step_n(s) * kTcKc;
+  const int ch = e / per, r = (e - ch * per) / kTcKc, kk = e - ch * per - r * kTcKc;
+  const int l = step_layer(s), cin = layer_cin(l), cout = layer_cout(l), k = ch * 9 * kTcCi + kk;
+  const __nv_bfloat16 *w = wbf + (l == 0 ? offs.x : l == 1 ? offs.y : l == 2 ? offs.z : offs.w);
+  __nv_bfloat16 v = __float2bfloat16_rn(0.f);
+  if (kk < 9 * kTcCi && k < 9 * step_k(s)) {
+    if (s < kLayers) {
+      if (r < cout) v = w[(size_t)r * cin * 9 + k];
+    } else if (r < cin) {
+      v = w[((size_t)(k / 9) * cin + r) * 9 + k % 9];
+    }
+  }
+  *reinterpret_cast<__nv_bfloat16 *>(out + base + ch * per * 2 + tc_off(r, kk)) = v;
 }
 
-// MODE kFwdRelu / kFwdLinear: the forward convolution above (x = layer
-// input [B][cin][kP], y = output [B][cout][kP], bias added, ReLU or not).
-// MODE kBwdData: the input gradient dx[b][ci][p] = (sum_co sum_tap
-// w[co][ci][tap] dy[b][co][p - off_tap]) [act[b][ci][p] > 0] as the same
-// implicit GEMM with the roles of the channels swapped: x = dy (gathered at
-// the negated tap offsets, K = cout * 9), B[ci][co * 9 + tap] =
-// w[co][ci][tap], N = cin rounded up to 16, and the ReLU mask of the
-// layer's input activation `act` applied in the epilogue (bias unused).
-constexpr int kFwdRelu = 0, kFwdLinear = 1, kBwdData = 2;
-
-template <int MODE>
-__global__ void __launch_bounds__(kTcThreads) conv_tc(int batch, int cin_l, int cout_l, int npad,
-                                                     int dil, const float *__restrict__ x,
-                                                     const __nv_bfloat16 *__restrict__ w,
-                                                     const float *__restrict__ bias,
-                                                     const float *__restrict__ act,
-                                                     float *__restrict__ y, int *err) {
-  constexpr bool BWD = MODE == kBwdData;
-  // Channels gathered (the GEMM's K / 9) and produced (its N).
-  const int cin = BWD ? cout_l : cin_l, cout = BWD ? cin_l : cout_l;
-  __shared__ __align__(1024) unsigned char a_hi[kTcM * kTcKc * 2];
-  __shared__ __align__(1024) unsigned char a_lo[kTcM * kTcKc * 2];
-  __shared__ __align__(1024) unsigned char b_w[kTcCols * kTcKc * 2];
-  __shared__ __align__(8) uint64_t bar;
-  __shared__ uint32_t tmem_holder;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int total = batch * kP, pos0 = blockIdx.x * kTcM;
-  const int K = cin * 9;
-  if (warp == 0) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
-                     tc_saddr(&tmem_holder)),
-                 "r"(kTcCols)
-                 : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-  }
-  if (tid == 0) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(tc_saddr(&bar)), "r"(1)
-                 : "memory");
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  }
-  // This thread's position for the gather (row tid of the tile) and the
-  // offsets of its nine taps within an input channel (-1 outside the image).
-  const int pos = pos0 + tid;
-  const bool row_ok = pos < total;
-  const int bs = row_ok ? pos / kP : 0, ps = row_ok ? pos - bs * kP : 0;
-  const int h = ps / kW, c = ps - h * kW;
-  int nb[9];
-#pragma unroll
-  for (int t = 0; t < 9; ++t) {
-    int dh, dc;
-    tap(t, dil, dh, dc);
-    const int hh = BWD ? h - dh : h + dh, cc = BWD ? c - dc : c + dc;
-    nb[t] = (row_ok && hh >= 0 && hh < kH && cc >= 0 && cc < kW) ? hh * kW + cc : -1;
-  }
-  const float *xb = x + (size_t)bs * cin * kP;
-  // idesc: D FP32 (bits 4-5 = 1), A and B BF16 (7-9 = 1, 10-12 = 1), both
-  // K-major, N >> 3 (17-22), M >> 4 (24-28).
-  const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(npad >> 3) << 17) |
-                         ((uint32_t)(kTcM >> 4) << 24);
-  bool ok = true;
-  uint32_t tmem = 0;
-  int ch = 0;
-  const int chunks = (cin + kTcCi - 1) / kTcCi;
-  for (; ch < chunks; ++ch) {
-    const int ci0 = ch * kTcCi;
-#pragma unroll
-    for (int g = 0; g < kTcKc / 8; ++g) {
-      uint32_t hi2[4], lo2[4];
-#pragma unroll
-      for (int e = 0; e < 8; e += 2) {
-        float v[2];
-#pragma unroll
-        for (int q = 0; q < 2; ++q) {
-          const int kk = 8 * g + e + q, j = kk / 9, t = kk - 9 * (kk / 9);
-          v[q] = 0.f;
-          if (kk < 9 * kTcCi && ci0 + j < cin && nb[t] >= 0)
-            v[q] = __ldg(xb + (size_t)(ci0 + j) * kP + nb[t]);
-        }
-        const __nv_bfloat162 h2 = __floats2bfloat162_rn(v[0], v[1]);
-        const float2 hf = __bfloat1622float2(h2);
-        const __nv_bfloat162 l2 = __floats2bfloat162_rn(v[0] - hf.x, v[1] - hf.y);
-        hi2[e / 2] = *reinterpret_cast<const uint32_t *>(&h2);
-        lo2[e / 2] = *reinterpret_cast<const uint32_t *>(&l2);
-      }
-      *reinterpret_cast<uint4 *>(a_hi + tc_off(tid, 8 * g)) =
-          make_uint4(hi2[0], hi2[1], hi2[2], hi2[3]);
-      *reinterpret_cast<uint4 *>(a_lo + tc_off(tid, 8 * g)) =
-          make_uint4(lo2[0], lo2[1], lo2[2], lo2[3]);
-    }
-    for (int i = tid; i < npad * kTcKc; i += kTcThreads) {
-      const int co = i / kTcKc, kk = i - co * kTcKc, k = ci0 * 9 + kk;
-      __nv_bfloat16 v = __float2bfloat16_rn(0.f);
-      if (co < cout && kk < 9 * kTcCi && k < K) {
-        // Forward: w[co][k]. Input gradient: row co is the layer's input
-        // channel, k = (output channel, tap) of the layer.
-        v = BWD ? w[((size_t)(k / 9) * cout + co) * 9 + (k - 9 * (k / 9))]
-                : w[(size_t)co * K + k];
-      }
-      *reinterpret_cast<__nv_bfloat16 *>(b_w + tc_off(co, kk)) = v;
-    }
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    tmem = tmem_holder;
-    if (tid == 0) {
-      for (int s = 0; s < kTcKc / 16; ++s) {
-        const uint32_t koff = s * 2 * kTcLBO;
-        const uint64_t bd = tc_desc(tc_saddr(b_w) + koff);
-        tc_mma(tmem, tc_desc(tc_saddr(a_hi) + koff), bd, idesc, (ch > 0 || s > 0) ? 1u : 0u);
-        tc_mma(tmem, tc_desc(tc_saddr(a_lo) + koff), bd, idesc, 1u);
-      }
-      asm volatile(
-          "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-              tc_saddr(&bar))
-          : "memory");
-    }
-    // The chunk's products must be done before its tiles are overwritten.
-    if (!tc_wait(tc_saddr(&bar), (uint32_t)(ch & 1))) ok = false;
-    if (__syncthreads_or(!ok)) {
-      ok = false;
-      break;
-    }
-  }
-  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  if (ok) {
-    const int row = 32 * warp + lane, g = pos0 + row;
-    const bool valid = g < total;
-    const int b = valid ? g / kP : 0, p = valid ? g - b * kP : 0;
-    for (int c0 = 0; c0 < npad; c0 += 16) {
-      uint32_t v[16];
-      const uint32_t ta = tmem + ((uint32_t)(32 * warp) << 16) + (uint32_t)c0;
-      asm volatile(
-          "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,"
-          "%14,%15}, [%16];"
-          : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]),
-            "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]),
-            "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
-          : "r"(ta));
-      asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-      if (valid) {
-#pragma unroll
-        for (int j = 0; j < 16; ++j) {
-          const int co = c0 + j;
-          if (co < cout) {
-            const size_t o = ((size_t)b * cout + co) * kP + p;
-            if (BWD) {
-              y[o] = act[o] > 0.f ? __uint_as_float(v[j]) : 0.f;
-            } else {
-              float r = __uint_as_float(v[j]) + bias[co];
-              if (MODE == kFwdRelu) r = fmaxf(r, 0.f);
-              y[o] = r;
-            }
-          }
-        }
-      }
-    }
-  } else if (tid == 0) {
-    atomicOr(err, 1);
-    // Bounded: give the products of the chunk that timed out (the last ones
-    // issued) more time to finish before the TMEM is freed.
-    tc_wait(tc_saddr(&bar), (uint32_t)(ch & 1));
-  }
-  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-  __syncthreads();
-  if (warp == 0)
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem),
-                 "r"(kTcCols)
-                 : "memory");
-}
-
-// ---- tensor-core weight gradients (tcgen05) --------------------------------
+// One image per CTA, all layers: the forward convolutions and the head, and
+// for training the loss and the input gradients back to layer 1, with the
+// image's tensor in shared memory between layers.
 //
-// dW[co][k] = sum_pos dy[pos][co] X[pos][k] and db[co] = sum_pos dy[pos][co]
-// as a GEMM whose reduction runs over the positions pos = b kP + p of the
-// batch: D[k][co] (M = 128 rows of k = ci * 9 + tap per CTA, the bias as row
-// k = cin * 9 with X = 1; N = cout rounded up to 16) accumulates
-// A[k][pos] B[co][pos] over chunks of 64 positions, with A = X^T the
-// transposed im2col of the layer input and B = dy^T. Both operands are FP32
-// values split into BF16 hi + lo parts; hi.hi + hi.lo + lo.hi (three
-// tcgen05.mma kind::f16 per 16 positions) carry the products to about 2^-16
-// relative, the FP32 accumulation order is fixed, and blockIdx.y splits the
-// chunks into kChunks ranges whose partial sums sum_chunks adds in order
-// (deterministic). Per chunk thread t gathers position t % 64 of rows
-// (t / 64) * 64 .. + 63 of A and every other row of B, one thread issues
-// the MMAs and commits them to an mbarrier every thread waits on (bounded;
-// a time-out raises the error flag). The epilogue reads row 32 w + lane of
-// the accumulator (tcgen05.ld.32x32b) and writes the CTA's partial sums in
-// the layout of the weights ((co cin + ci) 9 + tap, then the biases).
-__global__ void __launch_bounds__(kTcThreads) conv_weight_tc(int batch, int cin, int cout,
-                                                            int npad, int dil,
-                                                            const float *__restrict__ x,
-                                                            const float *__restrict__ dy,
-                                                            float *__restrict__ partial, int *err) {
-  __shared__ __align__(1024) unsigned char a_hi[kTcM * kTcKc * 2];
-  __shared__ __align__(1024) unsigned char a_lo[kTcM * kTcKc * 2];
-  __shared__ __align__(1024) unsigned char b_hi[kTcCols * kTcKc * 2];
-  __shared__ __align__(1024) unsigned char b_lo[kTcCols * kTcKc * 2];
-  __shared__ __align__(8) uint64_t bar;
-  __shared__ uint32_t tmem_holder;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int K = cin * 9;  // weight columns; row K is the bias
-  const int m0 = blockIdx.x * kTcM;
-  const int total = batch * kP;
-  const int n_chunks = (total + kTcKc - 1) / kTcKc;
-  const int c0 = (int)((long long)n_chunks * blockIdx.y / gridDim.y);
-  const int c1 = (int)((long long)n_chunks * (blockIdx.y + 1) / gridDim.y);
-  const size_t len = (size_t)cout * K + cout;
-  float *out = partial + (size_t)blockIdx.y * len;
-  const int k_out = m0 + 32 * warp + lane;  // the accumulator row this thread writes
-  auto out_index = [&](int co) {
-    return k_out < K ? (size_t)co * K + k_out : (size_t)cout * K + co;
-  };
-  if (c0 >= c1) {  // no positions in this range: zero partial sums
-    if (k_out <= K)
-      for (int co = 0; co < cout; ++co) out[out_index(co)] = 0.f;
-    return;
-  }
-  if (warp == 0) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
-                     tc_saddr(&tmem_holder)),
-                 "r"(kTcCols)
-                 : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-  }
-  if (tid == 0) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(tc_saddr(&bar)), "r"(1)
-                 : "memory");
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  }
-  const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(npad >> 3) << 17) |
-                         ((uint32_t)(kTcM >> 4) << 24);
-  const int j = tid & 63, half = tid >> 6;
-  bool ok = true;
-  uint32_t tmem = 0;
-  int ch = c0;
-  for (; ch < c1; ++ch) {
-    const int g = ch * kTcKc + j;
-    const bool valid = g < total;
-    const int b = valid ? g / kP : 0, p = valid ? g - b * kP : 0;
-    const int h = p / kW, c = p - h * kW;
-    const float *xb = x + (size_t)b * cin * kP;
-    // A: rows half * 64 .. + 63 at position column j.
-    int k = m0 + half * 64;
-    int ci = k / 9, t = k - 9 * ci;
-    for (int mm = 0; mm < 64; ++mm, ++k) {
-      float v = 0.f;
-      if (k < K) {
-        int dh, dc;
-        tap(t, dil, dh, dc);
-        const int hh = h + dh, cc = c + dc;
-        if (valid && hh >= 0 && hh < kH && cc >= 0 && cc < kW)
-          v = __ldg(xb + (size_t)ci * kP + hh * kW + cc);
-      } else if (k == K) {
-        v = valid ? 1.f : 0.f;
-      }
-      const __nv_bfloat16 vh = __float2bfloat16_rn(v);
-      const __nv_bfloat16 vl = __float2bfloat16_rn(v - __bfloat162float(vh));
-      *reinterpret_cast<__nv_bfloat16 *>(a_hi + tc_off(half * 64 + mm, j)) = vh;
-      *reinterpret_cast<__nv_bfloat16 *>(a_lo + tc_off(half * 64 + mm, j)) = vl;
-      if (++t == 9) {
-        t = 0;
-        ++ci;
-      }
-    }
-    // B: rows co = half, half + 2, ... at position column j.
-    for (int co = half; co < npad; co += 2) {
-      const float v =
-          (valid && co < cout) ? __ldg(dy + ((size_t)b * cout + co) * kP + p) : 0.f;
-      const __nv_bfloat16 vh = __float2bfloat16_rn(v);
-      const __nv_bfloat16 vl = __float2bfloat16_rn(v - __bfloat162float(vh));
-      *reinterpret_cast<__nv_bfloat16 *>(b_hi + tc_off(co, j)) = vh;
-      *reinterpret_cast<__nv_bfloat16 *>(b_lo + tc_off(co, j)) = vl;
-    }
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    tmem = tmem_holder;
-    if (tid == 0) {
-      for (int s = 0; s < kTcKc / 16; ++s) {
-        const uint32_t koff = s * 2 * kTcLBO;
-        const uint64_t ah = tc_desc(tc_saddr(a_hi) + koff), al = tc_desc(tc_saddr(a_lo) + koff);
-        const uint64_t bh = tc_desc(tc_saddr(b_hi) + koff), bl = tc_desc(tc_saddr(b_lo) + koff);
-        tc_mma(tmem, ah, bh, idesc, (ch > c0 || s > 0) ? 1u : 0u);
-        tc_mma(tmem, ah, bl, idesc, 1u);
-        tc_mma(tmem, al, bh, idesc, 1u);
-      }
-      asm volatile(
-          "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-              tc_saddr(&bar))
-          : "memory");
-    }
-    // The chunk's products must be done before its tiles are overwritten.
-    if (!tc_wait(tc_saddr(&bar), (uint32_t)((ch - c0) & 1))) ok = false;
-    if (__syncthreads_or(!ok)) {
-      ok = false;
-      break;
-    }
-  }
-  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  if (ok) {
-    for (int col = 0; col < npad; col += 16) {
-      uint32_t v[16];
-      const uint32_t ta = tmem + ((uint32_t)(32 * warp) << 16) + (uint32_t)col;
-      asm volatile(
-          "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,"
-          "%14,%15}, [%16];"
-          : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]),
-            "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]),
-            "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
-          : "r"(ta));
-      asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-      if (k_out <= K) {
+// Thread t < 200 owns position t: it gathers the 63 columns of a chunk for
+// its row of A (the tap offsets are per-thread addresses, the channel a
+// compile-time offset, so a column is one shared load), and later reads its
+// TMEM lane, adds the bias and the ReLU (or applies the ReLU mask) and
+// writes its column of the next tensor. Warp 7 streams the packed weights (a
+// ring of eight chunks, bulk copies) and issues the MMAs: two tiles of 128
+// rows, per 16 columns hi * W then lo * W. A has three stages, so that a
+// chunk's MMAs run under the next chunks' gathers. (Tiles straddling images,
+// gathered from global memory with the weights fetched element by element,
+// took 71 us a layer at 512 images.)
+constexpr int kImgThreads = 256, kImgRows = 7;  // 7 row warps
+struct ImageArgs {
+  int batch;
+  const float *x;
+  const unsigned char *packed;
+  const float *bias[kLayers];
+  float *misfit, *grad;                        // prediction, normalised units
+  // Prediction at states in physical units: x is [B][3][kP], coords the two
+  // coordinate channels, misfit m0 + ms m, gradient gs g.
+  const float *coords, *gs;
+  double m0, ms;
+  double *misfit_d;
+  const float *m_true, *g_true;                // training
+  float w_m, w_g;
+  double *loss;
+  uint32_t *xq, *act[3], *dq[4];               // split tensors for the weight gradients
+  int *err;
+};
+// ST stages of A (TMEM: D of the two row tiles, 64 columns each, then per
+// stage and tile the 32 columns of hi and of lo) and a ring of weights. With
+// at most one image per SM, three stages and one CTA per SM; with more
+// images, one stage and two CTAs per SM, which overlap each other's gather,
+// MMAs and epilogues (256 images, training: 139 us with one CTA per SM). The
+// CTAs of an SM never ask for more than its 512 columns, so no allocation
+// waits; the shared memory asked for sees to it.
+template <int ST>
+struct Img {
+  static constexpr int RING = ST > 1 ? 8 : 4, AHEAD = RING - 2;
+  static constexpr int COLS = ST > 1 ? 512 : 256;
+  static constexpr int USED = RING * 64 * kTcKc * 2 + 64 * kPW * 4 + 1024;
+  static constexpr int SMEM = ST > 1 ? 120 * 1024 : USED;
+  static_assert(USED <= SMEM && 128 + 128 * ST <= COLS, "one image");
+};
+constexpr int kImgW = 64 * kTcKc * 2, kImgACol = 128;
+
+struct ImageShared {
+  uint64_t full[3], done[3], w[8];
+  int2 chunk[64];  // offset and bytes of each chunk's weights
+  uint32_t tmem;
+  volatile int fail;
+  float red[256];
+  float y[4 * kP];
+};
+
+// TMEM columns of A: stage s, row tile m, hi; lo follows 32 columns on.
+__device__ __forceinline__ uint32_t a_col(uint32_t tmem, int s, int m) {
+  return tmem + kImgACol + 128u * s + 64u * m;
+}
+
+template <int REM>
+__device__ __forceinline__ void gather_chunk(const uint32_t *const src[9], uint32_t ta) {
+  constexpr int COLS = 9 * REM, GROUPS = (COLS + 15) / 16;
+  uint32_t w[16 * GROUPS];
 #pragma unroll
-        for (int q = 0; q < 16; ++q)
-          if (col + q < cout) out[out_index(col + q)] = __uint_as_float(v[q]);
-      }
+  for (int k = 0; k < 16 * GROUPS; ++k) w[k] = k < COLS ? src[k % 9][kPW * (k / 9)] : 0u;
+#pragma unroll
+  for (int g = 0; g < GROUPS; ++g) {
+    uint32_t h[8], l[8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      h[e] = __byte_perm(w[16 * g + 2 * e], w[16 * g + 2 * e + 1], 0x7632);
+      l[e] = __byte_perm(w[16 * g + 2 * e], w[16 * g + 2 * e + 1], 0x5410);
     }
-  } else if (tid == 0) {
-    atomicOr(err, 1);
-    // Bounded: give the products of the chunk that timed out more time to
-    // finish before the TMEM is freed.
-    tc_wait(tc_saddr(&bar), (uint32_t)((ch - c0) & 1));
+    tc_store<8>(ta + 8 * g, h);
+    tc_store<8>(ta + 32 + 8 * g, l);
+  }
+}
+
+// The row warps' part of step S: gather every chunk, then wait for the
+// products. n: chunks so far.
+template <int S, int ST>
+__device__ __forceinline__ void gather_step(ImageShared &sh, const uint32_t *act, uint32_t tmem,
+                                            int t, int &n) {
+  constexpr bool BWD = S >= kLayers;
+  constexpr int DIL = kDil[step_layer(S)], K = step_k(S);
+  constexpr int CHUNKS = step_chunks(S), REM = K - (CHUNKS - 1) * kTcCi;
+  const int h = t / kW, c = t - h * kW;
+  const uint32_t *src[9];
+#pragma unroll
+  for (int q = 0; q < 9; ++q) {
+    int dh, dc;
+    tap(q, DIL, dh, dc);
+    const int hh = BWD ? h - dh : h + dh, cc = BWD ? c - dc : c + dc;
+    const bool ok = t < kP && hh >= 0 && hh < kH && cc >= 0 && cc < kW;
+    src[q] = act + (ok ? hh * kW + cc : kP);
+  }
+  const uint32_t lanes = (uint32_t)(32 * ((t >> 5) & 3)) << 16;
+  for (int ch = 0; ch < CHUNKS; ++ch, ++n) {
+    const int s = n % ST;
+    if (n >= ST)
+      bar_wait(&sh.done[s], (uint32_t)(n / ST - 1) & 1u, &sh.fail);
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    __syncwarp();
+    const uint32_t ta = a_col(tmem, s, t >> 7) + lanes;
+    if (REM != kTcCi && ch == CHUNKS - 1)
+      gather_chunk<REM>(src, ta);
+    else
+      gather_chunk<kTcCi>(src, ta);
+#pragma unroll
+    for (int q = 0; q < 9; ++q) src[q] += kPW * kTcCi;
+    tc_stored();
+    __syncwarp();
+    if ((t & 31) == 0) bar_arrive(&sh.full[s]);
+  }
+  // The step's last commit covers all its products.
+  bar_wait(&sh.done[(n - 1) % ST], (uint32_t)((n - 1) / ST) & 1u, &sh.fail);
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+}
+
+// Warp 7: the weights of chunk q of the kernel's chunk list (one lane).
+template <int ST>
+__device__ __forceinline__ void load_weights(ImageShared &sh, const unsigned char *packed,
+                                             unsigned char *ring, int q, int total) {
+  if (q >= total) return;
+  const int2 c = sh.chunk[q];
+  bulk_load(ring + (q % Img<ST>::RING) * kImgW, packed + c.x, (uint32_t)c.y, &sh.w[q % Img<ST>::RING]);
+}
+
+// The MMAs of step S (the whole warp 7; one lane issues).
+template <int S, int ST>
+__device__ __forceinline__ void mma_step(ImageShared &sh, const unsigned char *packed,
+                                         unsigned char *ring, uint32_t tmem, int total, int &n) {
+  constexpr int CHUNKS = step_chunks(S), REM = step_k(S) - (CHUNKS - 1) * kTcCi;
+  const uint32_t idesc = tc_idesc(step_n(S));
+  for (int ch = 0; ch < CHUNKS; ++ch, ++n) {
+    const int s = n % ST, slot = n % Img<ST>::RING;
+    // The slot of the chunk loaded now held chunk n - 2: its products must be
+    // done. (With one stage they are: chunk n - 1 was gathered after them. A
+    // wait here could miss that phase, the barrier having gone two on.)
+    if (ST > 1 && n >= 2)
+      bar_wait(&sh.done[(n - 2) % ST], (uint32_t)((n - 2) / ST) & 1u, &sh.fail);
+    __syncwarp();
+    if (elect_one()) load_weights<ST>(sh, packed, ring, n + Img<ST>::AHEAD, total);
+    __syncwarp();
+    bar_wait(&sh.w[slot], (uint32_t)(n / Img<ST>::RING) & 1u, &sh.fail);
+    bar_wait(&sh.full[s], (uint32_t)(n / ST) & 1u, &sh.fail);
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    __syncwarp();
+    const uint32_t a = a_col(tmem, s, 0);
+    const uint64_t bd = tc_desc(tc_saddr(ring + slot * kImgW));
+    const int steps = ch == CHUNKS - 1 ? (9 * REM + 15) / 16 : 4;
+    if (elect_one()) {
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        if (k >= steps) break;
+        const uint64_t b = bd + (uint64_t)(k * 2 * kTcLBO >> 4);
+        // hi of both tiles, then lo: successive products do not share D.
+        const uint32_t acc = (ch > 0 || k > 0) ? 1u : 0u, ak = a + 8u * k;
+        tc_mma(tmem, ak, b, idesc, acc);
+        tc_mma(tmem + 64u, ak + 64u, b, idesc, acc);
+        tc_mma(tmem, ak + 32u, b, idesc, 1u);
+        tc_mma(tmem + 64u, ak + 96u, b, idesc, 1u);
+      }
+      tc_commit(tc_saddr(&sh.done[s]));
+    }
+    __syncwarp();
+  }
+}
+
+// Barrier of the row warps.
+__device__ __forceinline__ void rows_sync() {
+  asm volatile("barrier.sync 1, %0;" ::"n"(32 * kImgRows) : "memory");
+}
+
+// Epilogue of a hidden step: thread t's outputs into the image's tensor in
+// shared memory (and, for training, global memory). Forward: bias and ReLU;
+// backward: the ReLU mask of the layer's input activation.
+template <int S, bool TRAIN>
+__device__ __forceinline__ void finish_step(const ImageArgs &g, uint32_t *act, uint32_t tmem, int t,
+                                            int image) {
+  constexpr bool BWD = S >= kLayers;
+  constexpr int L = step_layer(S), N = BWD ? kCin[L] : kCout[L];
+  const uint32_t ta = tmem + ((uint32_t)(32 * ((t >> 5) & 3)) << 16) + 64u * (t >> 7);
+  uint32_t *out = !TRAIN ? nullptr : BWD ? g.dq[L - 1] : g.act[L < 3 ? L : 0];
+  const uint32_t *mask = BWD ? g.act[L - 1 < 3 ? (L > 0 ? L - 1 : 0) : 0] : nullptr;
+  const size_t at = (size_t)image * N * kPW + t;
+#pragma unroll
+  for (int c0 = 0; c0 < N; c0 += 16) {
+    uint32_t v[16], m[16];
+    if (BWD && t < kP)
+#pragma unroll
+      for (int j = 0; j < 16; ++j) m[j] = mask[at + (size_t)(c0 + j) * kPW];
+    tc_load16(ta + c0, v);
+    if (t >= kP) continue;
+#pragma unroll
+    for (int j = 0; j < 16; ++j) {
+      const int co = c0 + j;
+      float r = __uint_as_float(v[j]);
+      if (BWD)
+        r = (int)m[j] > 0 ? r : 0.f;
+      else
+        r = fmaxf(r + __ldg(g.bias[L] + co), 0.f);
+      const uint32_t w = split_word(r);
+      act[co * kPW + t] = w;
+      if (TRAIN) out[at + (size_t)co * kPW] = w;
+    }
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-  __syncthreads();
-  if (warp == 0)
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem),
-                 "r"(kTcCols)
-                 : "memory");
+  rows_sync();
 }
 
-__global__ void sum_chunks(size_t len, const float *__restrict__ partial, float *__restrict__ out) {
-  const size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
-  if (i >= len) return;
-  float s = 0.f;
-  for (int c = 0; c < kChunks; ++c) s += partial[(size_t)c * len + i];
-  out[i] = s;
-}
-
-// Fixed-order block sum of kThreads values.
-__device__ float block_sum(float v, float *red) {
-  red[threadIdx.x] = v;
-  __syncthreads();
-  for (int s = kThreads / 2; s > 0; s >>= 1) {
-    if ((int)threadIdx.x < s) red[threadIdx.x] += red[threadIdx.x + s];
-    __syncthreads();
+// Fixed-order sum over 256 values, the row warps' 224 and zeros.
+__device__ float rows_sum(float v, float *red, int t) {
+  red[t] = v;
+  if (t < 32) red[32 * kImgRows + t] = 0.f;
+  rows_sync();
+  for (int s = 128; s > 0; s >>= 1) {
+    if (t < s) red[t] += red[t + s];
+    rows_sync();
   }
   const float r = red[0];
-  __syncthreads();
+  rows_sync();
   return r;
 }
 
-__device__ float misfit_of(const float *yb, float *red) {
+template <bool TRAIN, int ST>
+__global__ void __launch_bounds__(kImgThreads, ST > 1 ? 1 : 2) net_images(const ImageArgs g) {
+  extern __shared__ __align__(1024) unsigned char smem[];
+  __shared__ ImageShared sh;
+  unsigned char *const base = smem + (1024 - (tc_saddr(smem) & 1023)) % 1024;
+  unsigned char *const ring = base;
+  uint32_t *const act = reinterpret_cast<uint32_t *>(ring + Img<ST>::RING * kImgW);
+  const int t = threadIdx.x, image = blockIdx.x;
+  constexpr int STEPS = TRAIN ? kSteps : kLayers;
+  int total = 0;
+#pragma unroll
+  for (int s = 0; s < STEPS; ++s) total += step_chunks(s);
+  if (t == 0) {
+    sh.fail = 0;
+    for (int i = 0; i < ST; ++i) {
+      bar_init(&sh.full[i], kImgRows);
+      bar_init(&sh.done[i], 1);
+    }
+    for (int i = 0; i < Img<ST>::RING; ++i) bar_init(&sh.w[i], 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (t >= 32 * kImgRows) tc_alloc(&sh.tmem, Img<ST>::COLS);
+  if (t < total) {
+    int s = 0, c = t, o = 0;
+    while (c >= step_chunks(s)) {
+      c -= step_chunks(s);
+      o += step_bytes(s++);
+    }
+    const int bytes = step_n(s) * kTcKc * 2;
+    sh.chunk[t] = make_int2(o + c * bytes, bytes);
+  }
+  // The image's features, split; zeros past each channel.
+  for (int i = t; i < 64 * kPW; i += kImgThreads) {
+    const int c = i / kPW, p = i - c * kPW;
+    uint32_t w = 0;
+    if (c < layer_cin(0) && p < kP) {
+      const float *from = !TRAIN && g.coords
+                              ? (c < 3 ? g.x + ((size_t)image * 3 + c) * kP : g.coords + (c - 3) * kP)
+                              : g.x + ((size_t)image * layer_cin(0) + c) * kP;
+      w = split_word(__ldg(from + p));
+      if (TRAIN) g.xq[((size_t)image * layer_cin(0) + c) * kPW + p] = w;
+    }
+    act[i] = w;
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem = sh.tmem;
+  int n = 0;
+  if (t >= 32 * kImgRows) {
+    if (elect_one())
+      for (int q = 0; q < Img<ST>::AHEAD; ++q) load_weights<ST>(sh, g.packed, ring, q, total);
+    __syncwarp();
+    mma_step<0, ST>(sh, g.packed, ring, tmem, total, n);
+    mma_step<1, ST>(sh, g.packed, ring, tmem, total, n);
+    mma_step<2, ST>(sh, g.packed, ring, tmem, total, n);
+    mma_step<3, ST>(sh, g.packed, ring, tmem, total, n);
+    if (TRAIN) {
+      mma_step<4, ST>(sh, g.packed, ring, tmem, total, n);
+      mma_step<5, ST>(sh, g.packed, ring, tmem, total, n);
+      mma_step<6, ST>(sh, g.packed, ring, tmem, total, n);
+    }
+  } else {
+    gather_step<0, ST>(sh, act, tmem, t, n);
+    finish_step<0, TRAIN>(g, act, tmem, t, image);
+    gather_step<1, ST>(sh, act, tmem, t, n);
+    finish_step<1, TRAIN>(g, act, tmem, t, image);
+    gather_step<2, ST>(sh, act, tmem, t, n);
+    finish_step<2, TRAIN>(g, act, tmem, t, image);
+    gather_step<3, ST>(sh, act, tmem, t, n);
+    // Head: gradient map = channels 0 .. 2, misfit = sum of channel 3.
+    uint32_t v[16];
+    tc_load16(tmem + ((uint32_t)(32 * ((t >> 5) & 3)) << 16) + 64u * (t >> 7), v);
+    float y[4];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) y[c] = __uint_as_float(v[c]) + __ldg(g.bias[3] + c);
+    const float m = rows_sum(t < kP ? y[3] : 0.f, sh.red, t);
+    if (!TRAIN) {
+      if (t < kP)
+        for (int c = 0; c < 3; ++c)
+          g.grad[((size_t)image * 3 + c) * kP + t] =
+              g.coords ? __fmul_rn(__ldg(g.gs + c * kP + t), y[c]) : y[c];
+      if (t == 0) {
+        if (g.coords)
+          g.misfit_d[image] = __dadd_rn(g.m0, __dmul_rn(g.ms, (double)m));
+        else
+          g.misfit[image] = m;
+      }
+    } else {
+      // Loss = w_m mean_b (m - m*)^2 + w_g mean_{b,c,p} (g - g*)^2 and its
+      // gradient with respect to the head's inputs. (The squares are summed
+      // in the order of 256 threads striding over [3][200].)
+      const float dm = m - g.m_true[image], ng = (float)g.batch * 3 * kP;
+      if (t < kP) {
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          const float diff = y[c] - g.g_true[((size_t)image * 3 + c) * kP + t];
+          sh.y[c * kP + t] = diff * diff;
+          y[c] = 2.f * g.w_g * diff / ng;
+        }
+        y[3] = 2.f * g.w_m * dm / (float)g.batch;
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          const uint32_t w = split_word(y[c]);
+          act[c * kPW + t] = w;
+          g.dq[3][((size_t)image * 4 + c) * kPW + t] = w;
+        }
+      }
+      rows_sync();
+      // Threads 224 .. 255 of that order are summed by the first warp.
+      auto strided = [&](int k) {
+        float s = 0.f;
+        for (int i = k; i < 3 * kP; i += 256) s += sh.y[i];
+        return s;
+      };
+      sh.red[t] = strided(t);
+      if (t < 32) sh.red[32 * kImgRows + t] = strided(32 * kImgRows + t);
+      rows_sync();
+      for (int s = 128; s > 0; s >>= 1) {
+        if (t < s) sh.red[t] += sh.red[t + s];
+        rows_sync();
+      }
+      if (t == 0)
+        g.loss[image] = (double)g.w_m * dm * dm / g.batch + (double)g.w_g * sh.red[0] / ng;
+      rows_sync();
+      gather_step<4, ST>(sh, act, tmem, t, n);
+      finish_step<4, TRAIN>(g, act, tmem, t, image);
+      gather_step<5, ST>(sh, act, tmem, t, n);
+      finish_step<5, TRAIN>(g, act, tmem, t, image);
+      gather_step<6, ST>(sh, act, tmem, t, n);
+      finish_step<6, TRAIN>(g, act, tmem, t, image);
+    }
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (t == 0 && sh.fail) {
+    atomicOr(g.err, 1);
+    // Bounded: give products in flight more time before the TMEM is freed.
+    sh.fail = 0;
+    bar_wait(&sh.done[0], 0u, &sh.fail);
+  }
+  __syncthreads();
+  if (t >= 32 * kImgRows) tc_dealloc(tmem, Img<ST>::COLS);
+}
+
+// ---- tensor-core weight gradients --------------------------------------------
+//
+// dW[co][k] = sum_pos dy[pos][co] X[pos][k] and db[co] = sum_pos dy[pos][co]
+// as a GEMM whose reduction runs over the positions of the batch's images:
+// D[k][co] (M = 128 rows of k = ci * 9 + tap per CTA, the bias as row
+// k = cin * 9 with X = 1). Both operands are split pairs; hi.hi + hi.lo +
+// lo.hi per 16 positions carry the products to about 2^-16 relative.
+// blockIdx.x is a tile of rows of one layer, blockIdx.y one of kChunks ranges
+// of images, whose partial sums sum_partials adds in order (deterministic).
+// Per image the tile's channels (with a border of zeros, so that a tap is an
+// offset) and dy go to shared memory; the next image's words are loaded into
+// registers meanwhile. Thread t builds row t % 128 of A: a position is a
+// compile-time offset, one shared load; positions run in chunks of 64 (the
+// last 16) through two stages, so that a chunk's MMAs run under the next
+// chunk's gather. Gathering every element from global memory with two-byte
+// shared stores took 780 us a layer at 512 images.
+constexpr int kWgThreads = 256;
+// (Row and channel pitches that spread a warp's 32 rows, three or four
+// channels of nine taps 1, 2 or 4 apart, over the banks.)
+constexpr int kPadW = kW + 9, kPadH = kH + 8, kPadP = kPadW * kPadH + 1, kDyP = 209;
+constexpr int kWgStage = 2 * 64 * kTcKc * 2;  // B hi, lo
+// TMEM: D (64 columns), then per stage 32 columns of A's hi and of its lo.
+constexpr int kWgCols = 256, kWgACol = 64;
+constexpr int kWgSmem = 2 * kWgStage + 16 * kPadP * 4 + 64 * kDyP * 4 + 1024;
+static_assert(kWgSmem > 114 * 1024, "one CTA per SM: its TMEM columns are then free");
+constexpr int kWgTiles[kLayers] = {1, 3, 5, 5};  // ceil((cin * 9 + 1) / 128)
+
+struct WeightArgs {
+  int batch;
+  const uint32_t *x[kLayers], *dy[kLayers];
+  float *partial;  // [kChunks][num_params]
+  size_t len;      // num_params
+  size_t off[kLayers];
+  int *err;
+};
+struct WeightShared {
+  uint64_t done[2];
+  uint32_t tmem;
+  volatile int fail;
+};
+
+// Groups G0 .. G0 + NG - 1 (eight positions each, 64 Q + 8 g + e) of chunk Q
+// of a row, as hi and lo pairs.
+template <int Q, int G0, int NG, bool PAD>
+__device__ __forceinline__ void weight_row(const uint32_t *src, uint32_t h[4 * NG],
+                                           uint32_t l[4 * NG]) {
+  uint32_t w[8 * NG];
+#pragma unroll
+  for (int i = 0; i < 8 * NG; ++i) {
+    const int p = 64 * Q + 8 * G0 + i;
+    w[i] = p < kP ? src[PAD ? (p / kW) * kPadW + p % kW : p] : 0u;
+  }
+#pragma unroll
+  for (int i = 0; i < 4 * NG; ++i) {
+    h[i] = __byte_perm(w[2 * i], w[2 * i + 1], 0x7632);
+    l[i] = __byte_perm(w[2 * i], w[2 * i + 1], 0x5410);
+  }
+}
+// The same into B's row at hi, lo.
+template <int Q, int G0, int NG>
+__device__ __forceinline__ void weight_row_b(const uint32_t *src, unsigned char *hi,
+                                             unsigned char *lo) {
+  uint32_t h[4 * NG], l[4 * NG];
+  weight_row<Q, G0, NG, false>(src, h, l);
+#pragma unroll
+  for (int g = 0; g < NG; ++g) {
+    *reinterpret_cast<uint4 *>(hi + (G0 + g) * kTcLBO) =
+        make_uint4(h[4 * g], h[4 * g + 1], h[4 * g + 2], h[4 * g + 3]);
+    *reinterpret_cast<uint4 *>(lo + (G0 + g) * kTcLBO) =
+        make_uint4(l[4 * g], l[4 * g + 1], l[4 * g + 2], l[4 * g + 3]);
+  }
+}
+
+template <int L>
+__device__ void weight_tile(const WeightArgs &g, WeightShared &sh, unsigned char *base, int mtile) {
+  constexpr int CIN = kCin[L], COUT = kCout[L], DIL = kDil[L], K = CIN * 9;
+  constexpr int NPAD = COUT < 16 ? 16 : COUT, NCH = CIN < 16 ? CIN : 16;
+  const int t = threadIdx.x;
+  const int b0 = (int)((long long)g.batch * blockIdx.y / gridDim.y);
+  const int b1 = (int)((long long)g.batch * (blockIdx.y + 1) / gridDim.y);
+  const int m0 = mtile * kTcM, ci0 = m0 / 9 < CIN - NCH ? m0 / 9 : CIN - NCH;
+  float *const out = g.partial + (size_t)blockIdx.y * g.len + g.off[L];
+  uint32_t *const xs = reinterpret_cast<uint32_t *>(base + 2 * kWgStage);
+  uint32_t *const ds = xs + 16 * kPadP;
+  for (int i = t; i < 16 * kPadP; i += kWgThreads) xs[i] = 0;
+  for (int i = t; i < 64 * kDyP; i += kWgThreads) ds[i] = 0;
+  // Row t % 128 of A, the half of its groups given by t / 128; row t % 64 of
+  // B, a quarter of its groups.
+  const int k = m0 + (t & 127), part = t >> 7;
+  const int ci = k / 9, tp = k - 9 * ci;
+  int dh, dc;
+  tap(tp, DIL, dh, dc);
+  const uint32_t *const src =
+      xs + (k < K ? (ci - ci0) * kPadP + (4 + dh) * kPadW + 4 + dc : 0);
+  const int co = t & 63, quarter = t >> 6;
+  const uint32_t *const dsrc = ds + co * kDyP;
+  const uint32_t lanes = (uint32_t)(32 * ((t >> 5) & 3)) << 16;
+  const int brow = (co >> 3) * kTcSBO + (co & 7) * 16;
+  const uint32_t idesc = tc_idesc(NPAD), tmem = sh.tmem;
+  // Thread t < 200 carries position t of every channel.
+  uint32_t px[NCH], pd[COUT];
+  auto fetch = [&](int b) {
+    if (t >= kP) return;
+    const uint32_t *x = g.x[L] + ((size_t)b * CIN + ci0) * kPW + t;
+    const uint32_t *d = g.dy[L] + (size_t)b * COUT * kPW + t;
+#pragma unroll
+    for (int c = 0; c < NCH; ++c) px[c] = __ldg(x + c * kPW);
+#pragma unroll
+    for (int c = 0; c < COUT; ++c) pd[c] = __ldg(d + c * kPW);
+  };
+  uint32_t *const xo = xs + (t / kW + 4) * kPadW + t % kW + 4;
+  if (b0 < b1) fetch(b0);
+  int n = 0;
+  auto chunk = [&](auto build, int steps, bool first) {
+    const int s = n & 1;
+    if (n >= 2) bar_wait(&sh.done[s], (uint32_t)((n >> 1) - 1) & 1u, &sh.fail);
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    __syncwarp();
+    unsigned char *const bh = base + s * kWgStage, *const bl = bh + 64 * kTcKc * 2;
+    const uint32_t a = tmem + kWgACol + 64u * s;
+    build(a + lanes, bh + brow, bl + brow);
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    tc_stored();
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    if (t < 32 && elect_one()) {
+      const uint64_t dh_ = tc_desc(tc_saddr(bh)), dl_ = tc_desc(tc_saddr(bl));
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        if (q >= steps) break;
+        const uint64_t ko = (uint64_t)(q * 2 * kTcLBO >> 4);
+        const uint32_t ah = a + 8u * q, al = ah + 32u;
+        tc_mma(tmem, ah, dh_ + ko, idesc, (first && q == 0) ? 0u : 1u);
+        tc_mma(tmem, ah, dl_ + ko, idesc, 1u);
+        tc_mma(tmem, al, dh_ + ko, idesc, 1u);
+      }
+      tc_commit(tc_saddr(&sh.done[s]));
+    }
+    ++n;
+  };
+  __syncthreads();
+  for (int b = b0; b < b1; ++b) {
+    if (t < kP) {
+#pragma unroll
+      for (int c = 0; c < NCH; ++c) xo[c * kPadP] = px[c];
+#pragma unroll
+      for (int c = 0; c < COUT; ++c) ds[c * kDyP + t] = pd[c];
+    }
+    __syncthreads();
+    if (b + 1 < b1) fetch(b + 1);
+    const bool first = b == b0;
+    // NA groups of the row for each half, NB of B's row for each quarter. Rows
+    // past the weights hold ones (the bias row, at valid positions) or zeros.
+#define PSV_CHUNK(Q, NA, NB)                                                              \
+  chunk(                                                                                  \
+      [&](uint32_t ta, unsigned char *bh, unsigned char *bl) {                            \
+        uint32_t h[4 * NA], l[4 * NA];                                                    \
+        if (part == 0)                                                                    \
+          weight_row<Q, 0, NA, true>(src, h, l);                                          \
+        else                                                                              \
+          weight_row<Q, NA, NA, true>(src, h, l);                                         \
+        if (k >= K) {                                                                     \
+          _Pragma("unroll") for (int i = 0; i < 4 * NA; ++i) {                            \
+            const int p = 64 * Q + 8 * NA * part + 2 * i;                                 \
+            h[i] = k == K && p < kP ? 0x3F803F80u : 0u;                                   \
+            l[i] = 0u;                                                                    \
+          }                                                                               \
+        }                                                                                 \
+        __syncwarp();                                                                     \
+        if (NA == 4) {                                                                    \
+          tc_store<8>(ta + 16 * part, h);                                                 \
+          tc_store<8>(ta + 16 * part + 8, h + 8 * (NA / 4));                              \
+          tc_store<8>(ta + 32 + 16 * part, l);                                            \
+          tc_store<8>(ta + 32 + 16 * part + 8, l + 8 * (NA / 4));                         \
+        } else {                                                                          \
+          tc_store<4>(ta + 4 * part, h);                                                  \
+          tc_store<4>(ta + 32 + 4 * part, l);                                             \
+        }                                                                                 \
+        if (co < NPAD) {                                                                  \
+          if (quarter == 0) weight_row_b<Q, 0, NB>(dsrc, bh, bl);                         \
+          if (quarter == 1) weight_row_b<Q, NB, NB>(dsrc, bh, bl);                        \
+          if (quarter == 2 && Q < 3) weight_row_b<Q, 2 * NB, NB>(dsrc, bh, bl);           \
+          if (quarter == 3 && Q < 3) weight_row_b<Q, 3 * NB, NB>(dsrc, bh, bl);           \
+        }                                                                                 \
+        __syncwarp();                                                                     \
+      },                                                                                  \
+      Q < 3 ? 4 : 1, first && Q == 0)
+    PSV_CHUNK(0, 4, 2);
+    PSV_CHUNK(1, 4, 2);
+    PSV_CHUNK(2, 4, 2);
+    PSV_CHUNK(3, 1, 1);
+#undef PSV_CHUNK
+    // (The chunks' barriers have ordered every read of xs and ds before the
+    // next image's words.)
+  }
+  if (n) bar_wait(&sh.done[(n - 1) & 1], (uint32_t)((n - 1) >> 1) & 1u, &sh.fail);
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  // Row 32 w + lane of the accumulator is k; warps 4 - 7 have none.
+  if (t < kTcM) {
+#pragma unroll
+    for (int c0 = 0; c0 < NPAD; c0 += 16) {
+      uint32_t v[16];
+      tc_load16(tmem + ((uint32_t)(32 * (t >> 5)) << 16) + c0, v);
+      if (k <= K)
+#pragma unroll
+        for (int j = 0; j < 16; ++j)
+          if (c0 + j < COUT)
+            out[k < K ? (size_t)(c0 + j) * K + k : (size_t)COUT * K + c0 + j] =
+                n ? __uint_as_float(v[j]) : 0.f;
+    }
+  }
+}
+
+__global__ void __launch_bounds__(kWgThreads, 1) net_weights(const WeightArgs g) {
+  extern __shared__ __align__(1024) unsigned char smem[];
+  __shared__ WeightShared sh;
+  unsigned char *const base = smem + (1024 - (tc_saddr(smem) & 1023)) % 1024;
+  const int t = threadIdx.x;
+  if (t < 32) tc_alloc(&sh.tmem, kWgCols);
+  if (t == 0) {
+    sh.fail = 0;
+    for (int i = 0; i < 2; ++i) bar_init(&sh.done[i], 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const int x = blockIdx.x;
+  if (x < 5)
+    weight_tile<2>(g, sh, base, x);
+  else if (x < 10)
+    weight_tile<3>(g, sh, base, x - 5);
+  else if (x < 13)
+    weight_tile<1>(g, sh, base, x - 10);
+  else
+    weight_tile<0>(g, sh, base, x - 13);
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (t == 0 && sh.fail) {
+    atomicOr(g.err, 1);
+    sh.fail = 0;
+    bar_wait(&sh.done[0], 0u, &sh.fail);
+  }
+  __syncthreads();
+  if (t < 32) tc_dealloc(sh.tmem, kWgCols);
+}
+constexpr int kWgTileCount = 14;
+static_assert(kWgTiles[0] + kWgTiles[1] + kWgTiles[2] + kWgTiles[3] == kWgTileCount, "row tiles");
+
+__global__ void sum_partials(size_t len, const float *__restrict__ partial,
+                             float *__restrict__ out) {
+  const size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
+  if (i >= len) return;
   float s = 0.f;
-  for (int p = threadIdx.x; p < kP; p += kThreads) s += yb[3 * kP + p];
-  return block_sum(s, red);
-}
-
-// Loss = w_m mean_b (m - m*)^2 + w_g mean_{b,c,p} (g - g*)^2 and its
-// gradient with respect to the last layer's output.
-__global__ void __launch_bounds__(kThreads) head_loss(int batch, const float *__restrict__ y4,
-                                                      const float *__restrict__ m_true,
-                                                      const float *__restrict__ g_true, float w_m,
-                                                      float w_g, float *__restrict__ dy4,
-                                                      double *__restrict__ loss_part) {
-  __shared__ float red[kThreads];
-  const int b = blockIdx.x;
-  const float *yb = y4 + (size_t)b * 4 * kP;
-  const float m = misfit_of(yb, red);
-  const float dm = m - m_true[b];
-  const float ng = (float)batch * 3 * kP;
-  float lg = 0.f;
-  for (int i = threadIdx.x; i < 3 * kP; i += kThreads) {
-    const float diff = yb[i] - g_true[(size_t)b * 3 * kP + i];
-    lg += diff * diff;
-    dy4[(size_t)b * 4 * kP + i] = 2.f * w_g * diff / ng;
-  }
-  for (int p = threadIdx.x; p < kP; p += kThreads)
-    dy4[(size_t)b * 4 * kP + 3 * kP + p] = 2.f * w_m * dm / (float)batch;
-  lg = block_sum(lg, red);
-  if (threadIdx.x == 0)
-    loss_part[b] = (double)w_m * dm * dm / batch + (double)w_g * lg / ng;
-}
-
-__global__ void sum_loss(int n, const double *__restrict__ part, double *__restrict__ out) {
-  if (threadIdx.x == 0 && blockIdx.x == 0) {
-    double s = 0;
-    for (int i = 0; i < n; ++i) s += part[i];
-    *out = s;
-  }
-}
-
-__global__ void __launch_bounds__(kThreads) head_predict(const float *__restrict__ y4,
-                                                         float *__restrict__ misfit,
-                                                         float *__restrict__ grad) {
-  __shared__ float red[kThreads];
-  const int b = blockIdx.x;
-  const float *yb = y4 + (size_t)b * 4 * kP;
-  const float m = misfit_of(yb, red);
-  for (int i = threadIdx.x; i < 3 * kP; i += kThreads) grad[(size_t)b * 3 * kP + i] = yb[i];
-  if (threadIdx.x == 0) misfit[b] = m;
+#pragma unroll 8
+  for (int c = 0; c < kChunks; ++c) s += partial[(size_t)c * len + i];
+  out[i] = s;
 }
 
 __global__ void adam_step(size_t n, float *__restrict__ p, const float *__restrict__ g,
@@ -545,33 +897,55 @@ Net::Net(int device, int max_batch) : device_(device), max_batch_(max_batch) {
   DeviceGuard guard(device_);
   check(cudaStreamCreateWithFlags(&stream_, cudaStreamNonBlocking), "cudaStreamCreate");
   const size_t n = num_params();
-  params_.allocate(n * sizeof(float));
-  wbf_.allocate(n * sizeof(__nv_bfloat16));
-  grads_.allocate(n * sizeof(float));
-  adam_m_.allocate(n * sizeof(float));
-  adam_v_.allocate(n * sizeof(float));
-  size_t maxlen = 0;
-  for (int l = 0; l < kLayers; ++l) maxlen = std::max(maxlen, layer_size(l));
-  partials_.allocate(kChunks * maxlen * sizeof(float));
-  for (int l = 0; l < kLayers; ++l)
-    act_[l].allocate((size_t)max_batch * kCout[l] * kP * sizeof(float));
-  for (auto &d : dact_) d.allocate((size_t)max_batch * kMaxC * kP * sizeof(float));
-  loss_partials_.allocate((size_t)max_batch * sizeof(double));
-  loss_.allocate(sizeof(double));
-  err_.allocate(sizeof(int));
-  check(cudaMemset(err_.get(), 0, sizeof(int)), "err flag");
+  params_.allocate(n * sizeof(float), false);
+  wbf_.allocate(n * sizeof(__nv_bfloat16), false);
+  grads_.allocate(n * sizeof(float), false);
+  adam_m_.allocate(n * sizeof(float), false);
+  adam_v_.allocate(n * sizeof(float), false);
+  packed_.allocate(kPackedBytes, false);
+  partials_.allocate(kChunks * n * sizeof(float), false);
+  const size_t image = (size_t)max_batch * kPW * sizeof(uint32_t);
+  xq_.allocate(image * kCin[0], false);
+  for (int l = 0; l < 3; ++l) act_[l].allocate(image * kCout[l], false);
+  for (int l = 0; l < kLayers; ++l) dq_[l].allocate(image * kCout[l], false);
+  // Per-image losses, then the error flag: one copy back a call.
+  result_.allocate((size_t)(max_batch + 1) * sizeof(double), false);
+  result_h_.resize(max_batch + 1);
+  for (auto f : {net_images<true, 3>, net_images<false, 3>})
+    check(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, Img<3>::SMEM),
+          "smem");
+  for (auto f : {net_images<true, 1>, net_images<false, 1>})
+    check(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, Img<1>::SMEM),
+          "smem");
+  check(cudaDeviceGetAttribute(&sms_, cudaDevAttrMultiProcessorCount, device_), "SMs");
+  check(cudaFuncSetAttribute(net_weights, cudaFuncAttributeMaxDynamicSharedMemorySize, kWgSmem),
+        "smem");
+  // (The buffers were cleared on the legacy stream, for which stream_ does not
+  // wait.)
+  check(cudaStreamSynchronize(cudaStreamLegacy), "network");
 }
 
-// Raises when a tensor-core convolution's bounded wait for its products
-// timed out (the flag is cleared for the next call).
-void Net::check_error() {
+int *Net::err() { return reinterpret_cast<int *>(result_.as<double>() + max_batch_); }
+
+// Waits for the stream and returns the sum of the per-image losses. Raises
+// when a bounded wait of a kernel ran out (the flag is cleared for the next
+// call).
+double Net::collect(int batch) {
+  // (The losses lie before the flag; with none to read, only the flag comes.)
+  const int first = max_batch_ - batch;
+  check(cudaMemcpyAsync(result_h_.data() + first, result_.as<double>() + first,
+                        (size_t)(batch + 1) * sizeof(double), cudaMemcpyDeviceToHost, stream_),
+        "result");
+  check(cudaStreamSynchronize(stream_), "network");
   int flag = 0;
-  check(cudaMemcpyAsync(&flag, err_.get(), sizeof(int), cudaMemcpyDeviceToHost, stream_), "err");
-  check(cudaStreamSynchronize(stream_), "err");
+  std::memcpy(&flag, &result_h_[max_batch_], sizeof(int));
   if (flag) {
-    check(cudaMemsetAsync(err_.get(), 0, sizeof(int), stream_), "err");
+    check(cudaMemsetAsync(err(), 0, sizeof(int), stream_), "err");
     throw Error(PSV_ERR_CUDA, "a tensor-core convolution timed out waiting for its products");
   }
+  double loss = 0;
+  for (int i = 0; i < batch; ++i) loss += result_h_[first + i];
+  return loss;
 }
 
 Net::~Net() {
@@ -594,6 +968,15 @@ void Net::refresh_bf16() {
   const size_t n = num_params();
   to_bf16<<<blocks(n), 256, 0, stream_>>>(n, params_.as<float>(), wbf_.as<__nv_bfloat16>());
   check(cudaGetLastError(), "to_bf16");
+  repack();
+}
+
+void Net::repack() {
+  const int4 offs = make_int4((int)weight_offset(0), (int)weight_offset(1), (int)weight_offset(2),
+                              (int)weight_offset(3));
+  pack_weights<<<blocks(kPackedBytes / 2), 256, 0, stream_>>>(
+      wbf_.as<__nv_bfloat16>(), packed_.as<unsigned char>(), offs);
+  check(cudaGetLastError(), "pack weights");
 }
 
 void Net::set_params(const float *host) {
@@ -616,92 +999,103 @@ void Net::get_params(float *host) {
   check(cudaStreamSynchronize(stream_), "get params");
 }
 
-void Net::forward(int batch, const float *x) {
-  const float *in = x;
-  for (int l = 0; l < kLayers; ++l) {
-    const __nv_bfloat16 *w = wbf_.as<__nv_bfloat16>() + weight_offset(l);
-    const float *bias = params_.as<float>() + bias_offset(l);
-    float *out = act_[l].as<float>();
-    const int npad = std::max(16, (kCout[l] + 15) / 16 * 16);
-    const unsigned tiles = static_cast<unsigned>((batch * kP + kTcM - 1) / kTcM);
-    if (l + 1 < kLayers)
-      conv_tc<kFwdRelu><<<tiles, kTcThreads, 0, stream_>>>(
-          batch, kCin[l], kCout[l], npad, kDil[l], in, w, bias, nullptr, out, err_.as<int>());
-    else
-      conv_tc<kFwdLinear><<<tiles, kTcThreads, 0, stream_>>>(
-          batch, kCin[l], kCout[l], npad, kDil[l], in, w, bias, nullptr, out, err_.as<int>());
-    check(cudaGetLastError(), "conv forward");
-    in = out;
-  }
+// The arguments both kinds of call share.
+static ImageArgs image_args(int batch, const float *x, const unsigned char *packed,
+                            const float *params, int *err) {
+  ImageArgs g{};
+  g.batch = batch;
+  g.x = x;
+  g.packed = packed;
+  for (int l = 0; l < kLayers; ++l) g.bias[l] = params + bias_offset(l);
+  g.err = err;
+  return g;
 }
 
-double Net::backward(int batch, const float *x, const float *m_true, const float *g_true,
-                     float w_misfit, float w_grad) {
-  float *cur = dact_[0].as<float>(), *other = dact_[1].as<float>();
-  head_loss<<<batch, kThreads, 0, stream_>>>(batch, act_[kLayers - 1].as<float>(), m_true, g_true,
-                                             w_misfit, w_grad, cur, loss_partials_.as<double>());
-  sum_loss<<<1, 32, 0, stream_>>>(batch, loss_partials_.as<double>(), loss_.as<double>());
-  check(cudaGetLastError(), "head loss");
-  for (int l = kLayers - 1; l >= 0; --l) {
-    const float *in = l == 0 ? x : act_[l - 1].as<float>();
-    const int rows = kCin[l] * 9 + 1;  // weights of one output channel, then its bias
-    const unsigned mtiles = static_cast<unsigned>((rows + kTcM - 1) / kTcM);
-    conv_weight_tc<<<dim3(mtiles, kChunks), kTcThreads, 0, stream_>>>(
-        batch, kCin[l], kCout[l], std::max(16, (kCout[l] + 15) / 16 * 16), kDil[l], in, cur,
-        partials_.as<float>(), err_.as<int>());
-    const size_t len = layer_size(l);
-    sum_chunks<<<blocks(len), 256, 0, stream_>>>(len, partials_.as<float>(),
-                                                 grads_.as<float>() + weight_offset(l));
-    check(cudaGetLastError(), "conv backward weight");
-    if (l > 0) {
-      const unsigned tiles = static_cast<unsigned>((batch * kP + kTcM - 1) / kTcM);
-      conv_tc<kBwdData><<<tiles, kTcThreads, 0, stream_>>>(
-          batch, kCin[l], kCout[l], std::max(16, (kCin[l] + 15) / 16 * 16), kDil[l], cur,
-          wbf_.as<__nv_bfloat16>() + weight_offset(l), nullptr, act_[l - 1].as<float>(), other,
-          err_.as<int>());
-      check(cudaGetLastError(), "conv backward data");
-      std::swap(cur, other);
-    }
+template <bool TRAIN>
+static void launch_images(const ImageArgs &g, bool two_per_sm, cudaStream_t s) {
+  if (two_per_sm)
+    net_images<TRAIN, 1><<<g.batch, kImgThreads, Img<1>::SMEM, s>>>(g);
+  else
+    net_images<TRAIN, 3><<<g.batch, kImgThreads, Img<3>::SMEM, s>>>(g);
+}
+
+// Forward, loss and parameter gradient (into grads_), without waiting.
+void Net::gradient(int batch, const float *x, const float *m_true, const float *g_true,
+                   float w_misfit, float w_grad) {
+  ImageArgs g = image_args(batch, x, packed_.as<unsigned char>(), params_.as<float>(), err());
+  g.m_true = m_true;
+  g.g_true = g_true;
+  g.w_m = w_misfit;
+  g.w_g = w_grad;
+  g.loss = result_.as<double>() + (max_batch_ - batch);
+  g.xq = xq_.as<uint32_t>();
+  for (int l = 0; l < 3; ++l) g.act[l] = act_[l].as<uint32_t>();
+  for (int l = 0; l < kLayers; ++l) g.dq[l] = dq_[l].as<uint32_t>();
+  launch_images<true>(g, batch > sms_, stream_);
+  check(cudaGetLastError(), "network forward and input gradients");
+  WeightArgs w{};
+  w.batch = batch;
+  for (int l = 0; l < kLayers; ++l) {
+    w.x[l] = l == 0 ? xq_.as<uint32_t>() : act_[l - 1].as<uint32_t>();
+    w.dy[l] = dq_[l].as<uint32_t>();
+    w.off[l] = weight_offset(l);
   }
-  double loss = 0;
-  check(cudaMemcpyAsync(&loss, loss_.get(), sizeof(double), cudaMemcpyDeviceToHost, stream_),
-        "loss");
-  check(cudaStreamSynchronize(stream_), "backward");
-  check_error();
-  return loss;
+  w.partial = partials_.as<float>();
+  w.len = num_params();
+  w.err = err();
+  net_weights<<<dim3(kWgTileCount, kChunks), kWgThreads, kWgSmem, stream_>>>(w);
+  check(cudaGetLastError(), "weight gradients");
+  sum_partials<<<blocks(w.len), 256, 0, stream_>>>(w.len, partials_.as<float>(),
+                                                   grads_.as<float>());
+  check(cudaGetLastError(), "sum of partials");
 }
 
 void Net::predict(int batch, const float *x, float *misfit, float *grad) {
   check_batch(batch);
   DeviceGuard guard(device_);
-  forward(batch, x);
-  head_predict<<<batch, kThreads, 0, stream_>>>(act_[kLayers - 1].as<float>(), misfit, grad);
-  check(cudaGetLastError(), "head predict");
-  check(cudaStreamSynchronize(stream_), "predict");
-  check_error();
+  ImageArgs g = image_args(batch, x, packed_.as<unsigned char>(), params_.as<float>(), err());
+  g.misfit = misfit;
+  g.grad = grad;
+  launch_images<false>(g, batch > sms_, stream_);
+  check(cudaGetLastError(), "network forward");
+  collect(0);
+}
+
+void Net::predict_states(int batch, const float *z, const float *coords, double m0, double ms,
+                         const float *gs, double *misfit, float *grad) {
+  check_batch(batch);
+  DeviceGuard guard(device_);
+  ImageArgs g = image_args(batch, z, packed_.as<unsigned char>(), params_.as<float>(), err());
+  g.coords = coords;
+  g.m0 = m0;
+  g.ms = ms;
+  g.gs = gs;
+  g.misfit_d = misfit;
+  g.grad = grad;
+  launch_images<false>(g, batch > sms_, stream_);
+  check(cudaGetLastError(), "network forward");
+  collect(0);
 }
 
 double Net::loss_grad(int batch, const float *x, const float *m_true, const float *g_true,
                       float w_misfit, float w_grad, float *dparams_host) {
   check_batch(batch);
   DeviceGuard guard(device_);
-  forward(batch, x);
-  const double loss = backward(batch, x, m_true, g_true, w_misfit, w_grad);
-  if (dparams_host) {
+  gradient(batch, x, m_true, g_true, w_misfit, w_grad);
+  if (dparams_host)
     check(cudaMemcpyAsync(dparams_host, grads_.get(), num_params() * sizeof(float),
                           cudaMemcpyDeviceToHost, stream_),
           "grads");
-    check(cudaStreamSynchronize(stream_), "grads");
-  }
-  return loss;
+  return collect(batch);
 }
 
 double Net::train_step(int batch, const float *x, const float *m_true, const float *g_true,
                        float w_misfit, float w_grad, const Adam &opt) {
   check_batch(batch);
   DeviceGuard guard(device_);
-  forward(batch, x);
-  const double loss = backward(batch, x, m_true, g_true, w_misfit, w_grad);
+  gradient(batch, x, m_true, g_true, w_misfit, w_grad);
+  // (As before the update: a time-out leaves the parameters alone.)
+  const double loss = collect(batch);
   ++step_;
   const float bc1 = 1.f - std::pow(opt.beta1, (float)step_);
   const float bc2 = 1.f - std::pow(opt.beta2, (float)step_);
@@ -711,6 +1105,7 @@ double Net::train_step(int batch, const float *x, const float *m_true, const flo
                                             wbf_.as<__nv_bfloat16>(), opt.lr, opt.beta1, opt.beta2,
                                             opt.eps, bc1, bc2);
   check(cudaGetLastError(), "adam");
+  repack();
   return loss;
 }
 

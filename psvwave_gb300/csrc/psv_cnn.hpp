@@ -23,6 +23,7 @@
 #include <cuda_runtime.h>
 
 #include <cstddef>
+#include <vector>
 
 #include "psv_model.hpp"
 
@@ -34,8 +35,7 @@ constexpr int kLayers = 4;
 constexpr int kCin[kLayers] = {5, 32, 64, 64};
 constexpr int kCout[kLayers] = {32, 64, 64, 4};
 constexpr int kDil[kLayers] = {1, 2, 4, 1};
-constexpr int kMaxC = 64;
-constexpr int kChunks = 32;  // position ranges of the weight-gradient partial sums
+constexpr int kChunks = 32;  // image ranges of the weight-gradient partial sums
 
 // Parameter vector layout: for each layer, weights [cout][cin][3][3] then
 // bias [cout].
@@ -58,6 +58,10 @@ class Net {
   void get_params(float *host);
   // Inference: x [B][5][kP] -> misfit [B], gradient [B][3][kP] (device).
   void predict(int batch, const float *x, float *misfit, float *grad);
+  // The same at states z [B][3][kP] in physical units: the network sees z and
+  // coords [2][kP]; misfit = m0 + ms m (FP64), gradient = gs g (gs [3][kP]).
+  void predict_states(int batch, const float *z, const float *coords, double m0, double ms,
+                      const float *gs, double *misfit, float *grad);
   // Loss and parameter gradient (host, num_params floats) of a batch.
   double loss_grad(int batch, const float *x, const float *m_true, const float *g_true,
                    float w_misfit, float w_grad, float *dparams_host);
@@ -68,21 +72,23 @@ class Net {
   int max_batch() const { return max_batch_; }
 
  private:
-  void forward(int batch, const float *x);
-  double backward(int batch, const float *x, const float *m_true, const float *g_true,
-                  float w_misfit, float w_grad);
+  void gradient(int batch, const float *x, const float *m_true, const float *g_true,
+                float w_misfit, float w_grad);
+  double collect(int batch);
+  int *err();
+  void repack();
   void refresh_bf16();
   void check_batch(int batch) const;
 
-  int device_, max_batch_;
+  int device_, max_batch_, sms_ = 0;
   cudaStream_t stream_ = nullptr;
   int step_ = 0;
   DeviceBuffer params_, wbf_, grads_, partials_, adam_m_, adam_v_;
-  DeviceBuffer act_[kLayers];   // layer outputs [B][cout][kP] (post-ReLU for 1..3)
-  DeviceBuffer dact_[2];        // gradient scratch [B][kMaxC][kP]
-  DeviceBuffer loss_partials_, loss_;
-  DeviceBuffer err_;  // int, raised by a tensor-core convolution's bounded wait
-  void check_error();
+  DeviceBuffer packed_;         // weights as the MMAs read them
+  DeviceBuffer xq_, act_[3];    // features and activations, split, [B][c][208 words]
+  DeviceBuffer dq_[kLayers];    // gradients with respect to each layer's output, likewise
+  DeviceBuffer result_;         // per-image losses, then the kernels' error flag
+  std::vector<double> result_h_;
 };
 
 }  // namespace cnn

@@ -148,6 +148,20 @@ int psv_cnn_predict(psv_cnn *n, int batch, const float *x_dev, float *misfit_dev
   });
 }
 
+int psv_cnn_predict_states(psv_cnn *n, int batch, const float *z_dev, const float *coords_dev,
+                           double m0, double ms, const float *gs_dev, double *misfit_dev,
+                           float *grad_dev) {
+  return guarded([&] {
+    need(n, "network");
+    need(z_dev, "z");
+    need(coords_dev, "coords");
+    need(gs_dev, "gs");
+    need(misfit_dev, "misfit");
+    need(grad_dev, "grad");
+    n->impl.predict_states(batch, z_dev, coords_dev, m0, ms, gs_dev, misfit_dev, grad_dev);
+  });
+}
+
 int psv_cnn_loss_grad(psv_cnn *n, int batch, const float *x_dev, const float *m_true_dev,
                       const float *g_true_dev, float w_misfit, float w_grad, double *loss,
                       float *dparams) {

@@ -103,6 +103,25 @@ def test_loss_gradient_matches_oracle_ragged_batch():
         assert rel_l2(d[a:b], d_ref[a:b]) <= 1e-4, l
 
 
+@pytest.mark.parametrize("B", [1, 152, 153, 600])
+def test_predict_equals_its_pieces(B):
+    """predict runs states to physical outputs in one kernel: the values of
+    the features, the normalised network and the scaling apart, bit for bit,
+    below and above one image per SM and across max_batch."""
+    net = sg.SurrogateNet(max_batch=512, seed=6)
+    rng = np.random.default_rng(B)
+    gs = torch.tensor(rng.random((3, 20, 10)).astype(np.float32), device=DEV)
+    net.norm = {"m0": 3.25e5, "ms": 1.7e4, "gs": gs}
+    z = torch.tensor(rng.standard_normal((B, 3, 20, 10)).astype(np.float32), device=DEV)
+    m, g = net.predict(z)
+    mf, gf = net.predict_features(net.features(z))
+    assert m.dtype == torch.float64 and torch.equal(m, 3.25e5 + 1.7e4 * mf.double())
+    assert torch.equal(g, gs * gf)
+    # An image's result does not depend on the batch it came in.
+    m1, g1 = net.predict(z[-1:])
+    assert torch.equal(m1, m[-1:]) and torch.equal(g1, g[-1:])
+
+
 def test_adam_step_matches_oracle():
     net = sg.SurrogateNet(max_batch=8, seed=5)
     p0 = net.get_params().astype(np.float64)
