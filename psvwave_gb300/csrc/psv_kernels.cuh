@@ -231,21 +231,37 @@ __global__ void __launch_bounds__(256) velocity_step(Grid<T> g, InjArgs q) {
 }
 
 // rtf[r][it] = rtf[r][it-1] + dt * v / (dx * dz), serially in time per
-// receiver, as src/fdModel.cpp:582-595 accumulates it.
+// receiver, as src/fdModel.cpp:582-595 accumulates it. One CTA a series: its
+// threads form the terms, one of them adds them up in shared memory. Bound by
+// the latency of the chain of additions (one thread a series doing all of it
+// took 470 us per 1000 steps, most of it the divisions).
+constexpr int kSumChunk = 1024;
 template <typename T>
-__global__ void receiver_cumsum(int nr, int nt, int n_steps, double dt, double dxdz,
-                                const T *raw_x, const T *raw_z, double *rtf_x, double *rtf_z) {
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= 2 * nr) return;
-  const int r = k >> 1;
-  const T *raw = (k & 1) ? raw_z : raw_x;
-  double *out = ((k & 1) ? rtf_z : rtf_x) + (size_t)r * nt;
-  raw += (size_t)r * nt;
-  double acc = 0;
-  for (int it = 0; it < n_steps; ++it) {
-    const double term = dt * (double)raw[it] / dxdz;
-    acc = it == 0 ? term : acc + term;
-    out[it] = acc;
+__global__ void __launch_bounds__(256) receiver_cumsum(int nt, int n_steps, double dt, double dxdz,
+                                                       const T *raw_x, const T *raw_z,
+                                                       double *rtf_x, double *rtf_z) {
+  __shared__ double v[kSumChunk];
+  const int r = blockIdx.x >> 1, tid = threadIdx.x;
+  const T *raw = ((blockIdx.x & 1) ? raw_z : raw_x) + (size_t)r * nt;
+  double *out = ((blockIdx.x & 1) ? rtf_z : rtf_x) + (size_t)r * nt;
+  double acc = -0.0;  // adds to any first term without a trace
+  for (int base = 0; base < n_steps; base += kSumChunk) {
+    for (int i = tid; i < kSumChunk; i += blockDim.x)
+      v[i] = base + i < n_steps ? dt * (double)raw[base + i] / dxdz : 0.0;
+    __syncthreads();
+    if (tid == 0) {
+      const int n = min(kSumChunk, n_steps - base);
+      for (int i = 0; i < n; i += 8) {  // past n: zeros that nothing reads
+        double t[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) t[k] = v[i + k];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) v[i + k] = acc = acc + t[k];
+      }
+    }
+    __syncthreads();
+    for (int i = tid; i < kSumChunk && base + i < n_steps; i += blockDim.x) out[base + i] = v[i];
+    __syncthreads();
   }
 }
 
@@ -385,9 +401,8 @@ cudaError_t run_forward(const SolverArgs &a, const InjPlan &plan, int shot, bool
       return receiver_cumsum_f32(a.nr, a.nt, it1, a.dt, a.dx * a.dz, (const float *)e.rec_vx,
                                  (const float *)e.rec_vz, a.rtf_ux + off, a.rtf_uz + off, s);
     else
-      kern::receiver_cumsum<T><<<(2 * a.nr + 127) / 128, 128, 0, s>>>(
-          a.nr, a.nt, it1, a.dt, a.dx * a.dz, e.rec_vx, e.rec_vz, a.rtf_ux + off,
-          a.rtf_uz + off);
+      kern::receiver_cumsum<T><<<2 * a.nr, 256, 0, s>>>(a.nt, it1, a.dt, a.dx * a.dz, e.rec_vx,
+                                                        e.rec_vz, a.rtf_ux + off, a.rtf_uz + off);
   }
   return cudaGetLastError();
 }

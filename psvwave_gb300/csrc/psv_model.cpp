@@ -121,6 +121,7 @@ Model::Model(const Config &cfg, int precision, int device)
       variant_ = kFusedCluster;
     resident_on_ = resident_.ctas() > 0;
   }
+  if (prec_ == PSV_FP64) resident_on_ = resident64_.ctas() > 0;
   synchronize();
 }
 
@@ -325,6 +326,10 @@ void Model::build_plans() {
   plan_maps_.clear();
   plan_terms_.resize(n_shots + 1);
   plan_maps_.resize(n_shots + 1);
+  resident::Grid on_chip;
+  on_chip.nx = geo_.nx;
+  on_chip.nz = nz;
+  for (int r = 0; r < cfg_.nr; ++r) on_chip.receivers.push_back(ix_rec_[r] * nz + iz_rec_[r]);
   for (int p = 0; p <= n_shots; ++p) {
     std::vector<InjTerm> terms;
     auto add = [&](int cell, int field, int index, int kind, double coef, double div) {
@@ -390,6 +395,13 @@ void Model::build_plans() {
       plan.map = plan_maps_[p].as<int>();
     }
     plans_[p] = plan;
+    on_chip.sources.emplace_back();
+    for (const auto &t : terms) on_chip.sources.back().push_back(t.cell);
+  }
+  if (prec_ == PSV_FP64) {
+    resident64_ = resident64::plan(on_chip, dx, dz);
+    const size_t mail = resident64::mailbox_bytes(resident64_);
+    if (mail_.bytes() < mail) mail_.allocate(mail, false);
   }
 }
 
@@ -1668,9 +1680,16 @@ void Model::forward_simulate(int shot, bool store, bool verbose, bool output_wav
                      fields2_[4].get()};
   auto run = [&](int it0, int it1, bool zero, bool fin) {
     cudaError_t e;
-    if (prec_ == PSV_FP64)
-      e = forward_f64(a, plan, shot, store, it0, it1, zero, fin, stream());
-    else if (is_tma())
+    if (prec_ == PSV_FP64) {
+      e = cudaSuccess;
+      const bool on_chip = use_resident64() && it1 > it0;
+      if (on_chip)
+        e = resident64::steps(a, plan, resident64_, shot, false, it0, it1 - it0, zero, store,
+                              mail_.get(), err_flag_.as<int>(), stream());
+      if (e == cudaSuccess)
+        e = forward_f64(a, plan, shot, store, on_chip ? it1 : it0, it1, zero && !on_chip, fin,
+                        stream());
+    } else if (is_tma())
       e = tma_forward(shot, store, it0, it1, zero, fin, nullptr);
     else if (variant_ == kFused)
       e = fast::forward(a, second, &cur_, plan, shot, store, it0, it1, zero, fin, stream());
@@ -1692,7 +1711,7 @@ void Model::forward_simulate(int shot, bool store, bool verbose, bool output_wav
     run(n_steps, n_steps, false, true);
   }
   finish("forward_simulate");
-  if (!async_ && is_tma()) check_device_error();
+  if (!async_ && (is_tma() || use_resident64())) check_device_error();
   if (verbose) {
     synchronize();
     double s = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
@@ -1807,7 +1826,10 @@ void Model::adjoint_simulate(int shot, bool verbose) {
   run_loop(1, shot, true, cfg_.nt, [&] {
     cudaError_t e;
     if (prec_ == PSV_FP64) {
-      e = adjoint_f64(a, plans_[cfg_.n_shots], shot, stream());
+      e = use_resident64()
+              ? resident64::steps(a, plans_[cfg_.n_shots], resident64_, shot, true, cfg_.nt - 1,
+                                  cfg_.nt, true, false, mail_.get(), err_flag_.as<int>(), stream())
+              : adjoint_f64(a, plans_[cfg_.n_shots], shot, stream());
       cur_ = 0;
     } else if (is_tma()) {
       e = tma_adjoint(shot);
@@ -1820,7 +1842,7 @@ void Model::adjoint_simulate(int shot, bool verbose) {
     cuda_check(e, "adjoint_simulate");
   });
   finish("adjoint_simulate");
-  if (!async_ && is_tma()) check_device_error();
+  if (!async_ && (is_tma() || use_resident64())) check_device_error();
   if (verbose) {
     synchronize();
     double s = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();

@@ -16,6 +16,7 @@
 #include "psv_solver.hpp"
 #include "psv_exact_tma.hpp"
 #include "psv_resident.hpp"
+#include "psv_resident_f64.hpp"
 #include "psv_tma.hpp"
 
 namespace psv {
@@ -228,6 +229,8 @@ class Model {
     return resident_.ctas() > 0 && (variant_ == kFusedCluster || resident_on_);
   }
   resident::Grid resident_grid() const;
+  resident64::Plan resident64_;  // FP64 models'
+  bool use_resident64() const { return resident64_.ctas() > 0 && resident_on_; }
   DeviceBuffer mail_;  // resident scheme: mailboxes between CTAs
   static constexpr double kClusterCells = 1.0e5;  // variant kFusedCluster by default up to this size
   int cur_ = 0;  // fused variants: 0 = fields_ hold the current state, 1 = fields2_

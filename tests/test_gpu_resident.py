@@ -119,3 +119,33 @@ def test_resident_multi_shot_gradient_equals_serial_calls():
     b.map_kernels_to_velocity()
     assert a.misfit == b.misfit
     assert np.array_equal(a.get_gradient_vector(), b.get_gradient_vector())
+
+
+# One to four rows a thread, uneven tiles, the largest that fits and the first
+# that does not.
+SIZES_F64 = [(20, 16), (17, 23), (64, 66), (250, 151), (96, 305), (31, 700), (400, 300),
+             (401, 430), (520, 600)]
+
+
+@pytest.mark.parametrize("nx,nz", SIZES_F64)
+def test_resident_fp64_equals_two_kernel_steps_bit_for_bit(nx, nz, tmp_path, monkeypatch):
+    monkeypatch.chdir(tmp_path)
+    out = []
+    for variant in ("two_kernel", None, "pieces"):
+        m = model(nx, nz, nt=70, precision="fp64")
+        if variant == "two_kernel":
+            m.kernel_variant = variant
+        # Twice: eagerly and captured.
+        for _ in range(2):
+            m.forward_simulate(0, True, output_wavefields=variant == "pieces")
+        assert m.kernel_variant == "two_kernel"
+        fields = m.get_wavefields()
+        m.calculate_l2_misfit()
+        m.calculate_l2_adjoint_sources()
+        m.reset_kernels()
+        for _ in range(2):
+            m.adjoint_simulate(0)
+        out.append(m.get_synthetic_data() + fields + m.get_snapshots() + m.get_lame_kernels() +
+                   m.get_wavefields())
+    for steps, resident, pieces in zip(*out):
+        assert np.array_equal(resident, steps) and np.array_equal(pieces, steps)
