@@ -33,6 +33,7 @@ UNITS = [
     ("psv_tma_f32.cu", []),
     ("psv_exact_tma.cu", []),
     ("psv_resident_f32.cu", []),
+    ("psv_resident_exact.cu", []),
     ("psv_resident_f64.cu", ["-fmad=false"]),
     ("psv_aux.cu", ["-fmad=false"]),
     ("psv_noalloc.cu", []),

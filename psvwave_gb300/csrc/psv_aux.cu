@@ -68,15 +68,36 @@ __global__ void lame_to_velocity(size_t n, const double *vp, const double *vs,
   }
 }
 
-__global__ void reverse_residual_sum(int rows, int nt, double dt, double dxdz, const double *syn,
-                                     const double *obs, double *adj) {
-  const int r = blockIdx.x * blockDim.x + threadIdx.x;
-  if (r >= rows) return;
-  const size_t off = (size_t)r * nt;
+// adj[r][n] = dt / dxdz * (sum of dt (syn - obs) from nt - 1 down to n), serially
+// in time. One CTA a series: its threads form the terms, one of them adds
+// them up in shared memory (one thread a series doing all of it waited for
+// two loads at every step).
+__global__ void __launch_bounds__(256) reverse_residual_sum(int nt, double dt, double dxdz,
+                                                            const double *syn, const double *obs,
+                                                            double *adj) {
+  constexpr int kChunk = 1024;
+  __shared__ double v[kChunk];
+  const size_t off = (size_t)blockIdx.x * nt;
+  const int tid = threadIdx.x;
   double acc = 0;
-  for (int n = nt - 1; n >= 0; --n) {
-    acc += dt * (syn[off + n] - obs[off + n]);
-    adj[off + n] = dt / dxdz * acc;
+  for (int end = nt; end > 0; end -= kChunk) {
+    const int n = min(kChunk, end);  // steps end - 1 down to end - n
+    for (int i = tid; i < kChunk; i += blockDim.x) {
+      const size_t o = off + end - 1 - i;
+      v[i] = i < n ? dt * (syn[o] - obs[o]) : 0.0;
+    }
+    __syncthreads();
+    if (tid == 0)
+      for (int i = 0; i < n; i += 8) {  // past n: zeros that nothing reads
+        double t[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) t[k] = v[i + k];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) v[i + k] = acc = acc + t[k];
+      }
+    __syncthreads();
+    for (int i = tid; i < n; i += blockDim.x) adj[off + end - 1 - i] = dt / dxdz * v[i];
+    __syncthreads();
   }
 }
 
@@ -104,7 +125,7 @@ unsigned blocks_for(size_t n) {
 cudaError_t exact_receiver_terms(int rows, int nt, double dt, double dxdz, const double *syn,
                                  const double *obs, double *adj, cudaStream_t s) {
   if (rows <= 0) return cudaSuccess;
-  reverse_residual_sum<<<(rows + 127) / 128, 128, 0, s>>>(rows, nt, dt, dxdz, syn, obs, adj);
+  reverse_residual_sum<<<rows, 256, 0, s>>>(nt, dt, dxdz, syn, obs, adj);
   return cudaGetLastError();
 }
 

@@ -507,6 +507,7 @@ void Model::build_descs() {
   }
   descs_h_ = std::move(descs);
   resident_ = resident::plan(resident_grid());
+  exact_plans_.clear();
   const size_t mail = resident::mailbox_bytes(resident_);
   if (mail_.bytes() < mail) mail_.allocate(mail, false);
   tma_ok_ = true;
@@ -597,6 +598,43 @@ cudaError_t Model::tma_adjoint(int shot) {
   return cudaGetLastError();
 }
 
+resident::ExactPlan Model::exact_plan(int lanes) const {
+  auto it = exact_plans_.find(lanes);
+  if (it == exact_plans_.end())
+    it = exact_plans_.emplace(lanes, resident::plan_exact(resident_grid(), lanes)).first;
+  return it->second;
+}
+
+// Lanes of an exact gradient resident on chip, and their plan (none: it does not
+// fit): as many as shots, up to kMaxExactLanes, that have room on the device and
+// in 60 % of its free memory.
+int Model::exact_resident_lanes(int C, int n_list, resident::ExactPlan *plan) const {
+  *plan = resident::ExactPlan();
+  if (!use_resident()) return 0;
+  DeviceGuard guard(device_);
+  size_t free_b = 0, total_b = 0;
+  if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) free_b = 0;
+  for (const auto &l : lanes_) free_b += l->bytes();
+  for (int lanes = std::max(1, std::min(n_list, kMaxExactLanes)); lanes >= 1; --lanes) {
+    const resident::ExactPlan p = exact_plan(lanes);
+    if (p.p.ctas() <= 0) continue;
+    if (lanes > 1 && static_cast<double>(lanes) * exact_resident_bytes(C, p) > 0.6 * free_b) continue;
+    *plan = p;
+    return lanes;
+  }
+  return 0;
+}
+
+size_t Model::exact_resident_bytes(int C, const resident::ExactPlan &p) const {
+  const int nt = cfg_.nt;
+  if (C <= 0 || C > nt) C = nt;
+  const size_t state = 5 * padded_size() * sizeof(float);
+  const size_t n_ck = (nt + C - 1) / C;
+  return n_ck * state + C * p.rate_stride * sizeof(float2) + state +
+         3 * padded_size() * sizeof(float) +
+         2 * static_cast<size_t>(cfg_.nr) * nt * sizeof(float) + resident::mailbox_bytes(p.p);
+}
+
 size_t Model::exact_lane_bytes(int C) const {
   const int nt = cfg_.nt;
   if (C <= 0 || C > nt) C = nt;
@@ -613,8 +651,7 @@ int Model::exact_lane_count(int C, int n_list) const {
   size_t free_b = 0, total_b = 0;
   if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) return 1;
   for (const auto &l : lanes_)
-    free_b += l->ckpt.bytes() + l->slots.bytes() + l->lam.bytes() + l->raw.bytes() +
-              l->part.bytes();
+    free_b += l->bytes();
   const size_t per = std::max<size_t>(exact_lane_bytes(C), 1);
   const size_t fit = static_cast<size_t>(0.6 * static_cast<double>(free_b)) / per;
   return static_cast<int>(std::max<size_t>(1, std::min<size_t>(
@@ -624,6 +661,12 @@ int Model::exact_lane_count(int C, int n_list) const {
 size_t Model::exact_bytes(int C) const {
   const int nt = cfg_.nt;
   if (C <= 0 || C > nt) C = nt;
+  resident::ExactPlan on_chip;
+  const int lanes = exact_resident_lanes(C, cfg_.n_shots, &on_chip);
+  if (lanes > 0)
+    return static_cast<size_t>(lanes) * exact_resident_bytes(C, on_chip) +
+           static_cast<size_t>(cfg_.n_shots) * 4 * grid_size() * sizeof(float2) +
+           7 * grid_size() * sizeof(double);
   if (prec_ == PSV_FP32 && tma_ok_ && is_tma())
     return static_cast<size_t>(exact_lane_count(C, cfg_.n_shots)) * exact_lane_bytes(C) +
            static_cast<size_t>(cfg_.n_shots) * 4 * grid_size() * sizeof(float2) +
@@ -1012,7 +1055,10 @@ double Model::exact_gradient_lanes(int C, const std::vector<int> &shot_list) {
   const size_t field_bytes = gp * sizeof(float), state_bytes = 5 * field_bytes;
   cudaStream_t ms = stream();
   const int n_list = static_cast<int>(shot_list.size());
-  const int K = std::max(1, exact_lane_count(C, std::max(n_list, 1)));
+  resident::ExactPlan on_chip;
+  const int on_chip_lanes = exact_resident_lanes(C, n_list, &on_chip);
+  const int K = on_chip_lanes > 0 ? on_chip_lanes
+                                  : std::max(1, exact_lane_count(C, std::max(n_list, 1)));
   // Forward steps of the lanes: the 32 x 60 shape (the vectorised tile
   // path, fewest instructions per point) when the lanes' tiles fill at
   // least two waves of resident CTAs between them; else the model's shape.
@@ -1040,8 +1086,14 @@ double Model::exact_gradient_lanes(int C, const std::vector<int> &shot_list) {
   if (ensure_lanes(K)) grown = true;
   for (auto &l : lanes_) {
     ensure(l->ckpt, n_ck * state_bytes);
-    ensure(l->slots, (C + 1) * state_bytes);
-    ensure(l->lam, kLamPlanes * field_bytes);
+    if (on_chip_lanes > 0) {
+      ensure(l->slots, C * on_chip.rate_stride * sizeof(float2));
+      ensure(l->lam, state_bytes);
+      ensure(l->mail, resident::mailbox_bytes(on_chip.p));
+    } else {
+      ensure(l->slots, (C + 1) * state_bytes);
+      ensure(l->lam, kLamPlanes * field_bytes);
+    }
     ensure(l->raw, std::max<size_t>(2 * static_cast<size_t>(nr) * nt * sizeof(float), 16));
     ensure(l->part, gp * (sizeof(float2) + sizeof(float)));
   }
@@ -1061,6 +1113,7 @@ double Model::exact_gradient_lanes(int C, const std::vector<int> &shot_list) {
   };
   for (auto &lp : lanes_) {
     ExactLane &l = *lp;
+    if (on_chip_lanes > 0) break;
     if (l.maps_slots == l.slots.get() && l.maps_lam == l.lam.get() && l.maps_C == C &&
         l.maps_cfg == ecfg)
       continue;
@@ -1078,6 +1131,72 @@ double Model::exact_gradient_lanes(int C, const std::vector<int> &shot_list) {
     l.maps_C = C;
     l.maps_cfg = ecfg;
   }
+
+  auto seismograms = [&](ExactLane &l, int shot, cudaStream_t s) {
+    if (!nr) return;
+    const size_t off = static_cast<size_t>(shot) * nr * nt;
+    const float *raw = l.raw.as<float>();
+    cuda_check(receiver_cumsum_f32(nr, nt, nt, cfg_.dt, cfg_.dx * cfg_.dz, raw,
+                                   raw + static_cast<size_t>(nr) * nt, rtf_[0].as<double>() + off,
+                                   rtf_[1].as<double>() + off, s),
+               "seismograms");
+    for (int c = 0; c < 2; ++c)
+      cuda_check(exact_receiver_terms(nr, nt, cfg_.dt, cfg_.dx * cfg_.dz,
+                                      rtf_[c].as<double>() + off, rtf_true_[c].as<double>() + off,
+                                      adj_[c].as<double>() + off, s),
+                 "receiver terms");
+  };
+
+  // Grids that fit on the chip. A forward pass keeps every C-th state; then,
+  // from the last segment back, each is run again from its state keeping the
+  // rates of its steps (the last one at once), and the adjoint goes through
+  // them. Same step kernel in both passes, so the same states whatever C is.
+  auto one_shot_on_chip = [&](ExactLane &l, int shot, cudaStream_t s) {
+    float2 *gs = gff_shots_.as<float2>() + static_cast<size_t>(shot) * 4 * g;
+    cuda_check(cudaMemsetAsync(gs, 0, 4 * g * sizeof(float2), s), "exact zero");
+    auto state = [&](float *b) { return fast::Fields{b, b + gp, b + 2 * gp, b + 3 * gp, b + 4 * gp}; };
+    float *ck = l.ckpt.as<float>(), *raw = l.raw.as<float>();
+    float2 *rates = l.slots.as<float2>();
+    int *err = err_flag_.as<int>();
+    const int last0 = (n_ck - 1) * C;
+    tma::SimDesc f = descs_h_[shot], b = descs_h_[n_shots + shot];
+    f.rec_vx = raw;
+    f.rec_vz = raw + static_cast<size_t>(nr) * nt;
+    f.set[0] = f.set[1] = state(ck + static_cast<size_t>(n_ck - 1) * 5 * gp);
+    resident::Dump keep;
+    keep.base = ck;
+    keep.stride = 5 * gp;
+    keep.every = C;
+    cuda_check(resident::steps(f, on_chip.p, false, 0, last0, 0, true, false, keep, l.mail.get(),
+                               err, s),
+               "exact forward");
+    const size_t off = static_cast<size_t>(shot) * nr * nt;
+    b.set[0] = b.set[1] = state(l.lam.as<float>());
+    b.a_ux = adj_[0].as<double>() + off;
+    b.a_uz = adj_[1].as<double>() + off;
+    b.stf = stf_d_.as<double>();
+    for (int k = n_ck - 1; k >= 0; --k) {
+      const int s0 = k * C, n = std::min(nt, s0 + C) - s0;
+      const bool last = k + 1 == n_ck;
+      f.set[0] = f.set[1] = state(ck + static_cast<size_t>(k) * 5 * gp);
+      if (!last) f.nr = 0;  // recorded already
+      cuda_check(resident::steps_keeping_rates(f, on_chip, s0, n, k == 0, rates, l.mail.get(), err, s),
+                 "exact forward");
+      if (last) seismograms(l, shot, s);
+      resident::ExactSteps x;
+      x.first = s0;
+      x.n_steps = n;
+      x.zero = last;
+      x.rates = rates;
+      x.src = plans_[shot];
+      x.part = l.part.as<float>();
+      x.sums[0] = gs;
+      x.sums[1] = gs + 2 * g;
+      x.sums[2] = gs + 3 * g;
+      x.flush = kFlushSteps;
+      cuda_check(resident::exact_steps(b, on_chip, x, l.mail.get(), err, s), "exact steps");
+    }
+  };
 
   auto one_shot = [&](ExactLane &l, int shot, cudaStream_t s) {
     unsigned char *ck = l.ckpt.as<unsigned char>(), *sl = l.slots.as<unsigned char>();
@@ -1131,18 +1250,7 @@ double Model::exact_gradient_lanes(int C, const std::vector<int> &shot_list) {
       }
     }
     const size_t off = static_cast<size_t>(shot) * nr * nt;
-    if (nr) {
-      cuda_check(receiver_cumsum_f32(nr, nt, nt, cfg_.dt, cfg_.dx * cfg_.dz, raw,
-                                     raw + static_cast<size_t>(nr) * nt,
-                                     rtf_[0].as<double>() + off, rtf_[1].as<double>() + off, s),
-                 "seismograms");
-      for (int c = 0; c < 2; ++c)
-        cuda_check(exact_receiver_terms(nr, nt, cfg_.dt, cfg_.dx * cfg_.dz,
-                                        rtf_[c].as<double>() + off,
-                                        rtf_true_[c].as<double>() + off,
-                                        adj_[c].as<double>() + off, s),
-                   "receiver terms");
-    }
+    seismograms(l, shot, s);
     cuda_check(cudaMemsetAsync(l.lam.get(), 0, l.lam.bytes(), s), "zero adjoint");
     // Adjoint state planes: l^{n+1} in (lv, lt), l^n out (ov, ot), swapped
     // after every step.
@@ -1211,7 +1319,12 @@ double Model::exact_gradient_lanes(int C, const std::vector<int> &shot_list) {
     const int li = i % K;
     ExactLane &l = *lanes_[li];
     cudaStream_t s = li == 0 ? ms : l.stream;
-    auto enqueue = [&] { one_shot(l, shot, s); };
+    auto enqueue = [&] {
+      if (on_chip_lanes > 0)
+        one_shot_on_chip(l, shot, s);
+      else
+        one_shot(l, shot, s);
+    };
     if (!use_graphs_) {
       enqueue();
       continue;

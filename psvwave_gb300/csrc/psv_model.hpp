@@ -300,7 +300,12 @@ class Model {
     cudaStream_t stream = nullptr;  // own stream (lanes >= 1)
     cudaEvent_t done = nullptr;
     // part: FP32 partial gradient sums, (lm, mu) pairs then b, padded grid
-    DeviceBuffer ckpt, slots, lam, raw, part;
+    // mail: mailboxes between CTAs (gradients resident on chip, whose slots
+    // hold the kept rates)
+    DeviceBuffer ckpt, slots, lam, raw, part, mail;
+    size_t bytes() const {
+      return ckpt.bytes() + slots.bytes() + lam.bytes() + raw.bytes() + part.bytes() + mail.bytes();
+    }
     std::vector<tma::Maps> slot_maps;  // input maps of each state slot
     exact_tma::Maps emaps;             // the exact step's maps over lam, slots, medium
     const void *maps_slots = nullptr;  // slots / lam / C / tile shape the maps were made for
@@ -326,6 +331,10 @@ class Model {
   static constexpr int kFlushSteps = 20;  // exact step: partial sums into the pairs
   int exact_lane_count(int C, int n_list) const;
   size_t exact_lane_bytes(int C) const;
+  resident::ExactPlan exact_plan(int lanes) const;
+  int exact_resident_lanes(int C, int n_list, resident::ExactPlan *plan) const;
+  size_t exact_resident_bytes(int C, const resident::ExactPlan &p) const;
+  mutable std::map<int, resident::ExactPlan> exact_plans_;  // by lanes
   double exact_gradient_lanes(int C, const std::vector<int> &shot_list);
   void destroy_lanes();
   // Injection plans: one per shot (sources) and one for the adjoint receivers.

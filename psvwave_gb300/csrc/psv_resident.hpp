@@ -56,13 +56,11 @@ Plan plan_mailbox(const Grid &g, int max_ctas, int per_sm);
 
 // States saved during a run: the state before step j of the launch goes to
 // base + (j / every) * stride when j % every == 0 (five planes of
-// nx * pitch floats). last: the final state too, where it falls on a
-// multiple of `every`.
+// nx * pitch floats).
 struct Dump {
   float *base = nullptr;
   size_t stride = 0;
   int every = 1;
-  int last = 0;
 };
 
 // Mailbox bytes of a plan (0 for a cluster).
@@ -76,6 +74,44 @@ size_t mailbox_bytes(const Plan &p);
 cudaError_t steps(const tma::SimDesc &d, const Plan &p, bool adjoint, int it0, int n_steps,
                   int parity, bool zero, bool store, const Dump &dump, void *mail, int *err,
                   cudaStream_t s);
+
+// ---- exact gradients (psv_resident_exact.cu) ----
+
+// The split of an exact gradient of one simulation: forward steps that keep
+// their rates, and the exact adjoint's steps, on the same tiles. n_src: the
+// most source points of a tile; smem: the adjoint's. lanes: how many run at
+// once, each on its share of the device.
+struct ExactPlan {
+  Plan p;
+  int n_src = 0;
+  size_t smem = 0;
+  size_t rate_stride = 0;  // float2 per step
+};
+ExactPlan plan_exact(const Grid &g, int lanes);
+
+// Steps it0, it0 + 1, ... of d from set 0 (zero: from zero fields), as
+// steps() takes them, keeping the rates of step it0 + k at
+// rates + k * rate_stride; final state in set n_steps & 1.
+cudaError_t steps_keeping_rates(const tma::SimDesc &d, const ExactPlan &p, int it0, int n_steps,
+                                bool zero, float2 *rates, void *mail, int *err, cudaStream_t s);
+
+// The exact adjoint (notation in psv_exact.cuh) of steps first + n_steps - 1
+// down to first: d.set[0] holds l of the last of them (zero: it is zero)
+// and takes l of the first; d.plan's terms add the series a_ux, a_uz to the
+// adjoint velocities. The gradients of lm, mu (with lambda = lm - 2 mu) and b
+// go into `sums`, float-float pairs, every `flush` steps; between launches
+// what is not in them yet is in part (three planes of nx * pitch).
+struct ExactSteps {
+  int first = 0, n_steps = 0;
+  bool zero = false;
+  const float2 *rates = nullptr;
+  InjPlan src{};  // the shot's source terms
+  float *part = nullptr;
+  float2 *sums[3] = {nullptr, nullptr, nullptr};
+  int flush = 1;
+};
+cudaError_t exact_steps(const tma::SimDesc &d, const ExactPlan &p, const ExactSteps &x,
+                        void *mail, int *err, cudaStream_t s);
 
 // ---- batches: forward steps of many simulations from zero fields ----
 

@@ -1,763 +1,19 @@
-// FP32 time stepping with the grid resident on chip; see psv_resident.hpp.
-//
-// Work split: a team's CTAs form tiles_x x tiles_z tiles. A tile of R rows
-// and C column pairs is split over `groups` groups of C threads: thread
-// (g, c) owns columns 2c, 2c + 1 of the group's kn consecutive rows (2 <= kn
-// <= K). Its points' five wave fields, lm, mu, b and taper factors stay in
-// registers for every step. Shared memory holds the tile's fields
-// F[R + 4][5][S] (vx vz txx tzz txz; S a compile-time stride) with two halo
-// rows and two halo columns on each side: a thread reads z neighbours, and x
-// neighbours outside its run, from there as float2.
-//
-// One time step is a stress and a velocity half-step. In a half-step each
-// thread advances its points, writes them to shared memory and sends the
-// tile's edge values (two rows, two columns) to the neighbouring CTAs. A
-// half-step's x stencils read one field with the forward difference (one row
-// before, two after) and one with the backward difference (two before, one
-// after): three words per column pair and side; its z stencils read a pair
-// of columns of two fields on each side. The CTA's last warps (helpers)
-// record the receivers and evaluate the injection terms meanwhile.
-//
-// Two links carry the edges:
-//  * Cluster (teams of up to 16 CTAs, one thread-block cluster): st.async
-//    writes a word straight into the neighbour's halo and counts its bytes on
-//    the neighbour's mbarrier, which completes a half-step once every thread
-//    of the CTA has arrived and every incoming byte has landed. (A halo cell
-//    is overwritten only after the neighbour has received all words of the
-//    previous half-step from that side, and each is sent by a thread that
-//    has finished reading that side's halo.)
-//  * Mailbox (any team, cooperative launch; a group is a warp): 128-bit words
-//    in global memory carry three values and the step's tag, written and read
-//    as single relaxed accesses, so a word whose tag matches carries its
-//    values, with no flag, fence or barrier between CTAs; the helpers wait for
-//    the tile's words and put them into the halo before the CTA's barrier. A
-//    warp sends its rows' edge columns with one store, its lanes reading them
-//    back from shared memory: one store a row and side, from one lane, cost
-//    0.4 us a half-step at 58 x 62 points. Two parities of every
-//    box suffice: a CTA writes step j + 2 only after it has received step
-//    j + 1, which its neighbour sent after a barrier that follows its reads of
-//    step j.
-//
-// Points outside the updated region [2, n - 2) carry lm = mu = b = 0 and a
-// taper factor of 1: their update adds zero. Arithmetic is written with
-// explicit fused multiply-adds so that every instantiation rounds alike.
-//
-// Every wait is bounded: a thread whose wait runs out raises *err and stops
-// waiting for the rest of the launch, which then ends by itself.
-#include "psv_resident.hpp"
-
-#include <cooperative_groups.h>
-
-#include <algorithm>
-#include <cstdint>
-#include <vector>
-
-#include "psv_tma_ptx.cuh"
-#include "psv_tma_terms.cuh"
+// FP32 forward and adjoint steps resident on chip (psv_resident_core.cuh): one
+// simulation, or a batch's members.
+#include "psv_resident_core.cuh"
 
 namespace psv {
 namespace resident {
-namespace cg = cooperative_groups;
 namespace {
 
-constexpr int kMaxThreads = 512;
-constexpr int kMinK = 3, kMaxK = 5;
-constexpr uint32_t kPolls = 1u << 20;  // about a second
-constexpr int kCommWords = 4;          // words received by one helper thread
-constexpr int kMaxCluster = 16;
-
-// First item of part k when n items are split evenly over parts.
-__host__ __device__ __forceinline__ int split(int k, int parts, int n) {
-  return (int)(((long long)k * n) / parts);
-}
-__host__ __device__ __forceinline__ int pairs(int nz) { return (nz + 1) / 2; }
-// Shared row strides: column pairs of a tile at most (S - 4) / 2.
-constexpr int kNarrow = 68, kWide = 156;
-
-// Mailbox word: three values and the tag, one 16-byte access. The x stencils
-// of a column need three values from a side (both fields' rows), the z
-// stencils of a row three as well (two columns of one field, one of the
-// other). Incoming words of a tile of R rows and C pairs: from above, from
-// below (2 C columns each), from the left and from the right (R rows each).
-struct alignas(16) Word {
-  float a, b, c;
-  uint32_t tag;
-};
-__host__ __device__ __forceinline__ int words(int R, int C) { return 4 * C + 2 * R; }
-constexpr int kBoxWords = 320;
-constexpr int kBox = 4 * kBoxWords;  // words of one CTA: [kind 2][parity 2][words]
-
-// (post and push carry no memory clobber: nothing else in the thread depends on
-// what they write, and a clobber in the row loop would keep the next row's
-// shared loads from being issued ahead.)
-__device__ __forceinline__ void post(Word *p, float a, float b, float c, uint32_t tag) {
-  const unsigned long long lo = (unsigned long long)__float_as_uint(b) << 32 | __float_as_uint(a);
-  const unsigned long long hi = (unsigned long long)tag << 32 | __float_as_uint(c);
-  asm volatile(
-      "{\n .reg .b128 w;\n mov.b128 w, {%1, %2};\n st.relaxed.gpu.global.b128 [%0], w;\n}" ::"l"(p),
-      "l"(lo), "l"(hi));
-}
-__device__ __forceinline__ Word peek(const Word *p) {
-  unsigned long long lo, hi;
-  asm volatile("{\n .reg .b128 w;\n ld.relaxed.gpu.global.b128 w, [%2];\n mov.b128 {%0, %1}, w;\n}"
-               : "=l"(lo), "=l"(hi)
-               : "l"(p)
-               : "memory");
-  Word w;
-  w.a = __uint_as_float((uint32_t)lo);
-  w.b = __uint_as_float((uint32_t)(lo >> 32));
-  w.c = __uint_as_float((uint32_t)hi);
-  w.tag = (uint32_t)(hi >> 32);
-  return w;
-}
-
-__device__ __forceinline__ uint32_t remote(uint32_t addr, int rank) {
-  uint32_t r;
-  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
-  return r;
-}
-// Writes a pair of columns into a neighbour's halo; its bytes complete on
-// the neighbour's mbarrier.
-__device__ __forceinline__ void push(uint32_t addr, float2 v, uint32_t bar) {
-  asm volatile(
-      "st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v2.b32 [%0], {%1, %2}, [%3];" ::
-          "r"(addr),
-      "r"(__float_as_uint(v.x)), "r"(__float_as_uint(v.y)), "r"(bar));
-}
-
-__device__ __forceinline__ float2 lds2(const float *p) {
-  return *reinterpret_cast<const float2 *>(p);
-}
-__device__ __forceinline__ void sts2(float *p, float2 v) { *reinterpret_cast<float2 *>(p) = v; }
-
-// a1 (p - m) + a2 (l - r): one staggered difference with folded coefficients.
-__device__ __forceinline__ float diff(float a1, float p, float m, float a2, float l, float r) {
-  return __fmaf_rn(a2, __fsub_rn(l, r), __fmul_rn(a1, __fsub_rn(p, m)));
-}
-// acc + the same.
-__device__ __forceinline__ float diff_add(float acc, float a1, float p, float m, float a2, float l,
-                                          float r) {
-  return __fmaf_rn(a2, __fsub_rn(l, r), __fmaf_rn(a1, __fsub_rn(p, m), acc));
-}
-
-struct Team {
-  int k, tiles_x, tiles_z, groups;
-  int n_rec, n_inj;  // most receivers and injection points of a tile
-  Word *mail;  // mailbox link: boxes of the team's CTA 0
-};
-
-template <bool ADJ, int K, int S, bool CLUSTER>
-__device__ __forceinline__ void member_steps(const tma::SimDesc &d, const Team &tm, int it0,
-                                             int n_steps, int parity, bool zero, int store,
-                                             const Dump &dump, int *err) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  constexpr int RS = 5 * S;  // one row of the five fields
-  constexpr int oVX = 0, oVZ = S, oXX = 2 * S, oZZ = 3 * S, oXZ = 4 * S;
-  const int nx = d.nx, nz = d.nz, ps = d.pitch;
-  const int ti = tm.k / tm.tiles_z, tj = tm.k - ti * tm.tiles_z;
-  const int x0 = split(ti, tm.tiles_x, nx), R = split(ti + 1, tm.tiles_x, nx) - x0;
-  const int c0 = split(tj, tm.tiles_z, pairs(nz)), C = split(tj + 1, tm.tiles_z, pairs(nz)) - c0;
-  const int z0 = 2 * c0;
-  const int Rm = (nx + tm.tiles_x - 1) / tm.tiles_x;
-  float *const F = reinterpret_cast<float *>(smem_raw);
-  const InjPlan &pl = d.plan;
-  // Injection points of the tile: the value each adds this step (vx, vz), its
-  // first term, and the points' slots by (row, column); then receivers.
-  float2 *const INJ = reinterpret_cast<float2 *>(F + (Rm + 4) * RS);
-  int *const inj_first = reinterpret_cast<int *>(INJ + tm.n_inj);
-  int *const rec_off = inj_first + tm.n_inj, *const rec_id = rec_off + tm.n_rec;
-  unsigned short *const slot_of = reinterpret_cast<unsigned short *>(rec_off + 2 * tm.n_rec);
-  __shared__ int s_count[2];
-  __shared__ __align__(8) uint64_t s_bar[2];  // of stress and velocity half-steps
-  const int tid = threadIdx.x, NT = blockDim.x;
-
-  // Compute threads come first, helper warps after them.
-  const int CW = CLUSTER ? (tm.groups * ((pairs(nz) + tm.tiles_z - 1) / tm.tiles_z) + 31) & ~31
-                         : 32 * tm.groups;
-  const bool helper = tid >= CW;
-  const int g = CLUSTER ? tid / C : tid >> 5, c = CLUSTER ? tid - g * C : tid & 31;
-  const bool mine = !helper && g < tm.groups && c < C;
-  const bool in_group = !helper && g < tm.groups;
-  const int r0 = in_group ? split(g, tm.groups, R) : 0;
-  const int kn = in_group ? split(g + 1, tm.groups, R) - r0 : 2;
-  auto has = [&](int k) { return k < 2 || k < kn; };
-  const bool up = ti > 0, down = ti + 1 < tm.tiles_x;
-  const bool left = tj > 0, right = tj + 1 < tm.tiles_z;
-  const bool send_up = up && mine && g == 0, send_dn = down && mine && g == tm.groups - 1;
-  const bool send_z = mine && ((left && c == 0) || (right && c == C - 1));
-  const int z = z0 + 2 * c;
-  float *const my = F + (2 + r0) * RS + 2 + 2 * c;  // own first row
-
-  // Shared fields (halo rows and columns at the grid's edges stay zero).
-  for (int i = tid; i < (Rm + 4) * RS; i += NT) F[i] = 0.f;
-  if (tid < 2) s_count[tid] = 0;
-  if (CLUSTER && tid == 0) {
-    for (int k = 0; k < 2; ++k)
-      asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(tma::smem_u32(&s_bar[k])),
-                   "r"(NT)
-                   : "memory");
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  }
-  __syncthreads();
-  auto in_tile = [&](int ix, int iz) {
-    return ix >= x0 && ix < x0 + R && iz >= z0 && iz < z0 + 2 * C;
-  };
-  // The tile's injection points and receivers.
-  for (int i = tid; i < pl.n; i += NT) {
-    const int cell = pl.terms[i].cell, ix = cell / nz, iz = cell - ix * nz;
-    if (in_tile(ix, iz) && (i == 0 || pl.terms[i - 1].cell != cell)) {
-      const int q = atomicAdd(&s_count[0], 1);
-      inj_first[q] = i;
-      INJ[q] = make_float2(0.f, 0.f);
-      slot_of[(ix - x0) * (S - 4) + iz - z0] = (unsigned short)q;
-    }
-  }
-  if (!ADJ)
-    for (int r = tid; r < d.nr; r += NT) {
-      const int cell = d.rec_cell[r], ix = cell / ps, iz = cell - ix * ps;
-      if (in_tile(ix, iz)) {
-        const int q = atomicAdd(&s_count[1], 1);
-        rec_off[q] = (ix - x0 + 2) * RS + 2 + iz - z0;
-        rec_id[q] = r;
-      }
-    }
-
-  // Own points: state, medium, taper.
-  float2 vx[K], vz[K], xx[K], zz[K], xz[K], lm[K], mu[K], bb[K], tp[K];
-  uint32_t inj_mask = 0;
-  const fast::Fields in = d.set[parity];
-  auto load = [&](const float *src, int x, int zc) {
-    if (x < 0 || x >= nx || zc < 0 || zc >= nz) return make_float2(0.f, 0.f);
-    float2 v = *reinterpret_cast<const float2 *>(src + (size_t)x * ps + zc);
-    if (zc + 1 >= nz) v.y = 0.f;
-    return v;
-  };
-  const float2 zero2 = make_float2(0.f, 0.f);
-#pragma unroll
-  for (int k = 0; k < K; ++k) {
-    vx[k] = vz[k] = xx[k] = zz[k] = xz[k] = lm[k] = mu[k] = bb[k] = zero2;
-    tp[k] = make_float2(1.f, 1.f);
-    if (k >= kn || !mine) continue;
-    const int x = x0 + r0 + k;
-    if (!zero) {
-      vx[k] = load(in.vx, x, z);
-      vz[k] = load(in.vz, x, z);
-      xx[k] = load(in.txx, x, z);
-      zz[k] = load(in.tzz, x, z);
-      xz[k] = load(in.txz, x, z);
-    }
-    const bool xi = x >= 2 && x < nx - 2;
-    const float2 l = load(d.lm, x, z), m = load(d.mu, x, z), b = load(d.b, x, z);
-    auto taper = [&](int iz) {
-      const int n = min(min(x + 1, nx - x), min(iz + 1, nz - iz));
-      return n < d.np ? d.taper_tab[n] : 1.f;
-    };
-    if (xi && z >= 2 && z < nz - 2) {
-      lm[k].x = l.x;
-      mu[k].x = m.x;
-      bb[k].x = b.x;
-      tp[k].x = taper(z);
-    }
-    if (xi && z + 1 >= 2 && z + 1 < nz - 2) {
-      lm[k].y = l.y;
-      mu[k].y = m.y;
-      bb[k].y = b.y;
-      tp[k].y = taper(z + 1);
-    }
-    if (pl.n && x >= pl.x0 && x < pl.x0 + pl.w)
-      for (int e = 0; e < 2; ++e)
-        if (z + e >= pl.z0 && z + e < pl.z0 + pl.h && z + e < nz &&
-            pl.map[(x - pl.x0) * pl.h + (z + e - pl.z0)] >= 0)
-          inj_mask |= 1u << (2 * k + e);
-  }
-  // The first stress half-step's velocities with their halos.
-  if (!zero)
-    for (int i = tid; i < (R + 4) * (C + 2); i += NT) {
-      const int r = i / (C + 2), q = i - r * (C + 2);
-      const int o = r * RS + 2 * q;
-      sts2(F + oVX + o, load(in.vx, x0 - 2 + r, z0 - 2 + 2 * q));
-      sts2(F + oVZ + o, load(in.vz, x0 - 2 + r, z0 - 2 + 2 * q));
-    }
-
-  // Where this thread's edge values go. Mailbox link: slots of the
-  // neighbours' boxes. Cluster link: cells of the neighbours' halos (in
-  // bytes, field vx) and their mbarriers.
-  const Word *const box = tm.mail + (size_t)tm.k * kBox;
-  Word *out_up = nullptr, *out_dn = nullptr, *out_z = nullptr;
-  const float *z_from = F;  // the edge columns this lane sends
-  uint32_t far_up = 0, far_dn = 0, far_z = 0, bar_up = 0, bar_dn = 0, bar_z = 0, in_bytes = 0;
-  if (CLUSTER) {
-    const uint32_t base = tma::smem_u32(F), bar = tma::smem_u32(&s_bar[0]);
-    const int k_up = tm.k - tm.tiles_z, k_dn = tm.k + tm.tiles_z;
-    const int k_z = c == 0 && left ? tm.k - 1 : tm.k + 1;
-    if (send_up) {
-      const int Ru = x0 - split(ti - 1, tm.tiles_x, nx);
-      far_up = remote(base + 4u * ((Ru + 2) * RS + 2 + 2 * c), k_up);
-      bar_up = remote(bar, k_up);
-    }
-    if (send_dn) {
-      far_dn = remote(base + 4u * (2 + 2 * c), k_dn);
-      bar_dn = remote(bar, k_dn);
-    }
-    if (send_z) {
-      const int Cl = c0 - split(tj - 1, tm.tiles_z, pairs(nz));
-      far_z = remote(base + 4u * ((2 + r0) * RS + (k_z < tm.k ? 2 + 2 * Cl : 0)), k_z);
-      bar_z = remote(bar, k_z);
-    }
-    in_bytes = 8u * ((up ? 3 * C : 0) + (down ? 3 * C : 0) + (left ? 2 * R : 0) + (right ? 2 * R : 0));
-  } else {
-    out_up = tm.mail + (size_t)(tm.k - tm.tiles_z) * kBox + 2 * C + 2 * c;
-    out_dn = tm.mail + (size_t)(tm.k + tm.tiles_z) * kBox + 2 * c;
-    // Lanes 0 .. 7 send the group's rows to the left, 16 .. 23 to the right
-    // (a neighbour's box follows its own column count).
-    const int l = tid & 31, k = l & 7;
-    if (in_group && k < kn && !(l & 8)) {
-      if (l < 16 && left) {
-        const int Cl = c0 - split(tj - 1, tm.tiles_z, pairs(nz));
-        out_z = tm.mail + (size_t)(tm.k - 1) * kBox + 4 * Cl + R + r0 + k;
-      } else if (l >= 16 && right) {
-        const int Cr = split(tj + 2, tm.tiles_z, pairs(nz)) - c0 - C;
-        out_z = tm.mail + (size_t)(tm.k + 1) * kBox + 4 * Cr + r0 + k;
-      }
-      z_from = F + (2 + r0 + k) * RS + (l < 16 ? 2 : 2 * C);
-    }
-  }
-  auto box_at = [&](int kind, uint32_t tag) { return (kind * 2 + (int)(tag & 1)) * kBoxWords; };
-  // End of a half-step (kind 0 stress, 1 velocity): every thread has written
-  // its points, and the halo words of the half-step have arrived. (Two
-  // mbarriers: a neighbour may send the next half-step's words while threads
-  // of this CTA still finish this one.)
-  bool alive = true;
-  uint32_t phase = 0;
-  auto meet = [&](int kind, bool incoming) {
-    if (!CLUSTER) {
-      asm volatile("bar.sync 0;" ::: "memory");
-      return;
-    }
-    const uint32_t bar = tma::smem_u32(&s_bar[kind]);
-    if (tid == 0)
-      asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar),
-                   "r"(incoming ? in_bytes : 0u)
-                   : "memory");
-    else
-      asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
-    if (alive && !tma::mbar_wait(&s_bar[kind], phase, kPolls)) {
-      alive = false;
-      atomicOr(err, 4);
-    }
-    phase ^= (uint32_t)kind;
-  };
-
-  const float c1x = ADJ ? -d.coef[0] : d.coef[0], c2x = ADJ ? -d.coef[1] : d.coef[1];
-  const float c1z = ADJ ? -d.coef[2] : d.coef[2], c2z = ADJ ? -d.coef[3] : d.coef[3];
-  if (CLUSTER)
-    cg::this_cluster().sync();
-  else
-    __syncthreads();
-
-  // ---- helper warps ----
-  if (helper) {
-    const int ct = tid - CW, CT = NT - CW;
-    const int n_inj = s_count[0], n_rec = s_count[1];
-    // Mailbox link: this thread's incoming words, where they lie in a box and
-    // where their values go in shared memory after a stress (0) and a velocity
-    // (1) half-step.
-    int in_at[kCommWords], to_a[kCommWords], to_b[kCommWords], to_c[kCommWords];
-    if (!CLUSTER) {
-      // Cells are given for the velocity half-step (vx, vz); the stress
-      // half-step's fields take their places below.
-#pragma unroll
-      for (int q = 0; q < kCommWords; ++q) {
-        const int i = ct + q * CT;
-        in_at[q] = -1;
-        to_a[q] = to_b[q] = to_c[q] = 0;
-        if (i < 4 * C) {
-          const int s = i / (2 * C), o = 2 + i - s * 2 * C;
-          if (!(s ? down : up)) continue;
-          in_at[q] = i;
-          // Above: P row -1, M rows -2, -1; below: P rows R, R + 1, M row R.
-          to_a[q] = (s ? R + 2 : 1) * RS + oVX + o;
-          to_b[q] = s ? (R + 3) * RS + oVX + o : oVZ + o;
-          to_c[q] = (s ? R + 2 : 1) * RS + oVZ + o;
-        } else if (i < words(R, C)) {
-          const int t = i - 4 * C, s = t / R, o = (2 + t - s * R) * RS + (s ? 2 + 2 * C : 0);
-          if (!(s ? right : left)) continue;
-          in_at[q] = i;
-          // Left: forward-difference field's second column, both of the other;
-          // right: both of the forward-difference field, first of the other.
-          to_a[q] = o + oVX + (s ? 0 : 1);
-          to_b[q] = o + (s ? oVX + 1 : oVZ);
-          to_c[q] = o + oVZ + (s ? 0 : 1);
-        }
-      }
-    }
-    // The stress half-step sends txz, txx along x and tzz, txz along z where
-    // the velocity half-step sends vx, vz.
-    auto cell = [&](int q, int to, int kind) {
-      if (kind) return to;
-      const bool vz_ = to % RS >= oVZ;
-      if (in_at[q] < 4 * C) return to + (vz_ ? oXX - oVZ : oXZ - oVX);
-      return to + (vz_ ? oXZ - oVZ : oZZ - oVX);
-    };
-    int st_a[kCommWords], st_b[kCommWords], st_c[kCommWords];
-#pragma unroll
-    for (int q = 0; q < kCommWords; ++q) {
-      st_a[q] = cell(q, to_a[q], 0);
-      st_b[q] = cell(q, to_b[q], 0);
-      st_c[q] = cell(q, to_c[q], 0);
-    }
-    // Waits for this thread's words of a half-step and puts them into the halo.
-    auto receive = [&](int kind, uint32_t tag) {
-      if (CLUSTER) return;
-      const Word *const from = box + box_at(kind, tag);
-      uint32_t open = 0;  // words still to come
-#pragma unroll
-      for (int q = 0; q < kCommWords; ++q)
-        if (in_at[q] >= 0) open |= 1u << q;
-      for (uint32_t i = 0; open && alive; ++i) {
-        Word w[kCommWords];
-#pragma unroll
-        for (int q = 0; q < kCommWords; ++q)
-          if (open >> q & 1u) w[q] = peek(from + in_at[q]);
-#pragma unroll
-        for (int q = 0; q < kCommWords; ++q)
-          if ((open >> q & 1u) && w[q].tag == tag) {
-            F[kind ? to_a[q] : st_a[q]] = w[q].a;
-            F[kind ? to_b[q] : st_b[q]] = w[q].b;
-            F[kind ? to_c[q] : st_c[q]] = w[q].c;
-            open &= ~(1u << q);
-          }
-        if (i == kPolls) {
-          alive = false;
-          atomicOr(err, 4);
-        }
-      }
-    };
-    // Item 2 q + f is field f of injection point q; helper thread i
-    // evaluates item i (and i + CT, ...) in the stress half-step. An item's term adds
-    // weight * (sample of its source or adjoint source); the first item's first
-    // term is kept in registers with its sample loaded one step ahead.
-    const double *inj_src = nullptr;
-    double inj_w = 0.0, inj_next = 0.0;
-    bool inj_more = false;
-    auto term_series = [&](const InjTerm &t) {
-      const double *src = t.kind == 0 ? d.stf : (t.field == 0 ? d.a_ux : d.a_uz);
-      return src + (size_t)t.index * d.nt;
-    };
-    auto term_weight = [&](const InjTerm &t) {
-      const int ix = t.cell / nz, iz = t.cell - ix * nz;
-      const double b = (double)d.b[(size_t)ix * ps + iz];
-      return (t.kind == 0 ? t.coef : 1.0) * d.dt_d * b / t.div;
-    };
-    // Sum of an item's terms at step `it`, from its skip-th on.
-    auto item_value = [&](int i, int it, int skip) {
-      const int q0 = inj_first[i >> 1], cell = pl.terms[q0].cell;
-      float v = 0.f;
-      for (int q = q0; q < pl.n && pl.terms[q].cell == cell; ++q) {
-        const InjTerm t = pl.terms[q];
-        if (t.field != (i & 1) || skip-- > 0) continue;
-        v += (float)(term_weight(t) * term_series(t)[it]);
-      }
-      return v;
-    };
-    if (ct < 2 * n_inj) {
-      const int q0 = inj_first[ct >> 1], cell = pl.terms[q0].cell;
-      for (int q = q0; q < pl.n && pl.terms[q].cell == cell; ++q) {
-        const InjTerm t = pl.terms[q];
-        if (t.field != (ct & 1)) continue;
-        if (!inj_src) {
-          inj_src = term_series(t);
-          inj_w = term_weight(t);
-          inj_next = inj_src[it0];
-        } else {
-          inj_more = true;
-        }
-      }
-    }
-    for (int j = 0; j < n_steps; ++j) {
-      const int it = ADJ ? it0 - j : it0 + j;
-      const uint32_t tag = (uint32_t)(j + 1);
-      const bool more = j + 1 < n_steps;
-      // Receivers: pre-step velocities.
-      if (!ADJ)
-        for (int i = ct; i < n_rec; i += CT) {
-          const size_t o = (size_t)rec_id[i] * d.nt + it;
-          d.rec_vx[o] = F[oVX + rec_off[i]];
-          d.rec_vz[o] = F[oVZ + rec_off[i]];
-        }
-      // What the tile's injection points add this step.
-      if (inj_src) {
-        float v = (float)(inj_w * inj_next);
-        if (inj_more) v += item_value(ct, it, 1);
-        reinterpret_cast<float *>(INJ)[ct] = v;
-        if (more) inj_next = inj_src[ADJ ? it - 1 : it + 1];
-      }
-      for (int i = ct + CT; i < 2 * n_inj; i += CT)
-        reinterpret_cast<float *>(INJ)[i] = item_value(i, it, 0);
-      receive(0, tag);
-      meet(0, true);
-      if (more) receive(1, tag);
-      meet(1, more);
-    }
-    if (CLUSTER) cg::this_cluster().sync();
-    return;
-  }
-
-  auto save = [&](float *base) {
-    const size_t gp = (size_t)nx * ps;
-#pragma unroll
-    for (int k = 0; k < K; ++k) {
-      if (k >= kn) continue;
-      float *q = base + (size_t)(x0 + r0 + k) * ps + z;
-      if (z + 1 < nz) {
-        sts2(q, vx[k]);
-        sts2(q + gp, vz[k]);
-        sts2(q + 2 * gp, xx[k]);
-        sts2(q + 3 * gp, zz[k]);
-        sts2(q + 4 * gp, xz[k]);
-      } else {
-        q[0] = vx[k].x;
-        q[gp] = vz[k].x;
-        q[2 * gp] = xx[k].x;
-        q[3 * gp] = zz[k].x;
-        q[4 * gp] = xz[k].x;
-      }
-    }
-  };
-
-  // Cluster link: sends the tile's edge columns of row k (the first thread of
-  // a group to the left, the last to the right): fields at o0, o1 of a row.
-  auto push_z = [&](int k, float2 f0, int o0, float2 f1, int o1, int kind) {
-    if (!CLUSTER || !send_z) return;
-    const uint32_t bar = bar_z + 8u * kind;
-    push(far_z + 4u * (k * RS + o0), f0, bar);
-    push(far_z + 4u * (k * RS + o1), f1, bar);
-  };
-  // Mailbox link: the same for the group's rows at once, read back from shared
-  // memory: the z stencils' forward-difference field at of, the other at ob.
-  auto post_z = [&](int of, int ob, int at, uint32_t tag) {
-    if (CLUSTER || !(left || right)) return;
-    __syncwarp();
-    if (!out_z) return;
-    const float2 f = lds2(z_from + of), b = lds2(z_from + ob);
-    if ((tid & 31) < 16)
-      post(out_z + at, f.x, f.y, b.x, tag);
-    else
-      post(out_z + at, f.y, b.x, b.y, tag);
-  };
-  // Sends the edge rows of a half-step's forward- (p, at op of a row) and
-  // backward-difference (m, at om) fields to the neighbours above and below.
-  auto publish_x = [&](const float2 *p, int op, const float2 *m, int om, int kind, int at,
-                       uint32_t tag) {
-    const uint32_t b8 = 8u * kind;
-    if (send_up) {
-      if (CLUSTER) {
-        push(far_up + 4u * op, p[0], bar_up + b8);
-        push(far_up + 4u * (RS + op), p[1], bar_up + b8);
-        push(far_up + 4u * om, m[0], bar_up + b8);
-      } else {
-        post(out_up + at, p[0].x, p[1].x, m[0].x, tag);
-        post(out_up + at + 1, p[0].y, p[1].y, m[0].y, tag);
-      }
-    }
-    if (send_dn) {
-      float2 pl1 = p[1], ml2 = m[0], ml1 = m[1];  // the last rows
-#pragma unroll
-      for (int k = 2; k < K; ++k)
-        if (has(k)) {
-          pl1 = p[k];
-          ml2 = m[k - 1];
-          ml1 = m[k];
-        }
-      if (CLUSTER) {
-        push(far_dn + 4u * (RS + op), pl1, bar_dn + b8);
-        push(far_dn + 4u * om, ml2, bar_dn + b8);
-        push(far_dn + 4u * (RS + om), ml1, bar_dn + b8);
-      } else {
-        post(out_dn + at, pl1.x, ml2.x, ml1.x, tag);
-        post(out_dn + at + 1, pl1.y, ml2.y, ml1.y, tag);
-      }
-    }
-  };
-  // Row i of a field: own, or one of the rows after the run.
-  auto row = [&](const float2 *own, int i, float2 a0, float2 a1) {
-    if (i < K && has(i)) return own[i];
-    return i == kn ? a0 : a1;
-  };
-
-  // Steps until the next snapshot step, and until the next saved state.
-  const bool snaps = d.accu[0] != nullptr && (ADJ || store);
-  int to_snap = ADJ ? it0 % d.si : (d.si - it0 % d.si) % d.si;
-  int to_dump = 0;
-  for (int j = 0; j < n_steps; ++j) {
-    const int it = ADJ ? it0 - j : it0 + j;
-    const bool snap = snaps && to_snap == 0;
-    to_snap = to_snap == 0 ? d.si - 1 : to_snap - 1;
-    if (!ADJ && dump.base) {
-      if (to_dump == 0 && mine) save(dump.base + (size_t)(j / dump.every) * dump.stride);
-      to_dump = to_dump == 0 ? dump.every - 1 : to_dump - 1;
-    }
-    if (snap && mine) {
-      const size_t soff = (size_t)(it / d.si) * nx * nz;
-#pragma unroll
-      for (int k = 0; k < K; ++k) {
-        if (k >= kn) continue;
-        const int x = x0 + r0 + k;
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          const int iz = z + e;
-          if (iz >= nz) continue;
-          const int gi = x * nz + iz;
-          const float a = e ? vx[k].y : vx[k].x, b = e ? vz[k].y : vz[k].x,
-                      sx = e ? xx[k].y : xx[k].x, sz = e ? zz[k].y : zz[k].x,
-                      sh = e ? xz[k].y : xz[k].x;
-          if (!ADJ) {
-            d.accu[0][soff + gi] = a;
-            d.accu[1][soff + gi] = b;
-            d.accu[2][soff + gi] = sx;
-            d.accu[3][soff + gi] = sz;
-            d.accu[4][soff + gi] = sh;
-          } else if (x >= d.fx0 && x < d.fx1 && iz >= d.fz0 && iz < d.fz1) {
-            const float *as[5] = {d.accu[0] + soff, d.accu[1] + soff, d.accu[2] + soff,
-                                  d.accu[3] + soff, d.accu[4] + soff};
-            const size_t gp = (size_t)x * ps + iz;
-            tma::correlate(d, as, gi, d.lm[gp], d.mu[gp], a, b, sx, sz, sh);
-          }
-        }
-      }
-    }
-    const uint32_t tag = (uint32_t)(j + 1);
-    // ---- stresses ----
-    int at = box_at(0, tag);
-    if (mine) {
-      // Rows around the run.
-      const float *const end = my + kn * RS;
-      const float2 p_b1 = lds2(my + oVX - RS), p_a0 = lds2(end + oVX), p_a1 = lds2(end + oVX + RS);
-      const float2 m_b2 = lds2(my + oVZ - 2 * RS), m_b1 = lds2(my + oVZ - RS),
-                   m_a0 = lds2(end + oVZ);
-#pragma unroll
-      for (int k = 0; k < K; ++k) {
-        if (has(k)) {
-          const float2 xm1 = k >= 1 ? vx[k - 1] : p_b1, x0v = vx[k],
-                       xp1 = row(vx, k + 1, p_a0, p_a1), xp2 = row(vx, k + 2, p_a0, p_a1);
-          const float2 zm2 = k >= 2 ? vz[k - 2] : (k == 1 ? m_b1 : m_b2),
-                       zm1 = k >= 1 ? vz[k - 1] : m_b1, z0v = vz[k],
-                       zp1 = row(vz, k + 1, m_a0, m_a0);
-          const float *pv = my + k * RS;
-          const float2 vxl = lds2(pv + oVX - 2), vxr = lds2(pv + oVX + 2);
-          const float2 vzl = lds2(pv + oVZ - 2), vzr = lds2(pv + oVZ + 2);
-          const float ex0 = diff(c1x, xp1.x, x0v.x, c2x, xm1.x, xp2.x);
-          const float ex1 = diff(c1x, xp1.y, x0v.y, c2x, xm1.y, xp2.y);
-          const float ez0 = diff(c1z, z0v.x, vzl.y, c2z, vzl.x, z0v.y);
-          const float ez1 = diff(c1z, z0v.y, z0v.x, c2z, vzl.y, vzr.x);
-          const float g0 = diff_add(diff(c1z, x0v.y, x0v.x, c2z, vxl.y, vxr.x), c1x, z0v.x, zm1.x,
-                                    c2x, zm2.x, zp1.x);
-          const float g1 = diff_add(diff(c1z, vxr.x, x0v.y, c2z, x0v.x, vxr.y), c1x, z0v.y, zm1.y,
-                                    c2x, zm2.y, zp1.y);
-          const float la0 = __fmaf_rn(-2.f, mu[k].x, lm[k].x);
-          const float la1 = __fmaf_rn(-2.f, mu[k].y, lm[k].y);
-          xx[k].x = __fmul_rn(tp[k].x, __fmaf_rn(lm[k].x, ex0, __fmaf_rn(la0, ez0, xx[k].x)));
-          xx[k].y = __fmul_rn(tp[k].y, __fmaf_rn(lm[k].y, ex1, __fmaf_rn(la1, ez1, xx[k].y)));
-          zz[k].x = __fmul_rn(tp[k].x, __fmaf_rn(la0, ex0, __fmaf_rn(lm[k].x, ez0, zz[k].x)));
-          zz[k].y = __fmul_rn(tp[k].y, __fmaf_rn(la1, ex1, __fmaf_rn(lm[k].y, ez1, zz[k].y)));
-          xz[k].x = __fmul_rn(tp[k].x, __fmaf_rn(mu[k].x, g0, xz[k].x));
-          xz[k].y = __fmul_rn(tp[k].y, __fmaf_rn(mu[k].y, g1, xz[k].y));
-          float *to = my + k * RS;
-          sts2(to + oXX, xx[k]);
-          sts2(to + oZZ, zz[k]);
-          sts2(to + oXZ, xz[k]);
-          push_z(k, zz[k], oZZ, xz[k], oXZ, 0);
-        }
-      }
-      publish_x(xz, oXZ, xx, oXX, 0, at, tag);
-    }
-    post_z(oZZ, oXZ, at, tag);
-    meet(0, true);
-    // ---- velocities ----
-    at = box_at(1, tag);
-    const bool more = j + 1 < n_steps;  // the last step's velocities stay here
-    if (mine) {
-      const float *const end = my + kn * RS;
-      const float2 p_b1 = lds2(my + oXZ - RS), p_a0 = lds2(end + oXZ), p_a1 = lds2(end + oXZ + RS);
-      const float2 m_b2 = lds2(my + oXX - 2 * RS), m_b1 = lds2(my + oXX - RS),
-                   m_a0 = lds2(end + oXX);
-#pragma unroll
-      for (int k = 0; k < K; ++k) {
-        if (has(k)) {
-          const float2 am2 = k >= 2 ? xx[k - 2] : (k == 1 ? m_b1 : m_b2),
-                       am1 = k >= 1 ? xx[k - 1] : m_b1, a0 = xx[k],
-                       ap1 = row(xx, k + 1, m_a0, m_a0);
-          const float2 bm1 = k >= 1 ? xz[k - 1] : p_b1, b0 = xz[k],
-                       bp1 = row(xz, k + 1, p_a0, p_a1), bp2 = row(xz, k + 2, p_a0, p_a1);
-          const float *pt = my + k * RS;
-          const float2 zl = lds2(pt + oZZ - 2), zr = lds2(pt + oZZ + 2);
-          const float2 sl = lds2(pt + oXZ - 2), sr = lds2(pt + oXZ + 2);
-          const float2 z0v = zz[k];
-          const float ax0 = diff_add(diff(c1x, a0.x, am1.x, c2x, am2.x, ap1.x), c1z, b0.x, sl.y,
-                                     c2z, sl.x, b0.y);
-          const float ax1 = diff_add(diff(c1x, a0.y, am1.y, c2x, am2.y, ap1.y), c1z, b0.y, b0.x,
-                                     c2z, sl.y, sr.x);
-          const float az0 = diff_add(diff(c1x, bp1.x, b0.x, c2x, bm1.x, bp2.x), c1z, z0v.y, z0v.x,
-                                     c2z, zl.y, zr.x);
-          const float az1 = diff_add(diff(c1x, bp1.y, b0.y, c2x, bm1.y, bp2.y), c1z, zr.x, z0v.y,
-                                     c2z, z0v.x, zr.y);
-          vx[k].x = __fmul_rn(tp[k].x, __fmaf_rn(bb[k].x, ax0, vx[k].x));
-          vx[k].y = __fmul_rn(tp[k].y, __fmaf_rn(bb[k].y, ax1, vx[k].y));
-          vz[k].x = __fmul_rn(tp[k].x, __fmaf_rn(bb[k].x, az0, vz[k].x));
-          vz[k].y = __fmul_rn(tp[k].y, __fmaf_rn(bb[k].y, az1, vz[k].y));
-          if (inj_mask >> (2 * k) & 3u) {
-#pragma unroll
-            for (int e = 0; e < 2; ++e) {
-              if (!(inj_mask >> (2 * k + e) & 1u)) continue;
-              const float2 add = INJ[slot_of[(r0 + k) * (S - 4) + 2 * c + e]];
-              if (e) {
-                vx[k].y += add.x;
-                vz[k].y += add.y;
-              } else {
-                vx[k].x += add.x;
-                vz[k].x += add.y;
-              }
-            }
-          }
-          float *to = my + k * RS;
-          sts2(to + oVX, vx[k]);
-          sts2(to + oVZ, vz[k]);
-          if (more) push_z(k, vx[k], oVX, vz[k], oVZ, 1);
-        }
-      }
-      if (more) publish_x(vx, oVX, vz, oVZ, 1, at, tag);
-    }
-    if (more) post_z(oVX, oVZ, at, tag);
-    meet(1, more);
-  }
-
-  if (mine) {
-    const fast::Fields out = d.set[parity ^ (n_steps & 1)];
-    float *const dst[5] = {out.vx, out.vz, out.txx, out.tzz, out.txz};
-#pragma unroll
-    for (int k = 0; k < K; ++k) {
-      if (k >= kn) continue;
-      const size_t o = (size_t)(x0 + r0 + k) * ps + z;
-      const float2 v[5] = {vx[k], vz[k], xx[k], zz[k], xz[k]};
-#pragma unroll
-      for (int f = 0; f < 5; ++f) {
-        dst[f][o] = v[f].x;
-        if (z + 1 < nz) dst[f][o + 1] = v[f].y;
-      }
-    }
-    if (!ADJ && dump.base && dump.last && n_steps % dump.every == 0)
-      save(dump.base + (size_t)(n_steps / dump.every) * dump.stride);
-  }
-  if (CLUSTER) cg::this_cluster().sync();
-}
-
-template <bool ADJ, int K, int S, bool CLUSTER>
+template <int MODE, int K, int S, bool CLUSTER>
 __global__ void __launch_bounds__(kMaxThreads, 1)
     resident_steps(const __grid_constant__ tma::SimDesc d, int tiles_x, int tiles_z, int groups,
                    int n_rec, int n_inj, int it0, int n_steps, int parity, int zero, int store,
                    const Dump dump, Word *mail, int *err) {
-  const Team t{(int)blockIdx.x, tiles_x, tiles_z, groups, n_rec, n_inj, mail};
-  member_steps<ADJ, K, S, CLUSTER>(d, t, it0, n_steps, parity, zero != 0, store, dump, err);
+  const Team t{(int)blockIdx.x, tiles_x, tiles_z, groups, n_rec, n_inj, 0, mail};
+  member_steps<MODE, K, S, CLUSTER>(d, t, it0, n_steps, parity, zero != 0, store, dump, RateIo(),
+                                    err);
 }
 
 // Mailbox link: the members' teams side by side in one cooperative launch.
@@ -769,8 +25,9 @@ __global__ void __launch_bounds__(kMaxThreads, 1)
                          int *err) {
   const Member m = members[cta_member[blockIdx.x]];
   const Team t{(int)blockIdx.x - m.first, m.tiles_x, m.tiles_z, m.groups, m.n_rec, m.n_inj,
-               mail + (size_t)m.first * kBox};
-  member_steps<false, K, S, CLUSTER>(sims[m.sim], t, 0, n_steps, 0, true, store, Dump(), err);
+               0, mail + (size_t)m.first * kBox};
+  member_steps<kForward, K, S, CLUSTER>(sims[m.sim], t, 0, n_steps, 0, true, store, Dump(),
+                                        RateIo(), err);
 }
 
 size_t smem_bytes(int Rm, int S, int nr, int n_terms) {
@@ -778,91 +35,10 @@ size_t smem_bytes(int Rm, int S, int nr, int n_terms) {
          (size_t)Rm * (S - 4) * sizeof(unsigned short) + 16;
 }
 
-struct Device {
-  int sms = 0, optin = 0;
-};
-bool device(Device &q) {
-  int dev = 0;
-  return cudaGetDevice(&dev) == cudaSuccess &&
-         cudaDeviceGetAttribute(&q.sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess &&
-         cudaDeviceGetAttribute(&q.optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) ==
-             cudaSuccess;
-}
-
-// Per-device launch attributes of a kernel, set once: the device's largest
-// shared memory, and clusters above the portable size.
-template <class Kern>
-cudaError_t configure(Kern kern, bool cluster, unsigned long long &configured) {
-  int dev = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e != cudaSuccess) return e;
-  const unsigned long long bit = 1ull << (dev & 63);
-  if (configured & bit) return cudaSuccess;
-  int optin = 0;
-  e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-  if (e != cudaSuccess) return e;
-  cudaFuncAttributes fa;
-  e = cudaFuncGetAttributes(&fa, kern);
-  if (e != cudaSuccess) return e;
-  e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           optin - (int)fa.sharedSizeBytes);
-  if (e == cudaSuccess && cluster)
-    e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-  if (e == cudaSuccess) configured |= bit;
-  return e;
-}
-
-// A cluster launch, or a cooperative one: either way a team's CTAs are
-// resident at once, as CTAs that wait on one another require.
-cudaLaunchConfig_t config(cudaLaunchAttribute *attr, bool cluster, int team, int ctas, int threads,
-                          size_t smem, cudaStream_t s) {
-  if (cluster) {
-    attr->id = cudaLaunchAttributeClusterDimension;
-    attr->val.clusterDim.x = team;
-    attr->val.clusterDim.y = 1;
-    attr->val.clusterDim.z = 1;
-  } else {
-    attr->id = cudaLaunchAttributeCooperative;
-    attr->val.cooperative = 1;
-  }
-  cudaLaunchConfig_t lc = {};
-  lc.gridDim = dim3(ctas);
-  lc.blockDim = dim3(threads);
-  lc.dynamicSmemBytes = smem;
-  lc.stream = s;
-  lc.attrs = attr;
-  lc.numAttrs = 1;
-  return lc;
-}
-
-// Calls f with the K, S and link of a plan as compile-time values.
-template <int K_, int S_, bool CL_>
-struct Tag {
-  static constexpr int K = K_, S = S_;
-  static constexpr bool CL = CL_;
-};
-template <class F>
-cudaError_t with_plan(int rows, int stride, bool cluster, F &&f) {
-  if (cluster && stride == kWide) {
-    if (rows == 3) return f(Tag<3, kWide, true>{});
-    if (rows == 4) return f(Tag<4, kWide, true>{});
-    if (rows == 5) return f(Tag<5, kWide, true>{});
-  } else if (cluster && stride == kNarrow) {
-    if (rows == 3) return f(Tag<3, kNarrow, true>{});
-    if (rows == 4) return f(Tag<4, kNarrow, true>{});
-    if (rows == 5) return f(Tag<5, kNarrow, true>{});
-  } else if (stride == kNarrow) {
-    if (rows == 3) return f(Tag<3, kNarrow, false>{});
-    if (rows == 4) return f(Tag<4, kNarrow, false>{});
-    if (rows == 5) return f(Tag<5, kNarrow, false>{});
-  }
-  return cudaErrorInvalidValue;
-}
-
-template <bool ADJ, class T>
+template <int MODE, class T>
 cudaError_t run(T, const tma::SimDesc &d, const Plan &p, int it0, int n_steps, int parity, int zero,
                 int store, const Dump &dump, void *mail, int *err, cudaStream_t s) {
-  auto kern = resident_steps<ADJ, T::K, T::S, T::CL>;
+  auto kern = resident_steps<MODE, T::K, T::S, T::CL>;
   static unsigned long long configured = 0;
   cudaError_t e = configure(kern, T::CL, configured);
   if (e != cudaSuccess) return e;
@@ -989,6 +165,36 @@ Plan plan_mailbox(const Grid &g, int max_ctas, int per_sm) {
   return fit(p, q, g, per_sm) ? p : Plan();
 }
 
+ExactPlan plan_exact(const Grid &g, int lanes) {
+  Device q;
+  ExactPlan e;
+  if (!device(q) || lanes < 1) return e;
+  // Fills what the adjoint adds to a plan; false when it does not fit.
+  auto complete = [&](const Plan &p) {
+    if (p.ctas() <= 0) return false;
+    const int P = pairs(g.nz), C = (P + p.tiles_z - 1) / p.tiles_z;
+    const int R = (g.nx + p.tiles_x - 1) / p.tiles_x;
+    const size_t cw = p.cluster ? (p.groups * C + 31) / 32 * 32 : 32 * p.groups;
+    const size_t rates = 5 * (size_t)p.rows * cw * sizeof(float2);
+    e.p = p;
+    e.n_src = 0;
+    for (const auto &cells : g.sources)
+      e.n_src = std::max(e.n_src, most_per_tile(p, g.nx, g.nz, cells));
+    e.rate_stride = p.ctas() * rates / sizeof(float2);
+    e.smem = p.smem + rates + (size_t)3 * R * (p.stride - 4) * sizeof(float) +
+             (size_t)e.n_src * 12 + (size_t)R * (p.stride - 4) * sizeof(unsigned short);
+    return e.smem + 64 <= (size_t)q.optin;
+  };
+  for (int nc = kMaxCluster; nc >= 1; --nc) {
+    const Plan p = plan_cluster(g, nc);
+    if (p.ctas() <= 0) continue;
+    if (complete(p)) return e;
+    break;  // fewer CTAs hold less
+  }
+  if (complete(plan_mailbox(g, q.sms / lanes, 1))) return e;
+  return ExactPlan();
+}
+
 size_t mailbox_bytes(const Plan &p) {
   return p.cluster ? 0 : (size_t)p.ctas() * kBox * sizeof(Word);
 }
@@ -1004,8 +210,8 @@ cudaError_t steps(const tma::SimDesc &d, const Plan &p, bool adjoint, int it0, i
   }
   const int z = zero ? 1 : 0, st = store ? 1 : 0;
   return with_plan(p.rows, p.stride, p.cluster, [&](auto t) {
-    return adjoint ? run<true>(t, d, p, it0, n_steps, parity, z, st, dump, mail, err, s)
-                   : run<false>(t, d, p, it0, n_steps, parity, z, st, dump, mail, err, s);
+    return adjoint ? run<kAdjoint>(t, d, p, it0, n_steps, parity, z, st, dump, mail, err, s)
+                   : run<kForward>(t, d, p, it0, n_steps, parity, z, st, dump, mail, err, s);
   });
 }
 

@@ -19,7 +19,7 @@ def rel(a, b):
     return np.linalg.norm(a - b) / np.linalg.norm(b)
 
 
-def model(nx, nz, nt=120, npb=6, seed=0, shots=1, precision="fp32"):
+def model(nx, nz, nt=120, npb=6, seed=0, shots=1, precision="fp32", near=False):
     nxi, nzi = nx - 2 * npb, nz - 2 * npb
     rng = np.random.default_rng(seed + 1000 * nx + nz)
     # Two sources of a shot at the same point: several terms per cell. Two
@@ -28,6 +28,9 @@ def model(nx, nz, nt=120, npb=6, seed=0, shots=1, precision="fp32"):
     zs = [int(rng.integers(1, nzi - 1)) for _ in range(shots)]
     rx = [int(v) for v in rng.integers(0, nxi, 9)]
     rz = [int(v) for v in rng.integers(0, nzi, 9)]
+    if near:  # where the wave of 120 steps arrives
+        rx = [min(max(xs[0] + int(v), 0), nxi - 1) for v in rng.integers(-8, 9, 9)]
+        rz = [min(max(zs[0] + int(v), 0), nzi - 1) for v in rng.integers(-8, 9, 9)]
     p = dict(nt=nt, nx_inner=nxi, nz_inner=nzi, nx_inner_boundary=1, nz_inner_boundary=1,
              dx=1.249, dz=1.3, dt=2.5e-4, np_boundary=npb, np_factor=0.05, scalar_rho=1500.0,
              scalar_vp=2000.0, scalar_vs=800.0, npx=1, npz=1, peak_frequency=90.0,
@@ -149,3 +152,25 @@ def test_resident_fp64_equals_two_kernel_steps_bit_for_bit(nx, nz, tmp_path, mon
                    m.get_wavefields())
     for steps, resident, pieces in zip(*out):
         assert np.array_equal(resident, steps) and np.array_equal(pieces, steps)
+
+
+@pytest.mark.parametrize("nx,nz,shots", [(20, 16, 1), (17, 23, 3), (68, 57, 1), (64, 66, 2),
+                                         (250, 151, 1), (250, 151, 5), (31, 700, 1),
+                                         (400, 300, 1), (400, 300, 3), (401, 257, 2),
+                                         (700, 515, 1), (900, 700, 1)])
+def test_resident_exact_gradient_is_as_accurate_as_per_step_launches(nx, nz, shots):
+    # Clusters and mailboxes, shots on shares of the device and one after the
+    # other, one and several segments, a grid that only the forward steps hold.
+    # Same criterion as above; sums in float-float pairs add nothing to it.
+    out = []
+    for variant, ck in (("fp64", 50), ("fused_tma", 50), (None, 50), (None, 0), (None, 7)):
+        m = model(nx, nz, shots=shots, near=True, precision="fp64" if variant == "fp64" else "fp32")
+        if variant == "fused_tma":
+            m.kernel_variant = variant
+        m.set_observed_data(*[np.zeros_like(a) for a in m.get_observed_data()])
+        for _ in range(3 if variant is None else 1):  # eager, graph capture, graph replay
+            misfit, g = m.exact_gradient(ck)
+        out.append([np.array([misfit])] + list(g))
+    for exact, per_step, resident, whole, sevenths in zip(*out):
+        assert rel(resident, exact) <= max(2 * rel(per_step, exact), 1e-6)
+        assert np.array_equal(resident, whole) and np.array_equal(resident, sevenths)
