@@ -631,7 +631,7 @@ size_t Model::exact_resident_bytes(int C, const resident::ExactPlan &p) const {
   const size_t state = 5 * padded_size() * sizeof(float);
   const size_t n_ck = (nt + C - 1) / C;
   return n_ck * state + C * p.rate_stride * sizeof(float2) + state +
-         3 * padded_size() * sizeof(float) +
+         3 * (1 + resident::log_entries(C, kFlushSteps)) * padded_size() * sizeof(float) +
          2 * static_cast<size_t>(cfg_.nr) * nt * sizeof(float) + resident::mailbox_bytes(p.p);
 }
 
@@ -1095,7 +1095,8 @@ double Model::exact_gradient_lanes(int C, const std::vector<int> &shot_list) {
       ensure(l->lam, kLamPlanes * field_bytes);
     }
     ensure(l->raw, std::max<size_t>(2 * static_cast<size_t>(nr) * nt * sizeof(float), 16));
-    ensure(l->part, gp * (sizeof(float2) + sizeof(float)));
+    ensure(l->part, 3 * gp * sizeof(float) *
+                        (on_chip_lanes > 0 ? 1 + resident::log_entries(C, kFlushSteps) : 1));
   }
   for (auto &b : gex_) ensure(b, g * sizeof(double));
   for (auto &b : kexact_) ensure(b, g * sizeof(double));
@@ -1190,6 +1191,7 @@ double Model::exact_gradient_lanes(int C, const std::vector<int> &shot_list) {
       x.rates = rates;
       x.src = plans_[shot];
       x.part = l.part.as<float>();
+      x.log = x.part + 3 * gp;
       x.sums[0] = gs;
       x.sums[1] = gs + 2 * g;
       x.sums[2] = gs + 3 * g;

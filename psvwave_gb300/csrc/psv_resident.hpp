@@ -79,12 +79,13 @@ cudaError_t steps(const tma::SimDesc &d, const Plan &p, bool adjoint, int it0, i
 
 // The split of an exact gradient of one simulation: forward steps that keep
 // their rates, and the exact adjoint's steps, on the same tiles. n_src: the
-// most source points of a tile; smem: the adjoint's. lanes: how many run at
+// most source points of a tile; smem, rate_smem: the adjoint's and the keeping
+// forward steps'. lanes: how many run at
 // once, each on its share of the device.
 struct ExactPlan {
   Plan p;
   int n_src = 0;
-  size_t smem = 0;
+  size_t smem = 0, rate_smem = 0;
   size_t rate_stride = 0;  // float2 per step
 };
 ExactPlan plan_exact(const Grid &g, int lanes);
@@ -99,17 +100,21 @@ cudaError_t steps_keeping_rates(const tma::SimDesc &d, const ExactPlan &p, int i
 // down to first: d.set[0] holds l of the last of them (zero: it is zero)
 // and takes l of the first; d.plan's terms add the series a_ux, a_uz to the
 // adjoint velocities. The gradients of lm, mu (with lambda = lm - 2 mu) and b
-// go into `sums`, float-float pairs, every `flush` steps; between launches
-// what is not in them yet is in part (three planes of nx * pitch).
+// are summed in FP32 for `flush` steps at a time, which are logged (log: three
+// planes of nx * pitch for each multiple of `flush` among the steps) and then
+// added to float-float pairs `sums` of nx * nz, later steps first; what a
+// launch leaves unlogged it hands to the next in part (three planes).
 struct ExactSteps {
   int first = 0, n_steps = 0;
   bool zero = false;
   const float2 *rates = nullptr;
   InjPlan src{};  // the shot's source terms
-  float *part = nullptr;
+  float *part = nullptr, *log = nullptr;
   float2 *sums[3] = {nullptr, nullptr, nullptr};
   int flush = 1;
 };
+// Entries of the log for n_steps steps at most.
+inline int log_entries(int n_steps, int flush) { return (n_steps - 1) / flush + 1; }
 cudaError_t exact_steps(const tma::SimDesc &d, const ExactPlan &p, const ExactSteps &x,
                         void *mail, int *err, cudaStream_t s);
 

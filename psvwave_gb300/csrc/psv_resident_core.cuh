@@ -152,16 +152,17 @@ struct Team {
 // Rates kept by kRates and read by kExact: per step (from step `first` on) and
 // CTA, five quantities of every thread's rows -- e_x, e_z, g_xz, then the
 // accelerations a_x, a_z, all times dt. kExact also: the shot's source terms,
-// the sums between launches (lm, mu, b: planes of nx * pitch), and the
-// gradients' pairs (nx * nz), into which the sums go every `flush` steps.
+// the sums between launches (lm, mu, b: planes of nx * pitch), and the log into
+// which they go every `flush` steps: those of step n to entry n / flush -
+// first_log, three such planes.
 struct RateIo {
   float2 *rates = nullptr;
   size_t stride = 0;
   int first = 0;
   InjPlan src{};
   float *part = nullptr;
-  float2 *sums[3] = {nullptr, nullptr, nullptr};
-  int flush = 1;
+  float *log = nullptr;
+  int flush = 1, first_log = 0;
 };
 
 // What member_steps runs: forward steps, the reference's adjoint steps, forward
@@ -182,12 +183,17 @@ __device__ __forceinline__ void bulk_load(void *to, const void *from, uint32_t b
       "l"(from), "r"(bytes), "r"(tma::smem_u32(bar))
       : "memory");
 }
-// (hi, lo) + x with the rounding error kept in lo (Knuth's TwoSum).
-__device__ __forceinline__ float2 ff_add(float2 a, float x) {
-  const float s = a.x + x;
-  const float bp = s - a.x;
-  const float e = (a.x - (s - bp)) + (x - bp);
-  return make_float2(s, a.y + e);
+// And back (the writes to shared memory it reads must be ordered before it with
+// a proxy fence); wait_stored: the group's shared memory may be reused.
+__device__ __forceinline__ void bulk_store(void *to, const void *from, uint32_t bytes) {
+  asm volatile(
+      "cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;\n"
+      "cp.async.bulk.commit_group;" ::"l"(to),
+      "r"(tma::smem_u32(from)), "r"(bytes)
+      : "memory");
+}
+__device__ __forceinline__ void wait_stored() {
+  asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
 }
 __device__ __forceinline__ float2 mul2(float2 a, float2 b) {
   return make_float2(__fmul_rn(a.x, b.x), __fmul_rn(a.y, b.y));
@@ -210,21 +216,23 @@ __device__ __forceinline__ void member_steps(const tma::SimDesc &d, const Team &
   const int Rm = (nx + tm.tiles_x - 1) / tm.tiles_x;
   float *const F = reinterpret_cast<float *>(smem_raw);
   const InjPlan &pl = d.plan;
-  // kExact: the step's rates (three for the stresses, two for the velocities)
-  // of every thread's rows, and the points' gradient sums of lm, mu and b.
+  // kRates, kExact: the step's rates (three for the stresses, two for the
+  // velocities) of every thread's rows; kExact: the points' gradient sums of lm,
+  // mu and b, and b T (in registers, with the rest, it made K = 5 spill).
   const int CW = CLUSTER ? (tm.groups * ((pairs(nz) + tm.tiles_z - 1) / tm.tiles_z) + 31) & ~31
                          : 32 * tm.groups;
   float2 *const rate_a = reinterpret_cast<float2 *>(F + (Rm + 4) * RS);
-  float2 *const rate_b = rate_a + (EX ? 3 * K * CW : 0);
-  float *const G = reinterpret_cast<float *>(rate_b + (EX ? 2 * K * CW : 0));
+  float2 *const rate_b = rate_a + (EX || RATES ? 3 * K * CW : 0);
+  float *const G = reinterpret_cast<float *>(rate_b + (EX || RATES ? 2 * K * CW : 0));
   // Injection points of the tile: the value each adds this step (vx, vz), its
   // first term, and the points' slots by (row, column); then receivers.
-  float2 *const INJ = reinterpret_cast<float2 *>(G + (EX ? 3 * Rm * (S - 4) : 0));
+  float2 *const INJ = reinterpret_cast<float2 *>(G + (EX ? 4 * Rm * (S - 4) : 0));
   const int n_points = tm.n_inj + (EX ? tm.n_src : 0);  // kExact: then source points
   int *const inj_first = reinterpret_cast<int *>(INJ + n_points);
   int *const rec_off = inj_first + n_points, *const rec_id = rec_off + tm.n_rec;
   unsigned short *const slot_of = reinterpret_cast<unsigned short *>(rec_off + 2 * tm.n_rec);
-  unsigned short *const src_slot_of = slot_of + Rm * (S - 4);  // kExact
+  // kExact: bytes, of injection points and of source points.
+  unsigned char *const slots_of = reinterpret_cast<unsigned char *>(slot_of);
   __shared__ int s_count[3];
   __shared__ __align__(8) uint64_t s_bar[2];  // of stress and velocity half-steps
   __shared__ __align__(8) uint64_t s_rate[2];  // kExact: of the rates' copies
@@ -271,17 +279,21 @@ __device__ __forceinline__ void member_steps(const tma::SimDesc &d, const Team &
       const int q = atomicAdd(&s_count[0], 1);
       inj_first[q] = i;
       INJ[q] = make_float2(0.f, 0.f);
-      slot_of[(ix - x0) * (S - 4) + iz - z0] = (unsigned short)q;
+      const int at = (ix - x0) * (S - 4) + iz - z0;
+      if (EX)
+        slots_of[2 * at] = (unsigned char)q;
+      else
+        slot_of[at] = (unsigned short)q;
     }
   }
   if (EX)
     for (int i = tid; i < io.src.n; i += NT) {
       const int cell = io.src.terms[i].cell, ix = cell / nz, iz = cell - ix * nz;
       if (in_tile(ix, iz) && (i == 0 || io.src.terms[i - 1].cell != cell)) {
-        const int q = tm.n_inj + atomicAdd(&s_count[2], 1);
-        inj_first[q] = i;
-        INJ[q] = make_float2(0.f, 0.f);
-        src_slot_of[(ix - x0) * (S - 4) + iz - z0] = (unsigned short)q;
+        const int q = atomicAdd(&s_count[2], 1);
+        inj_first[tm.n_inj + q] = i;
+        INJ[tm.n_inj + q] = make_float2(0.f, 0.f);
+        slots_of[2 * ((ix - x0) * (S - 4) + iz - z0) + 1] = (unsigned char)q;
       }
     }
   if (!BACK)
@@ -349,11 +361,11 @@ __device__ __forceinline__ void member_steps(const tma::SimDesc &d, const Team &
       bb[k].y = b.y;
       tp[k].y = taper_at(x, z + 1);
     }
-    if (EX) bb[k] = scale(x, z);
     if (EX) {
+      sts2(G + ((r0 + k) * 4 + 3) * (S - 4) + 2 * c, scale(x, z));
       const size_t gp = (size_t)nx * ps, o = (size_t)x * ps + z;
       for (int p = 0; p < 3; ++p)
-        sts2(G + ((r0 + k) * 3 + p) * (S - 4) + 2 * c,
+        sts2(G + ((r0 + k) * 4 + p) * (S - 4) + 2 * c,
              zero ? zero2 : *reinterpret_cast<const float2 *>(io.part + p * gp + o));
       if (io.src.n && x >= io.src.x0 && x < io.src.x0 + io.src.w)
         for (int e = 0; e < 2; ++e)
@@ -602,6 +614,19 @@ __device__ __forceinline__ void member_steps(const tma::SimDesc &d, const Team &
     };
     fetch(0, 0);
     fetch(0, 1);
+    // kRates: a step's rates go out after its half-steps' barriers, while the
+    // next half-step runs (stored by every thread as they were formed, they
+    // stood before the edge words: 6.9 us a step at 1100 x 500 against 4.6
+    // without rates).
+    auto put = [&](int j, int half) {
+      if (!RATES || ct != 0) return;
+      float2 *to = io.rates + (size_t)(it0 + j - io.first) * io.stride + (size_t)tm.k * 5 * K * CW +
+                   (half ? 3 * K * CW : 0);
+      bulk_store(to, half ? rate_b : rate_a, (half ? 2 : 3) * rate_bytes);
+    };
+    auto put_done = [&] {
+      if (RATES && ct == 0) wait_stored();
+    };
     for (int j = 0; j < n_steps; ++j) {
       const int it = BACK ? it0 - j : it0 + j;
       const uint32_t tag = (uint32_t)(j + 1);
@@ -622,12 +647,17 @@ __device__ __forceinline__ void member_steps(const tma::SimDesc &d, const Team &
       }
       for (int i = ct + CT; i < n_items; i += CT) values[place(i)] = item_value(i, it, 0);
       receive(0, tag);
+      put_done();
       meet(0, true);
       fetch(j + 1, 0);
+      put(j, 0);
       if (more) receive(1, tag);
+      put_done();
       meet(1, more);
       fetch(j + 1, 1);
+      put(j, 1);
     }
+    put_done();
     if (CLUSTER) cg::this_cluster().sync();
     return;
   }
@@ -716,8 +746,8 @@ __device__ __forceinline__ void member_steps(const tma::SimDesc &d, const Team &
   // The fields that a half-step's stencils read, row k of the run. kExact: the
   // scaled adjoint velocities w = b T l_v, and p = C T l_t (px, pz, q in the
   // places of txx, tzz, txz).
-  auto f_vx = [&](int k) { return EX ? mul2(bb[k], vx[k]) : vx[k]; };
-  auto f_vz = [&](int k) { return EX ? mul2(bb[k], vz[k]) : vz[k]; };
+  auto f_vx = [&](int k) { return EX ? lds2(my + k * RS + oVX) : vx[k]; };
+  auto f_vz = [&](int k) { return EX ? lds2(my + k * RS + oVZ) : vz[k]; };
   auto la_of = [&](int k) {
     return make_float2(__fmaf_rn(-2.f, mu[k].x, lm[k].x), __fmaf_rn(-2.f, mu[k].y, lm[k].y));
   };
@@ -733,11 +763,13 @@ __device__ __forceinline__ void member_steps(const tma::SimDesc &d, const Team &
   };
   auto f_xz = [&](int k) { return EX ? mul2(mu[k], xz[k]) : xz[k]; };
   // kRates: keeps rate q of row k, 0 outside the updated region.
-  float2 *keep_at = nullptr;
   auto keep = [&](int q, int k, float a, float b) {
     if (!(inside >> (2 * k) & 1u)) a = 0.f;
     if (!(inside >> (2 * k) & 2u)) b = 0.f;
-    keep_at[(q * K + k) * CW] = make_float2(a, b);
+    rate_a[(q * K + k) * CW + tid] = make_float2(a, b);
+  };
+  auto kept = [&] {
+    if (RATES) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   };
   // kExact: waits for the rates of half-step `half`.
   bool rates_in = true;
@@ -790,8 +822,6 @@ __device__ __forceinline__ void member_steps(const tma::SimDesc &d, const Team &
       }
     }
     const uint32_t tag = (uint32_t)(j + 1);
-    if (RATES)
-      keep_at = io.rates + (size_t)(it - io.first) * io.stride + (size_t)tm.k * 5 * K * CW + tid;
     // ---- stresses ----
     int at = box_at(0, tag);
     if (mine) {
@@ -837,7 +867,7 @@ __device__ __forceinline__ void member_steps(const tma::SimDesc &d, const Team &
             // e_z + y_zz e_x): the forward step forms lambda = lm - 2 mu.
             const float2 rx = rate_a[k * CW + tid], rz = rate_a[(K + k) * CW + tid],
                          rg = rate_a[(2 * K + k) * CW + tid];
-            float *const sum = G + (r0 + k) * 3 * (S - 4) + 2 * c;
+            float *const sum = G + (r0 + k) * 4 * (S - 4) + 2 * c;
             float2 sl = lds2(sum), sm = lds2(sum + (S - 4));
             sl.x = __fmaf_rn(__fadd_rn(xx[k].x, zz[k].x), __fadd_rn(rx.x, rz.x), sl.x);
             sl.y = __fmaf_rn(__fadd_rn(xx[k].y, zz[k].y), __fadd_rn(rx.y, rz.y), sl.y);
@@ -868,6 +898,7 @@ __device__ __forceinline__ void member_steps(const tma::SimDesc &d, const Team &
       publish_x(f_xz, oXZ, f_xx, oXX, 0, at, tag);
     }
     post_z(oZZ, oXZ, at, tag);
+    kept();
     meet(0, true);
     // ---- velocities ----
     at = box_at(1, tag);
@@ -907,7 +938,7 @@ __device__ __forceinline__ void member_steps(const tma::SimDesc &d, const Team &
             // v-bar = T l_v + E^T p.
             const float2 ra = rate_b[k * CW + tid], rb = rate_b[(K + k) * CW + tid];
             const float2 tx = mul2(tp[k], vx[k]), tz = mul2(tp[k], vz[k]);
-            float *const sum = G + ((r0 + k) * 3 + 2) * (S - 4) + 2 * c;
+            float *const sum = G + ((r0 + k) * 4 + 2) * (S - 4) + 2 * c;
             float2 sb = lds2(sum);
             sb.x = __fadd_rn(sb.x, __fmaf_rn(tx.x, ra.x, __fmul_rn(tz.x, rb.x)));
             sb.y = __fadd_rn(sb.y, __fmaf_rn(tx.y, ra.y, __fmul_rn(tz.y, rb.y)));
@@ -915,7 +946,7 @@ __device__ __forceinline__ void member_steps(const tma::SimDesc &d, const Team &
 #pragma unroll
               for (int e = 0; e < 2; ++e) {
                 if (!(src_mask >> (2 * k + e) & 1u)) continue;
-                const float2 add = INJ[src_slot_of[(r0 + k) * (S - 4) + 2 * c + e]];
+                const float2 add = INJ[tm.n_inj + slots_of[2 * ((r0 + k) * (S - 4) + 2 * c + e) + 1]];
                 if (e)
                   sb.y += add.x * vx[k].y + add.y * vz[k].y;
                 else
@@ -935,7 +966,8 @@ __device__ __forceinline__ void member_steps(const tma::SimDesc &d, const Team &
 #pragma unroll
             for (int e = 0; e < 2; ++e) {
               if (!(inj_mask >> (2 * k + e) & 1u)) continue;
-              const float2 add = INJ[slot_of[(r0 + k) * (S - 4) + 2 * c + e]];
+              const int p = (r0 + k) * (S - 4) + 2 * c + e;
+              const float2 add = INJ[EX ? slots_of[2 * p] : slot_of[p]];
               if (e) {
                 vx[k].y += add.x;
                 vz[k].y += add.y;
@@ -946,32 +978,33 @@ __device__ __forceinline__ void member_steps(const tma::SimDesc &d, const Team &
             }
           }
           float *to = my + k * RS;
-          const float2 wx = f_vx(k), wz = f_vz(k);
+          float2 wx = vx[k], wz = vz[k];
+          if (EX) {
+            const float2 w = lds2(G + ((r0 + k) * 4 + 3) * (S - 4) + 2 * c);
+            wx = mul2(w, wx);
+            wz = mul2(w, wz);
+          }
           sts2(to + oVX, wx);
           sts2(to + oVZ, wz);
           if (more) push_z(k, wx, oVX, wz, oVZ, 1);
         }
       }
       if (more) publish_x(f_vx, oVX, f_vz, oVZ, 1, at, tag);
-      // kExact: the sums go into the gradients' float-float pairs every so often.
+      // kExact: every so often the sums go out and start again.
       if (EX && it % io.flush == 0) {
-#pragma unroll
-        for (int k = 0; k < K; ++k) {
-          if (k >= kn) continue;
-          float *const sum = G + (r0 + k) * 3 * (S - 4) + 2 * c;
-#pragma unroll
-          for (int e = 0; e < 2; ++e) {
-            if (!((inside | src_mask) >> (2 * k + e) & 1u)) continue;
-            const size_t u = (size_t)(x0 + r0 + k) * nz + z + e;
-            for (int p = 0; p < 3; ++p) {
-              io.sums[p][u] = ff_add(io.sums[p][u], sum[p * (S - 4) + e]);
-              sum[p * (S - 4) + e] = 0.f;
-            }
+        float *to = io.log + (size_t)(it / io.flush - io.first_log) * 3 * nx * ps +
+                    (size_t)(x0 + r0) * ps + z;
+        float *sum = G + r0 * 4 * (S - 4) + 2 * c;
+#pragma unroll 1
+        for (int k = 0; k < kn; ++k, to += ps, sum += 4 * (S - 4))
+          for (int p = 0; p < 3; ++p) {
+            sts2(to + (size_t)p * nx * ps, lds2(sum + p * (S - 4)));
+            sts2(sum + p * (S - 4), zero2);
           }
-        }
       }
     }
     if (more) post_z(oVX, oVZ, at, tag);
+    kept();
     meet(1, more);
   }
 
@@ -991,7 +1024,7 @@ __device__ __forceinline__ void member_steps(const tma::SimDesc &d, const Team &
       if (EX)
         for (int p = 0; p < 3; ++p)
           *reinterpret_cast<float2 *>(io.part + (size_t)p * nx * ps + o) =
-              lds2(G + ((r0 + k) * 3 + p) * (S - 4) + 2 * c);
+              lds2(G + ((r0 + k) * 4 + p) * (S - 4) + 2 * c);
     }
   }
   if (CLUSTER) cg::this_cluster().sync();

@@ -49,8 +49,26 @@ cudaError_t run(T, const tma::SimDesc &d, const ExactPlan &q, int it0, int n_ste
                   static_cast<Word *>(mail)};
   cudaLaunchAttribute attr;
   cudaLaunchConfig_t lc = config(&attr, T::CL, p.ctas(), p.ctas(), p.threads,
-                                 MODE == kExact ? q.smem : p.smem, s);
+                                 MODE == kExact ? q.smem : q.rate_smem, s);
   return cudaLaunchKernelEx(&lc, kern, d, team, it0, n_steps, zero ? 1 : 0, io, err);
+}
+
+// Adds the log's entries to the pairs, the last entry first, with each addition's
+// rounding error kept in lo (Knuth's TwoSum).
+__global__ void __launch_bounds__(128) add_log(int nx, int nz, int pitch, int entries,
+                                               const float *log, float2 *a, float2 *b, float2 *c) {
+  const int iz = blockIdx.x * blockDim.x + threadIdx.x, ix = blockIdx.y, p = blockIdx.z;
+  if (iz >= nz) return;
+  float2 *const to = (p == 0 ? a : p == 1 ? b : c) + (size_t)ix * nz + iz;
+  const size_t plane = (size_t)nx * pitch;
+  const float *from = log + p * plane + (size_t)ix * pitch + iz;
+  float2 v = *to;
+  for (int k = entries - 1; k >= 0; --k) {
+    const float x = from[(size_t)k * 3 * plane];
+    const float s = v.x + x, t = s - v.x;
+    v = make_float2(s, v.y + ((v.x - (s - t)) + (x - t)));
+  }
+  *to = v;
 }
 
 }  // namespace
@@ -76,11 +94,17 @@ cudaError_t exact_steps(const tma::SimDesc &d, const ExactPlan &p, const ExactSt
   io.first = x.first;
   io.src = x.src;
   io.part = x.part;
-  for (int k = 0; k < 3; ++k) io.sums[k] = x.sums[k];
+  io.log = x.log;
   io.flush = x.flush;
-  return with_plan(p.p.rows, p.p.stride, p.p.cluster, [&](auto t) {
+  io.first_log = (x.first + x.flush - 1) / x.flush;
+  cudaError_t e = with_plan(p.p.rows, p.p.stride, p.p.cluster, [&](auto t) {
     return run<kExact>(t, d, p, x.first + x.n_steps - 1, x.n_steps, x.zero, io, mail, err, s);
   });
+  const int entries = (x.first + x.n_steps - 1) / x.flush - io.first_log + 1;
+  if (e != cudaSuccess || entries <= 0) return e;
+  const dim3 grid((d.nz + 127) / 128, d.nx, 3);
+  add_log<<<grid, 128, 0, s>>>(d.nx, d.nz, d.pitch, entries, x.log, x.sums[0], x.sums[1], x.sums[2]);
+  return cudaGetLastError();
 }
 
 }  // namespace resident

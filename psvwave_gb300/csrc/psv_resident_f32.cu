@@ -181,8 +181,9 @@ ExactPlan plan_exact(const Grid &g, int lanes) {
     for (const auto &cells : g.sources)
       e.n_src = std::max(e.n_src, most_per_tile(p, g.nx, g.nz, cells));
     e.rate_stride = p.ctas() * rates / sizeof(float2);
-    e.smem = p.smem + rates + (size_t)3 * R * (p.stride - 4) * sizeof(float) +
-             (size_t)e.n_src * 12 + (size_t)R * (p.stride - 4) * sizeof(unsigned short);
+    e.rate_smem = p.smem + rates;
+    e.smem = e.rate_smem + (size_t)4 * R * (p.stride - 4) * sizeof(float) + (size_t)e.n_src * 12;
+    if (p.n_inj > 256 || e.n_src > 256) return false;  // byte tables
     return e.smem + 64 <= (size_t)q.optin;
   };
   for (int nc = kMaxCluster; nc >= 1; --nc) {
