@@ -145,7 +145,7 @@ void Batch::pack() {
     for (size_t i = 0; i < set.size(); ++i) {
       const resident::Plan &p = set[i].p;
       members.push_back(resident::Member{set[i].k, l.ctas, p.tiles_x, p.tiles_z, p.groups, p.n_rec,
-                                         p.n_inj});
+                                         p.n_inj, p.n_term});
       ctas.insert(ctas.end(), p.ctas(), static_cast<int>(i));
       l.ctas += p.ctas();
       l.rows = std::max(l.rows, p.rows);

@@ -411,12 +411,15 @@ resident::Grid Model::resident_grid() const {
   g.nz = geo_.nz;
   for (int r = 0; r < cfg_.nr; ++r) g.receivers.push_back(ix_rec_[r] * geo_.nz + iz_rec_[r]);
   for (const auto &shot : cfg_.shots) {
-    std::vector<int> cells;
+    std::vector<int> cells, terms;
     for (int s : shot) {
       // The points of a source's stencil (build_plans).
       const int c = ix_src_[s] * geo_.nz + iz_src_[s], nz = geo_.nz;
       for (int o : {-nz - 1, -nz, -nz + 1, -1, 0, 1, nz - 1, nz}) cells.push_back(c + o);
+      for (int o : {-nz, 0, -1, 0, -nz + 1, 1, -nz - 1, -1, nz - 1, nz, -nz - 1, -nz})
+        terms.push_back(c + o);
     }
+    g.terms.push_back(terms);
     std::sort(cells.begin(), cells.end());
     cells.erase(std::unique(cells.begin(), cells.end()), cells.end());
     g.sources.push_back(cells);

@@ -21,21 +21,21 @@ namespace psv {
 namespace resident {
 
 // A grid to split: its size, and the cells (ix nz + iz) of its receivers
-// and of each shot's injection points.
+// of each shot's injection points, and of its injection terms (a cell per term).
 struct Grid {
   int nx = 0, nz = 0;
   std::vector<int> receivers;
-  std::vector<std::vector<int>> sources;
+  std::vector<std::vector<int>> sources, terms;
 };
 
 // How one simulation is split: tiles_x x tiles_z CTAs, blocks of `threads`
 // with `groups` thread groups of at most `rows` rows each, shared rows of
-// `stride` floats; n_rec, n_inj: the most receivers and injection points of a
-// tile. cluster: the team is one thread-block cluster; otherwise its edges go
+// `stride` floats; n_rec, n_inj, n_term: the most receivers, injection points
+// and terms of a tile. cluster: the team is one thread-block cluster; otherwise its edges go
 // through mailboxes. No CTAs: the grid does not fit.
 struct Plan {
   int tiles_x = 0, tiles_z = 0, groups = 0, rows = 0, threads = 0, stride = 0;
-  int n_rec = 0, n_inj = 0;
+  int n_rec = 0, n_inj = 0, n_term = 0;
   bool cluster = false;
   size_t smem = 0;
   int ctas() const { return tiles_x * tiles_z; }
@@ -84,7 +84,7 @@ cudaError_t steps(const tma::SimDesc &d, const Plan &p, bool adjoint, int it0, i
 // once, each on its share of the device.
 struct ExactPlan {
   Plan p;
-  int n_src = 0;
+  int n_src = 0, n_term = 0;
   size_t smem = 0, rate_smem = 0;
   size_t rate_stride = 0;  // float2 per step
 };
@@ -123,7 +123,7 @@ cudaError_t exact_steps(const tma::SimDesc &d, const ExactPlan &p, const ExactSt
 // One member of a batched launch: its CTAs first .. first + tiles_x tiles_z - 1
 // run simulation `sim` of the table.
 struct Member {
-  int sim, first, tiles_x, tiles_z, groups, n_rec, n_inj;
+  int sim, first, tiles_x, tiles_z, groups, n_rec, n_inj, n_term;
 };
 // One launch: CTAs first_cta .. first_cta + ctas - 1 of the CTA table (the
 // launch's member of each), members from first_member on. team > 0: clusters

@@ -145,7 +145,8 @@ __device__ __forceinline__ float diff_add(float acc, float a1, float p, float m,
 
 struct Team {
   int k, tiles_x, tiles_z, groups;
-  int n_rec, n_inj, n_src;  // most receivers, injection points and (kExact) sources of a tile
+  // Most receivers, injection points, source points (kExact) and terms of a tile.
+  int n_rec, n_inj, n_src, n_term;
   Word *mail;  // mailbox link: boxes of the team's CTA 0
 };
 
@@ -224,16 +225,21 @@ __device__ __forceinline__ void member_steps(const tma::SimDesc &d, const Team &
   float2 *const rate_a = reinterpret_cast<float2 *>(F + (Rm + 4) * RS);
   float2 *const rate_b = rate_a + (EX || RATES ? 3 * K * CW : 0);
   float *const G = reinterpret_cast<float *>(rate_b + (EX || RATES ? 2 * K * CW : 0));
-  // Injection points of the tile: the value each adds this step (vx, vz), its
-  // first term, and the points' slots by (row, column); then receivers.
-  float2 *const INJ = reinterpret_cast<float2 *>(G + (EX ? 4 * Rm * (S - 4) : 0));
+  // Injection terms of the tile (weight, next sample, series, field); its
+  // injection points: the value each adds this step (vx, vz), its first term and
+  // their number (<< 16), and the points' slots by (row, column); receivers.
+  double *const term_w = reinterpret_cast<double *>(G + (EX ? 4 * Rm * (S - 4) : 0));
+  double *const term_next = term_w + tm.n_term;
+  const double **const term_src = reinterpret_cast<const double **>(term_next + tm.n_term);
+  float2 *const INJ = reinterpret_cast<float2 *>(term_src + tm.n_term);
   const int n_points = tm.n_inj + (EX ? tm.n_src : 0);  // kExact: then source points
-  int *const inj_first = reinterpret_cast<int *>(INJ + n_points);
-  int *const rec_off = inj_first + n_points, *const rec_id = rec_off + tm.n_rec;
+  uint32_t *const inj_terms = reinterpret_cast<uint32_t *>(INJ + n_points);
+  int *const term_field = reinterpret_cast<int *>(inj_terms + n_points);
+  int *const rec_off = term_field + tm.n_term, *const rec_id = rec_off + tm.n_rec;
   unsigned short *const slot_of = reinterpret_cast<unsigned short *>(rec_off + 2 * tm.n_rec);
   // kExact: bytes, of injection points and of source points.
   unsigned char *const slots_of = reinterpret_cast<unsigned char *>(slot_of);
-  __shared__ int s_count[3];
+  __shared__ int s_count[4];
   __shared__ __align__(8) uint64_t s_bar[2];  // of stress and velocity half-steps
   __shared__ __align__(8) uint64_t s_rate[2];  // kExact: of the rates' copies
   const int tid = threadIdx.x, NT = blockDim.x;
@@ -255,7 +261,7 @@ __device__ __forceinline__ void member_steps(const tma::SimDesc &d, const Team &
 
   // Shared fields (halo rows and columns at the grid's edges stay zero).
   for (int i = tid; i < (Rm + 4) * RS; i += NT) F[i] = 0.f;
-  if (tid < 3) s_count[tid] = 0;
+  if (tid < 4) s_count[tid] = 0;
   if (EX && tid == 0)
     for (int k = 0; k < 2; ++k)
       asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(tma::smem_u32(&s_rate[k])),
@@ -272,30 +278,48 @@ __device__ __forceinline__ void member_steps(const tma::SimDesc &d, const Team &
   auto in_tile = [&](int ix, int iz) {
     return ix >= x0 && ix < x0 + R && iz >= z0 && iz < z0 + 2 * C;
   };
-  // The tile's injection points and receivers.
-  for (int i = tid; i < pl.n; i += NT) {
-    const int cell = pl.terms[i].cell, ix = cell / nz, iz = cell - ix * nz;
-    if (in_tile(ix, iz) && (i == 0 || pl.terms[i - 1].cell != cell)) {
+  // The tile's injection points and receivers. (kExact: the receivers' terms are
+  // the series themselves, and a source's derivative by b drops b.)
+  auto point = [&](const InjPlan &p, int i, int q) {
+    const int cell = p.terms[i].cell, ix = cell / nz, iz = cell - ix * nz;
+    int n = 1;
+    while (i + n < p.n && p.terms[i + n].cell == cell) ++n;
+    const int first = atomicAdd(&s_count[3], n);
+    inj_terms[q] = (uint32_t)first | (uint32_t)n << 16;
+    INJ[q] = make_float2(0.f, 0.f);
+    for (int k = 0; k < n; ++k) {
+      const InjTerm t = p.terms[i + k];
+      const double b = EX ? 1.0 : (double)d.b[(size_t)ix * ps + iz];
+      const double *src = (t.kind == 0 ? d.stf : t.field == 0 ? d.a_ux : d.a_uz) +
+                          (size_t)t.index * d.nt;
+      term_w[first + k] =
+          EX && t.kind != 0 ? 1.0 : (t.kind == 0 ? t.coef : 1.0) * d.dt_d * b / t.div;
+      term_src[first + k] = src;
+      term_next[first + k] = src[it0];
+      term_field[first + k] = t.field;
+    }
+  };
+  auto first_in_tile = [&](const InjPlan &p, int i, int &at) {
+    const int cell = p.terms[i].cell, ix = cell / nz, iz = cell - ix * nz;
+    at = (ix - x0) * (S - 4) + iz - z0;
+    return in_tile(ix, iz) && (i == 0 || p.terms[i - 1].cell != cell);
+  };
+  for (int i = tid, at; i < pl.n; i += NT)
+    if (first_in_tile(pl, i, at)) {
       const int q = atomicAdd(&s_count[0], 1);
-      inj_first[q] = i;
-      INJ[q] = make_float2(0.f, 0.f);
-      const int at = (ix - x0) * (S - 4) + iz - z0;
+      point(pl, i, q);
       if (EX)
         slots_of[2 * at] = (unsigned char)q;
       else
         slot_of[at] = (unsigned short)q;
     }
-  }
   if (EX)
-    for (int i = tid; i < io.src.n; i += NT) {
-      const int cell = io.src.terms[i].cell, ix = cell / nz, iz = cell - ix * nz;
-      if (in_tile(ix, iz) && (i == 0 || io.src.terms[i - 1].cell != cell)) {
+    for (int i = tid, at; i < io.src.n; i += NT)
+      if (first_in_tile(io.src, i, at)) {
         const int q = atomicAdd(&s_count[2], 1);
-        inj_first[tm.n_inj + q] = i;
-        INJ[tm.n_inj + q] = make_float2(0.f, 0.f);
-        slots_of[2 * ((ix - x0) * (S - 4) + iz - z0) + 1] = (unsigned char)q;
+        point(io.src, i, tm.n_inj + q);
+        slots_of[2 * at + 1] = (unsigned char)q;
       }
-    }
   if (!BACK)
     for (int r = tid; r < d.nr; r += NT) {
       const int cell = d.rec_cell[r], ix = cell / ps, iz = cell - ix * ps;
@@ -550,59 +574,24 @@ __device__ __forceinline__ void member_steps(const tma::SimDesc &d, const Team &
         }
       }
     };
-    // Item 2 q + f is field f of injection point q; helper thread i
-    // evaluates item i (and i + CT, ...) in the stress half-step. An item's term adds
-    // weight * (sample of its source or adjoint source); the first item's first
-    // term is kept in registers with its sample loaded one step ahead.
-    const double *inj_src = nullptr;
-    double inj_w = 0.0, inj_next = 0.0;
-    bool inj_more = false;
-    // Injection points come first, then (kExact) source points, in their own
-    // part of the list.
-    auto is_src = [&](int i) { return EX && (i >> 1) >= n_inj; };
-    auto point = [&](int i) { return is_src(i) ? tm.n_inj + (i >> 1) - n_inj : i >> 1; };
-    auto plan_of = [&](int i) -> const InjPlan & { return is_src(i) ? io.src : pl; };
-    auto term_series = [&](const InjTerm &t) {
-      const double *src = t.kind == 0 ? d.stf : (t.field == 0 ? d.a_ux : d.a_uz);
-      return src + (size_t)t.index * d.nt;
-    };
-    // (kExact: the receivers' terms are the series themselves, and a source's
-    // derivative by b drops b.)
-    auto term_weight = [&](const InjTerm &t) {
-      if (EX) return t.kind == 0 ? t.coef * d.dt_d / t.div : 1.0;
-      const int ix = t.cell / nz, iz = t.cell - ix * nz;
-      const double b = (double)d.b[(size_t)ix * ps + iz];
-      return (t.kind == 0 ? t.coef : 1.0) * d.dt_d * b / t.div;
-    };
-    // Sum of an item's terms at step `it`, from its skip-th on.
-    auto item_value = [&](int i, int it, int skip) {
-      const InjPlan &p = plan_of(i);
-      const int q0 = inj_first[point(i)], cell = p.terms[q0].cell;
-      float v = 0.f;
-      for (int q = q0; q < p.n && p.terms[q].cell == cell; ++q) {
-        const InjTerm t = p.terms[q];
-        if (t.field != (i & 1) || skip-- > 0) continue;
-        v += (float)(term_weight(t) * term_series(t)[it]);
+    // What the injection points add in this step: item 2 q + f is field f of point
+    // q (injection points first, then source points, in their own part of the
+    // list). The next step's samples are fetched in the velocity half-step.
+    const int n_terms = s_count[3];
+    auto add_terms = [&] {
+      for (int i = ct; i < n_items; i += CT) {
+        const int q = EX && (i >> 1) >= n_inj ? tm.n_inj + (i >> 1) - n_inj : i >> 1;
+        const uint32_t t = inj_terms[q];
+        float v = 0.f;
+        for (uint32_t k = t & 0xFFFFu; k < (t & 0xFFFFu) + (t >> 16); ++k)
+          if (term_field[k] == (i & 1)) v += (float)(term_w[k] * term_next[k]);
+        reinterpret_cast<float *>(INJ)[2 * q + (i & 1)] = v;
       }
-      return v;
     };
-    float *const values = reinterpret_cast<float *>(INJ);
-    auto place = [&](int i) { return 2 * point(i) + (i & 1); };
-    if (ct < n_items) {
-      const InjPlan &p = plan_of(ct);
-      const int q0 = inj_first[point(ct)], cell = p.terms[q0].cell;
-      for (int q = q0; q < p.n && p.terms[q].cell == cell; ++q) {
-        const InjTerm t = p.terms[q];
-        if (t.field != (ct & 1)) continue;
-        if (!inj_src) {
-          inj_src = term_series(t);
-          inj_w = term_weight(t);
-          inj_next = inj_src[it0];
-        } else {
-          inj_more = true;
-        }
-      }
-    }
+    auto fetch_terms = [&](int it) {
+#pragma unroll 4
+      for (int k = ct; k < n_terms; k += CT) term_next[k] = term_src[k][it];
+    };
     // kExact: the CTA's rates of a step, three per row for the stress half-step
     // and two for the velocity one, each fetched as its buffer becomes free.
     const uint32_t rate_bytes = 8u * K * CW;
@@ -638,19 +627,13 @@ __device__ __forceinline__ void member_steps(const tma::SimDesc &d, const Team &
           d.rec_vx[o] = F[oVX + rec_off[i]];
           d.rec_vz[o] = F[oVZ + rec_off[i]];
         }
-      // What the tile's injection points add this step.
-      if (inj_src) {
-        float v = (float)(inj_w * inj_next);
-        if (inj_more) v += item_value(ct, it, 1);
-        values[place(ct)] = v;
-        if (more) inj_next = inj_src[BACK ? it - 1 : it + 1];
-      }
-      for (int i = ct + CT; i < n_items; i += CT) values[place(i)] = item_value(i, it, 0);
+      add_terms();
       receive(0, tag);
       put_done();
       meet(0, true);
       fetch(j + 1, 0);
       put(j, 0);
+      if (more) fetch_terms(BACK ? it - 1 : it + 1);
       if (more) receive(1, tag);
       put_done();
       meet(1, more);

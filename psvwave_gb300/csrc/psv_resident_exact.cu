@@ -46,7 +46,7 @@ cudaError_t run(T, const tma::SimDesc &d, const ExactPlan &q, int it0, int n_ste
     if (e != cudaSuccess) return e;
   }
   const Team team{0, p.tiles_x, p.tiles_z, p.groups, p.n_rec, p.n_inj, q.n_src,
-                  static_cast<Word *>(mail)};
+                  MODE == kExact ? q.n_term : p.n_term, static_cast<Word *>(mail)};
   cudaLaunchAttribute attr;
   cudaLaunchConfig_t lc = config(&attr, T::CL, p.ctas(), p.ctas(), p.threads,
                                  MODE == kExact ? q.smem : q.rate_smem, s);

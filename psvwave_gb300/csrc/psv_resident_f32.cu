@@ -9,9 +9,9 @@ namespace {
 template <int MODE, int K, int S, bool CLUSTER>
 __global__ void __launch_bounds__(kMaxThreads, 1)
     resident_steps(const __grid_constant__ tma::SimDesc d, int tiles_x, int tiles_z, int groups,
-                   int n_rec, int n_inj, int it0, int n_steps, int parity, int zero, int store,
+                   int n_rec, int n_inj, int n_term, int it0, int n_steps, int parity, int zero, int store,
                    const Dump dump, Word *mail, int *err) {
-  const Team t{(int)blockIdx.x, tiles_x, tiles_z, groups, n_rec, n_inj, 0, mail};
+  const Team t{(int)blockIdx.x, tiles_x, tiles_z, groups, n_rec, n_inj, 0, n_term, mail};
   member_steps<MODE, K, S, CLUSTER>(d, t, it0, n_steps, parity, zero != 0, store, dump, RateIo(),
                                     err);
 }
@@ -25,13 +25,14 @@ __global__ void __launch_bounds__(kMaxThreads, 1)
                          int *err) {
   const Member m = members[cta_member[blockIdx.x]];
   const Team t{(int)blockIdx.x - m.first, m.tiles_x, m.tiles_z, m.groups, m.n_rec, m.n_inj,
-               0, mail + (size_t)m.first * kBox};
+               0, m.n_term, mail + (size_t)m.first * kBox};
   member_steps<kForward, K, S, CLUSTER>(sims[m.sim], t, 0, n_steps, 0, true, store, Dump(),
                                         RateIo(), err);
 }
 
-size_t smem_bytes(int Rm, int S, int nr, int n_terms) {
-  return (size_t)5 * (Rm + 4) * S * sizeof(float) + (size_t)n_terms * 12 + (size_t)nr * 8 +
+size_t smem_bytes(int Rm, int S, int nr, int n_points, int n_terms) {
+  return (size_t)5 * (Rm + 4) * S * sizeof(float) + (size_t)n_points * 12 +
+         (size_t)n_terms * 28 + (size_t)nr * 8 +
          (size_t)Rm * (S - 4) * sizeof(unsigned short) + 16;
 }
 
@@ -44,7 +45,7 @@ cudaError_t run(T, const tma::SimDesc &d, const Plan &p, int it0, int n_steps, i
   if (e != cudaSuccess) return e;
   cudaLaunchAttribute attr;
   cudaLaunchConfig_t lc = config(&attr, T::CL, p.ctas(), p.ctas(), p.threads, p.smem, s);
-  return cudaLaunchKernelEx(&lc, kern, d, p.tiles_x, p.tiles_z, p.groups, p.n_rec, p.n_inj, it0,
+  return cudaLaunchKernelEx(&lc, kern, d, p.tiles_x, p.tiles_z, p.groups, p.n_rec, p.n_inj, p.n_term, it0,
                             n_steps, parity, zero, store, dump, static_cast<Word *>(mail), err);
 }
 
@@ -124,7 +125,9 @@ bool fit(Plan &p, const Device &q, const Grid &g, int per_sm) {
   p.n_rec = most_per_tile(p, g.nx, g.nz, g.receivers);
   p.n_inj = most_per_tile(p, g.nx, g.nz, g.receivers);  // the adjoint injects at receivers
   for (const auto &cells : g.sources) p.n_inj = std::max(p.n_inj, most_per_tile(p, g.nx, g.nz, cells));
-  p.smem = smem_bytes(r_max, p.stride, p.n_rec, p.n_inj);
+  p.n_term = 2 * p.n_rec;  // of the adjoint
+  for (const auto &cells : g.terms) p.n_term = std::max(p.n_term, most_per_tile(p, g.nx, g.nz, cells));
+  p.smem = smem_bytes(r_max, p.stride, p.n_rec, p.n_inj, p.n_term);
   // (1 KB of every resident CTA's share is the system's.)
   return (p.smem + 1024 + 64) * per_sm <= (size_t)q.optin + 1024;
 }
@@ -180,9 +183,15 @@ ExactPlan plan_exact(const Grid &g, int lanes) {
     e.n_src = 0;
     for (const auto &cells : g.sources)
       e.n_src = std::max(e.n_src, most_per_tile(p, g.nx, g.nz, cells));
+    // Both the receivers' and the shot's terms.
+    e.n_term = 0;
+    for (const auto &cells : g.terms) e.n_term = std::max(e.n_term, most_per_tile(p, g.nx, g.nz, cells));
+    e.n_term += 2 * p.n_rec;
+    if (e.n_term > 0xFFFF) return false;
     e.rate_stride = p.ctas() * rates / sizeof(float2);
     e.rate_smem = p.smem + rates;
-    e.smem = e.rate_smem + (size_t)4 * R * (p.stride - 4) * sizeof(float) + (size_t)e.n_src * 12;
+    e.smem = e.rate_smem + (size_t)4 * R * (p.stride - 4) * sizeof(float) + (size_t)e.n_src * 12 +
+             (size_t)(e.n_term - p.n_term) * 28;
     if (p.n_inj > 256 || e.n_src > 256) return false;  // byte tables
     return e.smem + 64 <= (size_t)q.optin;
   };

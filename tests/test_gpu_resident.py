@@ -19,7 +19,8 @@ def rel(a, b):
     return np.linalg.norm(a - b) / np.linalg.norm(b)
 
 
-def model(nx, nz, nt=120, npb=6, seed=0, shots=1, precision="fp32", near=False):
+def model(nx, nz, nt=120, npb=6, seed=0, shots=1, precision="fp32", near=False,
+          column=False):
     nxi, nzi = nx - 2 * npb, nz - 2 * npb
     rng = np.random.default_rng(seed + 1000 * nx + nz)
     # Two sources of a shot at the same point: several terms per cell. Two
@@ -31,13 +32,16 @@ def model(nx, nz, nt=120, npb=6, seed=0, shots=1, precision="fp32", near=False):
     if near:  # where the wave of 120 steps arrives
         rx = [min(max(xs[0] + int(v), 0), nxi - 1) for v in rng.integers(-8, 9, 9)]
         rz = [min(max(zs[0] + int(v), 0), nzi - 1) for v in rng.integers(-8, 9, 9)]
+    if column:
+        rx, rz = [xs[0]] * 99, [int(v) for v in rng.permutation(nzi)[:99]]
     p = dict(nt=nt, nx_inner=nxi, nz_inner=nzi, nx_inner_boundary=1, nz_inner_boundary=1,
              dx=1.249, dz=1.3, dt=2.5e-4, np_boundary=npb, np_factor=0.05, scalar_rho=1500.0,
              scalar_vp=2000.0, scalar_vs=800.0, npx=1, npz=1, peak_frequency=90.0,
              source_timeshift=0.0, delay_cycles_per_shot=0, n_sources=2 * shots,
              ix_sources=[x for x in xs for _ in range(2)],
              iz_sources=[z for z in zs for _ in range(2)], moment_angles=[30.0, 75.0] * shots,
-             which_source_to_fire_in_which_shot=[[2 * s, 2 * s + 1] for s in range(shots)], nr=10,
+             which_source_to_fire_in_which_shot=[[2 * s, 2 * s + 1] for s in range(shots)],
+             nr=len(rx) + 1,
              ix_receivers=rx + rx[:1], iz_receivers=rz + rz[:1], snapshot_interval=10)
     m = psv.fdModel.from_parameters(p, precision=precision)
     v = 1.0 + 0.1 * rng.random((3, nx, nz))
@@ -174,3 +178,19 @@ def test_resident_exact_gradient_is_as_accurate_as_per_step_launches(nx, nz, sho
     for exact, per_step, resident, whole, sevenths in zip(*out):
         assert rel(resident, exact) <= max(2 * rel(per_step, exact), 1e-6)
         assert np.array_equal(resident, whole) and np.array_equal(resident, sevenths)
+
+
+def test_resident_many_terms_in_one_tile():
+    # A column of receivers, more than a helper warp has threads, whose adjoint
+    # sources and their points fall into one tile.
+    out = []
+    for variant in ("fp64", "fused_tma", None):
+        m = model(250, 151, precision="fp64" if variant == "fp64" else "fp32", column=True)
+        if variant == "fused_tma":
+            m.kernel_variant = variant
+        m.set_observed_data(*[np.zeros_like(a) for a in m.get_observed_data()])
+        m.run_model(False, True)
+        out.append([m.get_gradient_vector()] + list(m.exact_gradient(50)[1]) +
+                   list(m.get_lame_kernels()))
+    for exact, per_step, resident in zip(*out):
+        assert rel(resident, exact) <= max(2 * rel(per_step, exact), 1e-6)
