@@ -48,7 +48,7 @@ def parse():
                    help="run one NT-step forward of the c1 workload and exit (for ncu captures)")
     p.add_argument("--ncu-case-small", type=int, default=0, metavar="NT",
                    help="run one NT-step forward of the c0 workload (the default scheme there: "
-                        "cluster-resident), launch by launch, and exit (for ncu captures)")
+                        "resident on chip), launch by launch, and exit (for ncu captures)")
     p.add_argument("--ncu-case-exact", type=int, default=0, metavar="NT",
                    help="run one exact gradient of one NT-step shot of the c3 workload, launch by "
                         "launch, and exit (for ncu captures)")

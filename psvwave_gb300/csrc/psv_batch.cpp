@@ -529,7 +529,7 @@ int Batch::autotune(int n_steps) {
   if (members_.empty()) return tile_cfg_;
   // Every (launch scheme, tile shape) pair on n_steps steps of the members
   // currently active, each timed on its third run (after the build and the
-  // graph capture), and the cluster-resident scheme when the members fit;
+  // graph capture), and the resident scheme when the members fit;
   // the fastest is kept.
   float best = 0;
   int best_cfg = tile_cfg_;

@@ -102,8 +102,8 @@ bool fit(Plan &p, const Device &q, const Grid &g, int per_sm) {
     return false;
   // Helper warps: one for a cluster; enough for the tile's words otherwise,
   // one per SM partition on full blocks (their polls then cost each
-  // partition's compute warps alike: 12 + 4 warps took 5.7 us a step at
-  // 1103 x 497 points, 13 + 3 warps 5.9).
+  // partition's compute warps alike: at 1103 x 497 points 12 + 4 warps take
+  // 4.7 us a step, 12 + 2 warps 5.0).
   int help = 1;
   if (!p.cluster) {
     if (words(r_max, C) > kBoxWords) return false;
