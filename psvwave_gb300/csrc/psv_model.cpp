@@ -609,8 +609,10 @@ resident::ExactPlan Model::exact_plan(int lanes) const {
 }
 
 // Lanes of an exact gradient resident on chip, and their plan (none: it does not
-// fit): as many as shots, up to kMaxExactLanes, that have room on the device and
-// in 60 % of its free memory.
+// fit): the fewest that take the shots in as few turns as fit on the device and
+// in 60 % of its free memory, up to kMaxResidentLanes (a step at 250 x 150, eight
+// shots: four 16-CTA clusters 1.9 us per shot, eight lanes for the seven that
+// run at once 1.2).
 int Model::exact_resident_lanes(int C, int n_list, resident::ExactPlan *plan) const {
   *plan = resident::ExactPlan();
   if (!use_resident()) return 0;
@@ -618,7 +620,10 @@ int Model::exact_resident_lanes(int C, int n_list, resident::ExactPlan *plan) co
   size_t free_b = 0, total_b = 0;
   if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) free_b = 0;
   for (const auto &l : lanes_) free_b += l->bytes();
-  for (int lanes = std::max(1, std::min(n_list, kMaxExactLanes)); lanes >= 1; --lanes) {
+  n_list = std::max(n_list, 1);
+  for (int turns = 1; turns <= n_list; ++turns) {
+    const int lanes = (n_list + turns - 1) / turns;
+    if (lanes > kMaxResidentLanes) continue;
     const resident::ExactPlan p = exact_plan(lanes);
     if (p.p.ctas() <= 0) continue;
     if (lanes > 1 && static_cast<double>(lanes) * exact_resident_bytes(C, p) > 0.6 * free_b) continue;
