@@ -281,8 +281,9 @@ def fwi_gradients_c3(steps, with_cpu=False):
     out["roofline"] = {"bound": "hbm", "bytes_per_gradient": per_grad,
                        "achieved": per_grad / t / 1e9, "peak": peak, "unit": "GB/s",
                        "frac": per_grad / t / 1e9 / peak, "peak_source": kind,
-                       "note": "whole checkpointed gradient, all kernels, 8 shots in "
-                               "concurrent lanes"}
+                       "note": "whole checkpointed gradient, all kernels; bytes of steps that "
+                               "stream every field (a gradient resident on chip moves "
+                               "40 bytes per cell and step instead of 202)"}
     if with_cpu:
         out["cpu_baseline"] = cpu_baseline_c3()
     return out

@@ -19,7 +19,7 @@
 // per step and shot through L2 and DRAM (13 a forward step, 25 an adjoint
 // step) in three launches; this moves 10, in two launches per segment. Then, as
 // for all resident steps, computation and the exchange of edges. us per step
-// and shot, those kernels -> these: 250 x 150 25.0 -> 7.4 (one shot), 8.6 -> 1.9
+// and shot, those kernels -> these: 250 x 150 25.0 -> 7.4 (one shot), 8.6 -> 1.2
 // (eight at a time); 500 x 300 29.6 -> 8.3, 10.2 -> 5.6; 900 x 450 36.6 -> 11.8,
 // 15.5 -> 11.0; 1100 x 500 35.9 -> 16.6, 19.0 -> 15.7. Grids that do not fit with
 // the adjoint's shared memory keep them.
