@@ -895,10 +895,10 @@ __device__ __forceinline__ void member_steps(const tma::SimDesc &d, const Team &
           } else {
             const float la0 = __fmaf_rn(-2.f, mu[k].x, lm[k].x);
             const float la1 = __fmaf_rn(-2.f, mu[k].y, lm[k].y);
-            xx[k].x = __fmul_rn(tp[k].x, __fmaf_rn(lm[k].x, ex0, __fmaf_rn(la0, ez0, xx[k].x)));
-            xx[k].y = __fmul_rn(tp[k].y, __fmaf_rn(lm[k].y, ex1, __fmaf_rn(la1, ez1, xx[k].y)));
-            zz[k].x = __fmul_rn(tp[k].x, __fmaf_rn(la0, ex0, __fmaf_rn(lm[k].x, ez0, zz[k].x)));
-            zz[k].y = __fmul_rn(tp[k].y, __fmaf_rn(la1, ex1, __fmaf_rn(lm[k].y, ez1, zz[k].y)));
+            xx[k].x = __fmul_rn(tp[k].x, __fadd_rn(xx[k].x, __fmaf_rn(lm[k].x, ex0, __fmul_rn(la0, ez0))));
+            xx[k].y = __fmul_rn(tp[k].y, __fadd_rn(xx[k].y, __fmaf_rn(lm[k].y, ex1, __fmul_rn(la1, ez1))));
+            zz[k].x = __fmul_rn(tp[k].x, __fadd_rn(zz[k].x, __fmaf_rn(la0, ex0, __fmul_rn(lm[k].x, ez0))));
+            zz[k].y = __fmul_rn(tp[k].y, __fadd_rn(zz[k].y, __fmaf_rn(la1, ex1, __fmul_rn(lm[k].y, ez1))));
             xz[k].x = __fmul_rn(tp[k].x, __fmaf_rn(mu[k].x, g0, xz[k].x));
             xz[k].y = __fmul_rn(tp[k].y, __fmaf_rn(mu[k].y, g1, xz[k].y));
           }
