@@ -35,18 +35,25 @@ struct alignas(128) SimDesc {
   int nx = 0, nz = 0, pitch = 0, np = 0, nt = 0, nr = 0, si = 1;
   float dt = 0, idx = 0, idz = 0;
   double dt_d = 0;
-  // The resident step's stencil coefficients times dt / dx and dt / dz (9/8 and
-  // 1/24 along x, then z), each rounded once.
+  // The resident step's stencil coefficients times dt / dx and dt / dz: a1 and
+  // a2 along x, then z. a1 is 9/8 h (h = dt / dx) rounded; a2, 1/24 h, is
+  // rounded from (a1 - h) / 3, so that the difference of a linear field,
+  // a1 - 3 a2, is h to 2^-27. (Each rounded by itself, the scheme's step was
+  // up to 2^-25 off, a phase error that grows with time: misfits of 250 x 150
+  // points and 2000 steps were 1.4e-7 off 64-bit ones.) The cubic term that
+  // this leaves, a1 - 27 a2, is below 2^-20 h.
   float coef[4] = {0, 0, 0, 0};
+  static void step_coefficients(double h, float *a) {
+    a[0] = static_cast<float>(9.0 / 8.0 * h);
+    a[1] = static_cast<float>((static_cast<double>(a[0]) - h) / 3.0);
+  }
   void set_steps(double dt, double dx, double dz) {
     this->dt = static_cast<float>(dt);
     idx = static_cast<float>(1.0 / dx);
     idz = static_cast<float>(1.0 / dz);
     dt_d = dt;
-    coef[0] = static_cast<float>(9.0 / 8.0 * dt / dx);
-    coef[1] = static_cast<float>(1.0 / 24.0 * dt / dx);
-    coef[2] = static_cast<float>(9.0 / 8.0 * dt / dz);
-    coef[3] = static_cast<float>(1.0 / 24.0 * dt / dz);
+    step_coefficients(dt / dx, coef);
+    step_coefficients(dt / dz, coef + 2);
   }
   const float *lm = nullptr, *b = nullptr, *taper_tab = nullptr;
   const float *mu = nullptr;  // (the TMA steps read mu through the maps)
