@@ -589,9 +589,11 @@ __device__ __forceinline__ void member_steps(const tma::SimDesc &d, const Team &
     auto place = [&](int i) {
       return EX && (i >> 1) >= n_inj ? tm.n_inj + (i >> 1) - n_inj : i >> 1;
     };
-    auto item_value = [&](int i, int skip) {
+    // v and the terms of item i after the first `skip`, added one by one in the
+    // plan's order, so that an item's sum does not depend on the thread it falls
+    // to. (-0 adds to a first term without a trace.)
+    auto item_value = [&](int i, float v, int skip) {
       const uint32_t t = inj_terms[place(i)];
-      float v = 0.f;
       for (uint32_t k = t & 0xFFFFu; k < (t & 0xFFFFu) + (t >> 16); ++k)
         if (term_field[k] == (i & 1) && skip-- <= 0) v += (float)(term_w[k] * term_next[k]);
       return v;
@@ -612,11 +614,11 @@ __device__ __forceinline__ void member_steps(const tma::SimDesc &d, const Team &
     auto add_terms = [&] {
       if (own_src) {
         float v = (float)(own_w * own_next);
-        if (table) v += item_value(ct, 1);
+        if (table) v = item_value(ct, v, 1);
         *own_value = v;
       }
       for (int i = ct + CT; i < n_items; i += CT)
-        values[2 * place(i) + (i & 1)] = item_value(i, 0);
+        values[2 * place(i) + (i & 1)] = item_value(i, -0.f, 0);
     };
     auto fetch_terms = [&](int it) {
       if (!table) return;
@@ -963,9 +965,9 @@ __device__ __forceinline__ void member_steps(const tma::SimDesc &d, const Team &
                 if (!(src_mask >> (2 * k + e) & 1u)) continue;
                 const float2 add = INJ[tm.n_inj + slots_of[2 * ((r0 + k) * (S - 4) + 2 * c + e) + 1]];
                 if (e)
-                  sb.y += add.x * vx[k].y + add.y * vz[k].y;
+                  sb.y = __fadd_rn(sb.y, __fmaf_rn(add.x, vx[k].y, __fmul_rn(add.y, vz[k].y)));
                 else
-                  sb.x += add.x * vx[k].x + add.y * vz[k].x;
+                  sb.x = __fadd_rn(sb.x, __fmaf_rn(add.x, vx[k].x, __fmul_rn(add.y, vz[k].x)));
               }
             }
             sts2(sum, sb);

@@ -1,0 +1,66 @@
+"""What the resident scheme keeps whatever its split, its launch and the
+other work on the device."""
+import numpy as np
+import pytest
+
+import psvwave_gb300 as psv
+
+pytestmark = pytest.mark.gpu
+
+
+def model(nx, nz, sources, receivers, nt=120, npb=6, shots=None, precision="fp32", **kw):
+    """Sources and receivers are (ix, iz) of the inner grid."""
+    shots = shots or [list(range(len(sources)))]
+    p = dict(nt=nt, nx_inner=nx - 2 * npb, nz_inner=nz - 2 * npb, nx_inner_boundary=1,
+             nz_inner_boundary=1, dx=1.249, dz=1.3, dt=2.5e-4, np_boundary=npb, np_factor=0.05,
+             scalar_rho=1500.0, scalar_vp=2000.0, scalar_vs=800.0, npx=1, npz=1,
+             peak_frequency=90.0, source_timeshift=0.0, delay_cycles_per_shot=0,
+             n_sources=len(sources), ix_sources=[s[0] for s in sources],
+             iz_sources=[s[1] for s in sources],
+             moment_angles=[17.0 + 31.0 * k for k in range(len(sources))],
+             which_source_to_fire_in_which_shot=shots, nr=len(receivers),
+             ix_receivers=[r[0] for r in receivers], iz_receivers=[r[1] for r in receivers],
+             snapshot_interval=10)
+    p.update(kw)
+    m = psv.fdModel.from_parameters(p, precision=precision)
+    v = 1.0 + 0.1 * np.random.default_rng(nx + nz).random((3, m.nx, m.nz))
+    m.set_parameter_fields(2000.0 * v[0], 800.0 * v[1], 1500.0 * v[2])
+    return m
+
+
+@pytest.mark.parametrize("nx,nz", [(68, 57), (250, 151), (400, 300)])
+def test_coincident_sources_and_receivers_sum_in_one_order(nx, nz):
+    # Six sources at each of four neighbouring points, four receivers at each
+    # of 24: several terms of a field at a point, more points than a team's
+    # smallest number of helper threads serves one each. Every run gives the
+    # same bits, alone and in a batch whose larger member brings more helpers.
+    def make():
+        x = nx // 3
+        return model(nx, nz, [(x, 12 + k % 4) for k in range(24)],
+                     [(x + 3, 4 + k % 24) for k in range(96)])
+
+    ref = None
+    for _ in range(3):
+        m = make()
+        for _ in range(4):  # eager, graph capture, graph replays
+            m.forward_simulate(0, True)
+            out = list(m.get_synthetic_data())
+            m.set_observed_data(*[0.0 * a for a in out])
+            m.calculate_l2_misfit()
+            m.calculate_l2_adjoint_sources()
+            m.reset_kernels()
+            m.adjoint_simulate(0)
+            out += list(m.get_lame_kernels()) + list(m.get_wavefields())
+            out += list(m.exact_gradient(50)[1])
+            ref = ref or out
+            for a, b in zip(out, ref):
+                assert np.array_equal(a, b)
+    ms = [make(), model(nx + 90, nz + 40, [(20, 20)], [(30, 30)])]
+    b = psv.Batch()
+    for m in ms:
+        b.add(m, 0)
+    b.cluster = True
+    for _ in range(4):
+        b.forward()
+        for a, c in zip(ms[0].get_synthetic_data(), ref):
+            assert np.array_equal(a, c)
