@@ -231,6 +231,8 @@ int psv_set_async(psv_model *m, int async_calls);
  * default: a loop is captured on its second identical call) or always launch
  * kernel by kernel (0). No counterpart in the reference. */
 int psv_set_graph_capture(psv_model *m, int enable);
+/* Waits for the model's work; PSV_ERR_CUDA when a bounded wait inside the
+ * kernels of an asynchronous call has run out. */
 int psv_synchronize(psv_model *m);
 /* Parameter fields from device FP64 buffers [nx][nz]. */
 int psv_set_parameter_fields_device(psv_model *m, const double *vp, const double *vs,

@@ -512,7 +512,7 @@ int psv_set_graph_capture(psv_model *m, int enable) {
 }
 
 int psv_synchronize(psv_model *m) {
-  return guarded([&] { M(m).synchronize(); });
+  return guarded([&] { M(m).wait(); });
 }
 
 int psv_set_parameter_fields_device(psv_model *m, const double *vp, const double *vs,

@@ -1644,7 +1644,10 @@ int Model::autotune(int n_steps) {
   return best_cfg;
 }
 
+// Raises when a bounded wait of one of the model's kernels ran out since the
+// last look (and clears the flag).
 void Model::check_device_error() {
+  DeviceGuard guard(device_);
   int flag = 0;
   cuda_check(cudaMemcpyAsync(&flag, err_flag_.get(), sizeof(int), cudaMemcpyDeviceToHost, stream()),
              "error flag");
@@ -1654,6 +1657,11 @@ void Model::check_device_error() {
     cudaStreamSynchronize(stream());
     throw Error(PSV_ERR_CUDA, "a CTA timed out waiting for its TMA tile copies");
   }
+}
+
+void Model::wait() {
+  synchronize();
+  if (steps_wait()) check_device_error();
 }
 
 void Model::clear_graphs() {
@@ -1834,7 +1842,7 @@ void Model::forward_simulate(int shot, bool store, bool verbose, bool output_wav
     run(n_steps, n_steps, false, true);
   }
   finish("forward_simulate");
-  if (!async_ && (is_tma() || use_resident64())) check_device_error();
+  if (!async_ && steps_wait()) check_device_error();
   if (verbose) {
     synchronize();
     double s = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
@@ -1965,7 +1973,7 @@ void Model::adjoint_simulate(int shot, bool verbose) {
     cuda_check(e, "adjoint_simulate");
   });
   finish("adjoint_simulate");
-  if (!async_ && (is_tma() || use_resident64())) check_device_error();
+  if (!async_ && steps_wait()) check_device_error();
   if (verbose) {
     synchronize();
     double s = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
@@ -2038,6 +2046,7 @@ void Model::run_model(bool verbose, bool simulate_adjoint) {
   }
   async_ = was_async;
   finish("run_model");
+  if (!async_ && steps_wait()) check_device_error();
 }
 
 void Model::update_from_velocity() {

@@ -184,6 +184,7 @@ class Model {
     if (!on) clear_graphs();
   }
   void synchronize();
+  void wait();  // and raises what the steps' bounded waits reported
 
   enum DataKind { kSynthetic = 0, kObserved = 1, kAdjoint = 2 };
 
@@ -245,6 +246,8 @@ class Model {
                           cudaEvent_t *events,
                           bool allow_resident = true);
   cudaError_t tma_adjoint(int shot);
+  // Whether the time steps' kernels wait for copies or for one another.
+  bool steps_wait() const { return is_tma() || use_resident64(); }
   void check_device_error();
 
   // Whole time loops captured as CUDA graphs, keyed by (direction, shot,
