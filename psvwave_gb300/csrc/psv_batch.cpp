@@ -461,7 +461,7 @@ void Batch::forward(bool store, int n_steps) {
   int flag = 0;
   cuda_check(cudaMemcpy(&flag, err_flag_.get(), sizeof(int), cudaMemcpyDeviceToHost), "error flag");
   if (flag) {
-    cudaMemset(err_flag_.get(), 0, sizeof(int));
+    cudaMemsetAsync(err_flag_.get(), 0, sizeof(int), stream_);
     throw Error(PSV_ERR_CUDA, "a CTA timed out waiting for its TMA tile copies");
   }
 }

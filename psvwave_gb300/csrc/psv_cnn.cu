@@ -1230,6 +1230,8 @@ CoarseMap::CoarseMap(int device, int nx_, int nz_, int np_, int ncx_, int ncz_, 
   const size_t n = (size_t)3 * ncx * ncz;
   upload(mean_, std::vector<double>(mean, mean + n));
   upload(sigma_, std::vector<double>(sigma, sigma + n));
+  // (On the legacy stream, for which stream_ does not wait.)
+  cuda_check(cudaStreamSynchronize(cudaStreamLegacy), "upload coarse map");
   cuda_check(cudaStreamCreateWithFlags(&stream_, cudaStreamNonBlocking), "cudaStreamCreate");
 }
 

@@ -403,6 +403,9 @@ void Model::build_plans() {
     const size_t mail = resident64::mailbox_bytes(resident64_);
     if (mail_.bytes() < mail) mail_.allocate(mail, false);
   }
+  // (Cleared and uploaded on the legacy stream, for which the model's stream
+  // does not wait.)
+  cuda_check(cudaStreamSynchronize(cudaStreamLegacy), "upload injection terms");
 }
 
 resident::Grid Model::resident_grid() const {
@@ -2241,6 +2244,7 @@ void Model::set_stf(const double *stf) {
     cuda_check(cudaMemcpy(stf_d_.get(), stf_.data(), stf_.size() * sizeof(double),
                           cudaMemcpyHostToDevice),
                "upload stf");
+  cuda_check(cudaStreamSynchronize(cudaStreamLegacy), "upload stf");
 }
 
 void Model::set_moment(const double *moment) {

@@ -64,3 +64,31 @@ def test_coincident_sources_and_receivers_sum_in_one_order(nx, nz):
         b.forward()
         for a, c in zip(ms[0].get_synthetic_data(), ref):
             assert np.array_equal(a, c)
+
+
+@pytest.mark.parametrize("precision", ["fp32", "fp64"])
+def test_set_moment_is_complete_when_it_returns(precision):
+    # The injection terms' buffers are cleared and filled on the legacy stream,
+    # here behind other work; the simulation runs on the model's own.
+    import torch
+
+    def make():
+        return model(68, 57, [(20, 20), (30, 25)], [(24, 24)], precision=precision)
+
+    tensors = [np.array([[[1.0, 0.3 * k], [-0.2, 0.5 + k]]] * 2) for k in range(6)]
+    ref = []
+    for t in tensors:
+        m = make()
+        m.set_moment(t)
+        torch.cuda.synchronize()
+        m.forward_simulate(0, False)
+        ref.append(m.get_synthetic_data())
+    m = make()
+    busy = torch.zeros(1 << 26, device="cuda")
+    for t, r in zip(tensors, ref):
+        for _ in range(20):
+            busy.add_(1.0)
+        m.set_moment(t)
+        m.forward_simulate(0, False)
+        for a, b in zip(m.get_synthetic_data(), r):
+            assert a.any() and np.array_equal(a, b)
