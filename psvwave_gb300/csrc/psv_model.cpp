@@ -1418,8 +1418,22 @@ double Model::exact_gradient_lanes(int C, const std::vector<int> &shot_list) {
 }
 
 bool Model::run_model_lanes_ok() const {
-  return prec_ == PSV_FP32 && tma_ok_ && cfg_.n_shots > 1 && !use_resident() &&
-         (variant_ == kFusedTma || variant_ == kFusedTmaPersistent);
+  const int shots = cfg_.n_shots;
+  if (prec_ != PSV_FP32 || !tma_ok_ || shots < 2 ||
+      (variant_ != kFusedTma && variant_ != kFusedTmaPersistent))
+    return false;
+  if (!use_resident()) return true;
+  // A grid resident on chip takes the whole device for one shot; per-step
+  // launches of up to kMaxLanes shots overlap. us per step and shot, forward and
+  // adjoint, resident | lanes: 400 x 260, 3 shots 5.5 | 5.4, 4 shots 5.5 | 4.3,
+  // 8 shots 5.4 | 2.6; 700 x 400, 3: 6.8 | 6.8, 4: 6.9 | 5.7, 8: 6.8 | 5.7;
+  // 850 x 420, 4: 7.6 | 6.7, 8: 7.5 | 7.3; 900 x 450, 4: 7.5 | 7.8, 8: 7.6 | 8.6.
+  // A last round of one to three shots costs the lanes most of a full one, at
+  // nine shots: 400 x 260 5.4 | 3.7, 700 x 400 6.8 | 6.9, 850 x 420 7.5 | 8.4.
+  const double cells = static_cast<double>(geo_.nx) * geo_.nz;
+  const int last = shots % kMaxLanes;
+  if (shots < 4 || cells > 3.8e5) return false;
+  return cells <= 2.5e5 || last == 0 || last >= 4;
 }
 
 // run_model with the shots in concurrent lanes (FP32, per-step TMA

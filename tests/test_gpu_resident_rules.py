@@ -92,3 +92,24 @@ def test_set_moment_is_complete_when_it_returns(precision):
         m.forward_simulate(0, False)
         for a, b in zip(m.get_synthetic_data(), r):
             assert a.any() and np.array_equal(a, b)
+
+
+# Where concurrent lanes of per-step launches are quicker than one resident shot
+# after another (four shots or more, up to 380 k points), and where not.
+@pytest.mark.parametrize("nx,nz,shots,lanes", [(400, 300, 4, True), (400, 300, 3, False),
+                                               (400, 300, 9, True), (700, 400, 8, True),
+                                               (700, 400, 9, False), (900, 450, 4, False),
+                                               (250, 151, 4, False)])
+def test_gradients_of_several_shots_run_side_by_side(nx, nz, shots, lanes):
+    def gradient(variant):
+        m = model(nx, nz, [(20 + 9 * k, 20) for k in range(shots)], [(60, 30), (90, 30)],
+                  shots=[[k] for k in range(shots)], nt=60)
+        if variant:
+            m.kernel_variant = variant
+        m.set_observed_data(*[0.0 * a for a in m.get_observed_data()])
+        m.run_model(False, True)
+        return m.get_synthetic_data() + m.get_wavefields() + m.get_lame_kernels()
+
+    out = gradient(None)
+    for scheme, same in (("fused_tma", lanes), ("fused_cluster", not lanes)):
+        assert all(np.array_equal(a, b) for a, b in zip(out, gradient(scheme))) == same
