@@ -636,9 +636,18 @@ int Model::exact_resident_lanes(int C, int n_list, resident::ExactPlan *plan) co
   return 0;
 }
 
+// Steps between the checkpoints of an exact gradient resident on chip: at
+// least eight, because a segment costs two launches and their start (us per
+// shot-step, eight shots of 500 x 300 points: segments of 1 step 19.9, 2 12.9,
+// 4 10.0, 10 7.9; per-step launches 15.6, 11.9, 9.9, 8.6). The results are the
+// same, and a few steps' rates take less memory than the states they replace.
+int Model::resident_segment(int C) const {
+  return C <= 0 || C > cfg_.nt ? cfg_.nt : std::min(cfg_.nt, std::max(C, 8));
+}
+
 size_t Model::exact_resident_bytes(int C, const resident::ExactPlan &p) const {
   const int nt = cfg_.nt;
-  if (C <= 0 || C > nt) C = nt;
+  C = resident_segment(C);
   const size_t state = 5 * padded_size() * sizeof(float);
   const size_t n_ck = (nt + C - 1) / C;
   return n_ck * state + C * p.rate_stride * sizeof(float2) + state +
@@ -1061,13 +1070,14 @@ int Model::ensure_lanes(int K) {
 double Model::exact_gradient_lanes(int C, const std::vector<int> &shot_list) {
   const int nt = cfg_.nt, n_shots = cfg_.n_shots, nr = cfg_.nr;
   if (C <= 0 || C > nt) C = nt;
-  const int n_ck = (nt + C - 1) / C;
   const size_t gp = padded_size(), g = grid_size();
   const size_t field_bytes = gp * sizeof(float), state_bytes = 5 * field_bytes;
   cudaStream_t ms = stream();
   const int n_list = static_cast<int>(shot_list.size());
   resident::ExactPlan on_chip;
   const int on_chip_lanes = exact_resident_lanes(C, n_list, &on_chip);
+  if (on_chip_lanes > 0) C = resident_segment(C);
+  const int n_ck = (nt + C - 1) / C;
   const int K = on_chip_lanes > 0 ? on_chip_lanes
                                   : std::max(1, exact_lane_count(C, std::max(n_list, 1)));
   // Forward steps of the lanes: the 32 x 60 shape (the vectorised tile

@@ -337,6 +337,7 @@ class Model {
   size_t exact_lane_bytes(int C) const;
   resident::ExactPlan exact_plan(int lanes) const;
   int exact_resident_lanes(int C, int n_list, resident::ExactPlan *plan) const;
+  int resident_segment(int C) const;
   size_t exact_resident_bytes(int C, const resident::ExactPlan &p) const;
   mutable std::map<int, resident::ExactPlan> exact_plans_;  // by lanes
   double exact_gradient_lanes(int C, const std::vector<int> &shot_list);

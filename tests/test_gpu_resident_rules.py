@@ -113,3 +113,18 @@ def test_gradients_of_several_shots_run_side_by_side(nx, nz, shots, lanes):
     out = gradient(None)
     for scheme, same in (("fused_tma", lanes), ("fused_cluster", not lanes)):
         assert all(np.array_equal(a, b) for a, b in zip(out, gradient(scheme))) == same
+
+
+@pytest.mark.parametrize("nx,nz,shots", [(68, 57, 1), (400, 300, 3)])
+def test_short_segments_of_an_exact_gradient_run_as_segments_of_eight_steps(nx, nz, shots):
+    out, held = [], []
+    for ck in (1, 2, 7, 8, 50, 0):
+        m = model(nx, nz, [(20 + 9 * k, 20) for k in range(shots)], [(26, 24), (40, 30)],
+                  shots=[[k] for k in range(shots)], nt=70)
+        m.set_observed_data(*[0.0 * a for a in m.get_observed_data()])
+        misfit, g = m.exact_gradient(ck)
+        out.append([np.array(misfit)] + list(g))
+        held.append(m.exact_bytes(ck))
+    for o in out[1:]:
+        assert all(np.array_equal(a, b) for a, b in zip(o, out[0]))
+    assert held[0] == held[1] == held[2] == held[3]
