@@ -615,7 +615,9 @@ resident::ExactPlan Model::exact_plan(int lanes) const {
 // fit): the fewest that take the shots in as few turns as fit on the device and
 // in 60 % of its free memory, up to kMaxResidentLanes (a step at 250 x 150, eight
 // shots: four 16-CTA clusters 1.9 us per shot, eight lanes for the seven that
-// run at once 1.2).
+// run at once 1.2). The kept rates are padded to whole warps (2.6 times a state
+// at 2000 x 66 points), so one lane too has to fit in the free memory, unless
+// per-step launches would need as much.
 int Model::exact_resident_lanes(int C, int n_list, resident::ExactPlan *plan) const {
   *plan = resident::ExactPlan();
   if (!use_resident()) return 0;
@@ -629,7 +631,9 @@ int Model::exact_resident_lanes(int C, int n_list, resident::ExactPlan *plan) co
     if (lanes > kMaxResidentLanes) continue;
     const resident::ExactPlan p = exact_plan(lanes);
     if (p.p.ctas() <= 0) continue;
-    if (lanes > 1 && static_cast<double>(lanes) * exact_resident_bytes(C, p) > 0.6 * free_b) continue;
+    const double bytes = static_cast<double>(lanes) * exact_resident_bytes(C, p);
+    if (lanes > 1 ? bytes > 0.6 * free_b : bytes > 0.9 * free_b && bytes > exact_lane_bytes(C))
+      continue;
     *plan = p;
     return lanes;
   }
@@ -1352,7 +1356,7 @@ double Model::exact_gradient_lanes(int C, const std::vector<int> &shot_list) {
       enqueue();
       continue;
     }
-    GraphEntry &ge = graphs_[std::make_tuple(3 + li, shot, K, C)];
+    GraphEntry &ge = graphs_[std::make_tuple((on_chip_lanes > 0 ? 40 : 3) + li, shot, K, C)];
     if (ge.exec) {
       cuda_check(cudaGraphLaunch(ge.exec, s), "cudaGraphLaunch");
       continue;

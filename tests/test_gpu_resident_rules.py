@@ -128,3 +128,16 @@ def test_short_segments_of_an_exact_gradient_run_as_segments_of_eight_steps(nx, 
     for o in out[1:]:
         assert all(np.array_equal(a, b) for a, b in zip(o, out[0]))
     assert held[0] == held[1] == held[2] == held[3]
+
+
+def test_exact_gradients_that_fit_by_per_step_launches_still_do():
+    # 2000 x 66 points split into two columns of 17 pairs: kept on chip, the rates
+    # of a step take 2.6 times a state. A run whose states take half of the free
+    # memory has to stay below it. (Nothing is allocated here.)
+    import torch
+
+    free = torch.cuda.mem_get_info()[0]
+    nt = int(0.5 * free / (5 * 2000 * 68 * 4)) // 10 * 10
+    m = model(2000, 66, [(20, 20)], [(24, 24)], nt=nt)
+    assert m.exact_bytes(0) <= 0.9 * free
+    assert m.exact_bytes(100) <= 0.1 * free
