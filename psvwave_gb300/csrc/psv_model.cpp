@@ -1895,11 +1895,14 @@ int Model::profile_forward(int shot, int n_steps, double *per_step_ms, double *k
   void *second[5] = {fields2_[0].get(), fields2_[1].get(), fields2_[2].get(), fields2_[3].get(),
                      fields2_[4].get()};
   cudaError_t err;
-  if (variant_ == kFusedTmaPersistent || variant_ == kFusedCluster) {
+  const bool f64 = use_resident64();
+  if (f64 || use_resident() || variant_ == kFusedTmaPersistent) {
     // One launch for all steps: time it whole; the per-step figure is its
     // share.
     cudaEventRecord(ev.front(), stream());
-    err = tma_forward(shot, false, 0, n_steps, true, false, nullptr);
+    err = f64 ? resident64::steps(a, plans_[shot], resident64_, shot, false, 0, n_steps, true,
+                                  false, mail_.get(), err_flag_.as<int>(), stream())
+              : tma_forward(shot, false, 0, n_steps, true, false, nullptr);
     cudaEventRecord(ev.back(), stream());
     cudaError_t sync = cudaStreamSynchronize(stream());
     float ms = 0;
@@ -1907,6 +1910,7 @@ int Model::profile_forward(int shot, int n_steps, double *per_step_ms, double *k
     for (auto &e : ev) cudaEventDestroy(e);
     cuda_check(err, "profile_forward");
     cuda_check(sync, "profile_forward");
+    check_device_error();
     if (per_step_ms) *per_step_ms = ms / n_steps;
     if (kernel_ms && max_kernels > 0) kernel_ms[0] = ms / n_steps;
     return 1;
@@ -1914,7 +1918,7 @@ int Model::profile_forward(int shot, int n_steps, double *per_step_ms, double *k
   if (prec_ == PSV_FP64)
     err = forward_f64(a, plans_[shot], shot, false, 0, n_steps, true, false, stream());
   else if (variant_ == kFusedTma)
-    err = tma_forward(shot, false, 0, n_steps, true, false, a.events, false);
+    err = tma_forward(shot, false, 0, n_steps, true, false, a.events);
   else if (variant_ == kFused)
     err = fast::forward(a, second, &cur_, plans_[shot], shot, false, 0, n_steps, true, false,
                         stream());
@@ -1970,10 +1974,11 @@ void Model::set_variant(int v) {
 }
 
 const char *Model::step_kernel_name(int k) const {
+  if (use_resident()) return k == 0 ? "resident_steps" : "";
+  if (use_resident64()) return k == 0 ? "resident_steps_f64" : "";
   if (variant_ == kFused) return k == 0 ? "fused_step" : "";
   if (variant_ == kFusedTma) return k == 0 ? "fused_step_tma" : "";
   if (variant_ == kFusedTmaPersistent) return k == 0 ? "fused_steps_tma" : "";
-  if (variant_ == kFusedCluster) return k == 0 ? "resident_steps" : "";
   return k == 0 ? "stress_step" : (k == 1 ? "velocity_step" : "");
 }
 

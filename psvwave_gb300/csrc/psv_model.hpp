@@ -168,7 +168,7 @@ class Model {
   void get_exact_gradient(double *g_vp, double *g_vs, double *g_rho, bool device_pointers);
   size_t exact_bytes(int checkpoint_every) const;
   int variant() const { return variant_; }
-  int kernels_per_step() const { return variant_ == kTwoKernel ? 2 : 1; }
+  int kernels_per_step() const { return variant_ == kTwoKernel && !use_resident64() ? 2 : 1; }
   // The FP32 variants built on the TMA step's descriptors (the resident
   // scheme shares them, and the exact adjoint's recompute runs the TMA step).
   bool is_tma() const {

@@ -141,3 +141,19 @@ def test_exact_gradients_that_fit_by_per_step_launches_still_do():
     m = model(2000, 66, [(20, 20)], [(24, 24)], nt=nt)
     assert m.exact_bytes(0) <= 0.9 * free
     assert m.exact_bytes(100) <= 0.1 * free
+
+
+@pytest.mark.parametrize("nx,nz,precision,variant,kernels", [
+    (68, 57, "fp32", None, {"resident_steps"}), (400, 300, "fp32", None, {"resident_steps"}),
+    (400, 300, "fp32", "fused_tma", {"fused_step_tma"}),
+    (400, 300, "fp32", "fused_tma_persistent", {"fused_steps_tma"}),
+    (400, 300, "fp32", "fused_cluster", {"resident_steps"}),
+    (68, 57, "fp64", None, {"resident_steps_f64"}),
+    (68, 57, "fp64", "two_kernel", {"stress_step", "velocity_step"})])
+def test_profile_times_the_kernel_that_simulations_run(nx, nz, precision, variant, kernels):
+    m = model(nx, nz, [(20, 20)], [(24, 24)], precision=precision)
+    if variant:
+        m.kernel_variant = variant
+    per_step, ms = m.profile_forward(0, 50)
+    assert set(ms) == kernels
+    assert 0 < max(ms.values()) <= per_step * 1.001
