@@ -266,7 +266,7 @@ const char *psv_step_kernel_name(const psv_model *m, int k);
  * a step as soon as their neighbours have finished the previous one; the
  * default on large grids) or PSV_VARIANT_FUSED_CLUSTER (every time step in
  * one launch that keeps the grid on chip; the default on small grids). Until
- * a variant or tile shape is set, larger grids that fit on the chip run
+ * a variant or another tile shape is set, larger grids that fit on the chip run
  * resident as well. Results of the FP32 variants agree to FP32 rounding. No
  * counterpart in the reference. */
 enum psv_variant {

@@ -1621,10 +1621,9 @@ void Model::get_exact_gradient(double *g_vp, double *g_vs, double *g_rho, bool d
 void Model::set_tile_cfg(int cfg) {
   if (cfg < 0 || cfg >= tma::kNumTileCfgs) throw Error(PSV_ERR_INVALID_ARGUMENT, "unknown tile shape");
   DeviceGuard guard(device_);
-  if (resident_on_) clear_graphs();
-  resident_on_ = false;
   if (cfg == tile_cfg_) return;
   clear_graphs();
+  resident_on_ = false;
   tile_cfg_ = cfg;
   if (tma_ok_) {
     synchronize();

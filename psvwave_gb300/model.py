@@ -584,9 +584,9 @@ class fdModel:
         (all time steps in one launch that keeps the grid on chip; the
         default on small grids), 'fused' (one launch per step, FP32) or
         'two_kernel' (stress and velocity launches; the FP64 variant).
-        Until a variant or tile shape is set (or autotuned), larger grids
-        that fit on the chip run resident too, and the variant names the
-        step that takes over when they do not."""
+        Until a variant or another tile shape is set (or autotuned), larger
+        grids that fit on the chip run resident too, and the variant names
+        the step that takes over when they do not."""
         v = ctypes.c_int()
         _capi.check(self._lib.psv_get_kernel_variant(self._h, ctypes.byref(v)))
         return {k: n for n, k in self.VARIANTS.items()}[v.value]

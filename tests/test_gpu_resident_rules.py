@@ -157,3 +157,11 @@ def test_profile_times_the_kernel_that_simulations_run(nx, nz, precision, varian
     per_step, ms = m.profile_forward(0, 50)
     assert set(ms) == kernels
     assert 0 < max(ms.values()) <= per_step * 1.001
+
+
+def test_setting_the_tile_shape_a_model_has_changes_nothing():
+    m = model(400, 300, [(20, 20)], [(24, 24)])
+    m.tile_shape = m.tile_shape
+    assert set(m.profile_forward(0, 20)[1]) == {"resident_steps"}
+    m.tile_shape = "32x60"  # another one selects the tile step
+    assert set(m.profile_forward(0, 20)[1]) == {"fused_step_tma"}
