@@ -267,14 +267,17 @@ const char *psv_step_kernel_name(const psv_model *m, int k);
  * default on large grids) or PSV_VARIANT_FUSED_CLUSTER (every time step in
  * one launch that keeps the grid on chip; the default on small grids). Until
  * a variant or another tile shape is set, larger grids that fit on the chip run
- * resident as well. Results of the FP32 variants agree to FP32 rounding. No
- * counterpart in the reference. */
+ * resident as well, and so do FP64 grids that fit. Setting PSV_VARIANT_DEFAULT
+ * returns to the choice a new model has (the getter then names its variant).
+ * Results of the FP32 variants agree to FP32 rounding; FP64 runs are the same
+ * bits either way. No counterpart in the reference. */
 enum psv_variant {
   PSV_VARIANT_FUSED = 0,
   PSV_VARIANT_TWO_KERNEL = 1,
   PSV_VARIANT_FUSED_TMA = 2,
   PSV_VARIANT_FUSED_TMA_PERSISTENT = 3,
-  PSV_VARIANT_FUSED_CLUSTER = 4
+  PSV_VARIANT_FUSED_CLUSTER = 4,
+  PSV_VARIANT_DEFAULT = 5
 };
 int psv_set_kernel_variant(psv_model *m, int variant);
 int psv_get_kernel_variant(const psv_model *m, int *variant);

@@ -122,6 +122,7 @@ Model::Model(const Config &cfg, int precision, int device)
     resident_on_ = resident_.ctas() > 0;
   }
   if (prec_ == PSV_FP64) resident_on_ = resident64_.ctas() > 0;
+  default_variant_ = variant_;
   synchronize();
 }
 
@@ -162,6 +163,7 @@ Model::Model(const Model &o)
   }
   build_descs();
   resident_on_ = o.resident_on_;
+  default_variant_ = o.default_variant_;
 }
 
 Model::~Model() {
@@ -1948,6 +1950,11 @@ int Model::profile_forward(int shot, int n_steps, double *per_step_ms, double *k
 }
 
 void Model::set_variant(int v) {
+  if (v == PSV_VARIANT_DEFAULT) {
+    set_variant(default_variant_);
+    resident_on_ = resident_.ctas() > 0 || resident64_.ctas() > 0;
+    return;
+  }
   if (v != kFused && v != kTwoKernel && v != kFusedTma && v != kFusedTmaPersistent &&
       v != kFusedCluster)
     throw Error(PSV_ERR_INVALID_ARGUMENT, "unknown kernel variant");

@@ -226,6 +226,7 @@ class Model {
   // for models whose variant and tile shape were left to the default.
   resident::Plan resident_;
   bool resident_on_ = false;
+  int default_variant_ = kTwoKernel;  // a new model's
   bool use_resident() const {
     return resident_.ctas() > 0 && (variant_ == kFusedCluster || resident_on_);
   }

@@ -574,7 +574,7 @@ class fdModel:
         return per_step.value, dict(zip(names, list(ks)[:n.value]))
 
     VARIANTS = {"fused": 0, "two_kernel": 1, "fused_tma": 2, "fused_tma_persistent": 3,
-                "fused_cluster": 4}
+                "fused_cluster": 4, "default": 5}
 
     @property
     def kernel_variant(self):
@@ -586,7 +586,8 @@ class fdModel:
         'two_kernel' (stress and velocity launches; the FP64 variant).
         Until a variant or another tile shape is set (or autotuned), larger
         grids that fit on the chip run resident too, and the variant names
-        the step that takes over when they do not."""
+        the step that takes over when they do not; FP64 models that fit
+        run resident likewise. Setting 'default' returns to that choice."""
         v = ctypes.c_int()
         _capi.check(self._lib.psv_get_kernel_variant(self._h, ctypes.byref(v)))
         return {k: n for n, k in self.VARIANTS.items()}[v.value]

@@ -165,3 +165,22 @@ def test_setting_the_tile_shape_a_model_has_changes_nothing():
     assert set(m.profile_forward(0, 20)[1]) == {"resident_steps"}
     m.tile_shape = "32x60"  # another one selects the tile step
     assert set(m.profile_forward(0, 20)[1]) == {"fused_step_tma"}
+
+
+@pytest.mark.parametrize("nx,nz,precision,other", [
+    (68, 57, "fp32", "fused_tma"), (400, 300, "fp32", "fused_tma"),
+    (68, 57, "fp64", "two_kernel"), (520, 600, "fp64", "two_kernel")])
+def test_default_variant_restores_a_new_models_choice(nx, nz, precision, other):
+    m = model(nx, nz, [(20, 20)], [(24, 24)], precision=precision)
+    name, kernels = m.kernel_variant, set(m.profile_forward(0, 20)[1])
+    m.forward_simulate(0, False)
+    ref = m.get_synthetic_data()
+    m.kernel_variant = other
+    if nx * nz < 200000:
+        assert set(m.profile_forward(0, 20)[1]) != kernels
+    m.forward_simulate(0, False)
+    m.kernel_variant = "default"
+    assert m.kernel_variant == name and set(m.profile_forward(0, 20)[1]) == kernels
+    for _ in range(3):
+        m.forward_simulate(0, False)
+        assert all(np.array_equal(a, b) for a, b in zip(m.get_synthetic_data(), ref))
