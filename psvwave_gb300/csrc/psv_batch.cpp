@@ -558,7 +558,7 @@ int Batch::autotune(int n_steps) {
     }
   }
   // The resident scheme, in clusters and in mailbox teams with one or two
-  // CTAs per SM (few launches: timed on the second run).
+  // CTAs per SM, timed alike.
   bool best_cluster = false;
   Layout best_layout;
   if (cluster_fits()) {
@@ -578,6 +578,7 @@ int Batch::autotune(int n_steps) {
       layout_ = l;
       packed_.clear();
       set_cluster(true);
+      forward(false, n_steps);
       forward(false, n_steps);
       cudaEventRecord(a, stream_);
       forward(false, n_steps);

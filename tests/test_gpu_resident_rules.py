@@ -184,3 +184,15 @@ def test_default_variant_restores_a_new_models_choice(nx, nz, precision, other):
     for _ in range(3):
         m.forward_simulate(0, False)
         assert all(np.array_equal(a, b) for a, b in zip(m.get_synthetic_data(), ref))
+
+
+def test_batch_autotune_times_every_scheme_on_a_graph_replay():
+    # 16 steps of 64 small members: 0.32 ms resident, 0.44 ms by tiles. With the
+    # capture of its graph inside the timed window the resident scheme lost.
+    ms = [model(68, 57, [(20, 20)], [(24, 24)]) for _ in range(64)]
+    b = psv.Batch()
+    for m in ms:
+        b.add(m, 0)
+    for _ in range(3):
+        b.autotune(16)
+        assert b.cluster
