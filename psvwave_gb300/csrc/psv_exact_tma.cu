@@ -48,6 +48,7 @@
 #include "psv_exact_tma.hpp"
 
 #include <algorithm>
+#include <atomic>
 #include <cstdint>
 
 #include "psv_tma.hpp"
@@ -542,7 +543,7 @@ cudaError_t accumulate(size_t n, const float2 *const ff[4], double *const out[4]
 }
 
 cudaError_t step(const Maps &maps, const Step &a, cudaStream_t s) {
-  static unsigned long long configured = 0;
+  static std::atomic<unsigned long long> configured{0};
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;

@@ -18,6 +18,7 @@
 // fused in.
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <cstdint>
 
 #include "psv_fast.hpp"
@@ -252,7 +253,7 @@ __global__ void __launch_bounds__(NT, 4) fused_step(const StepArgs a) {
 template <bool ADJ>
 cudaError_t launch(const StepArgs &a, cudaStream_t s) {
   // The shared-memory opt-in is a per-device attribute: set it once per device.
-  static unsigned long long configured = 0;
+  static std::atomic<unsigned long long> configured{0};
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;

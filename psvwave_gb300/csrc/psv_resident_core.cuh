@@ -52,6 +52,7 @@
 #include <cooperative_groups.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cstdint>
 #include <vector>
 
@@ -1061,7 +1062,7 @@ bool device(Device &q) {
 // Per-device launch attributes of a kernel, set once: the device's largest
 // shared memory, and clusters above the portable size.
 template <class Kern>
-cudaError_t configure(Kern kern, bool cluster, unsigned long long &configured) {
+cudaError_t configure(Kern kern, bool cluster, std::atomic<unsigned long long> &configured) {
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;

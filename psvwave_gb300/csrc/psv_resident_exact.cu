@@ -42,7 +42,7 @@ template <int MODE, class T>
 cudaError_t run(T, const tma::SimDesc &d, const ExactPlan &q, int it0, int n_steps, bool zero,
                 const RateIo &io, void *mail, int *err, cudaStream_t s) {
   auto kern = resident_exact<MODE, T::K, T::S, T::CL>;
-  static unsigned long long configured = 0;
+  static std::atomic<unsigned long long> configured{0};
   cudaError_t e = configure(kern, T::CL, configured);
   if (e != cudaSuccess) return e;
   const Plan &p = q.p;

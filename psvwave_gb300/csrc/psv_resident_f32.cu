@@ -40,7 +40,7 @@ template <int MODE, class T>
 cudaError_t run(T, const tma::SimDesc &d, const Plan &p, int it0, int n_steps, int parity, int zero,
                 int store, const Dump &dump, void *mail, int *err, cudaStream_t s) {
   auto kern = resident_steps<MODE, T::K, T::S, T::CL>;
-  static unsigned long long configured = 0;
+  static std::atomic<unsigned long long> configured{0};
   cudaError_t e = configure(kern, T::CL, configured);
   if (e != cudaSuccess) return e;
   cudaLaunchAttribute attr;
@@ -55,7 +55,7 @@ int active_clusters(const Plan &p) {
   with_plan(p.rows, p.stride, true, [&](auto t) {
     using T = decltype(t);
     auto kern = resident_steps_batch<T::K, T::S, true>;
-    static unsigned long long configured = 0;
+    static std::atomic<unsigned long long> configured{0};
     cudaError_t e = configure(kern, true, configured);
     if (e != cudaSuccess) return e;
     cudaLaunchAttribute attr;
@@ -237,7 +237,7 @@ cudaError_t steps_batch(const tma::SimDesc *sims, const Member *members, const i
   return with_plan(l.rows, l.stride, l.team > 0, [&](auto t) {
     using T = decltype(t);
     auto kern = resident_steps_batch<T::K, T::S, T::CL>;
-    static unsigned long long configured = 0;
+    static std::atomic<unsigned long long> configured{0};
     cudaError_t e = configure(kern, T::CL, configured);
     if (e != cudaSuccess) return e;
     cudaLaunchAttribute attr;

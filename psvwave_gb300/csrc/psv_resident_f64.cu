@@ -33,6 +33,7 @@
 #include "psv_resident_f64.hpp"
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstdint>
 #include <vector>
@@ -574,7 +575,7 @@ size_t mailbox_bytes(const Plan &p) { return (size_t)p.ctas() * p.box * sizeof(W
 namespace {
 template <bool ADJ, int K, bool Z>
 cudaError_t launch(const Args &a, const Plan &p, cudaStream_t s) {
-  static unsigned long long configured = 0;
+  static std::atomic<unsigned long long> configured{0};
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;

@@ -40,6 +40,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cstdint>
 
 #include "psv_tma.hpp"
@@ -957,7 +958,7 @@ __global__ void __launch_bounds__(S::NT, S::MINB)
 
 // The shared-memory opt-in is a per-device attribute: set it once per device.
 template <class K>
-cudaError_t configure(K kernel, int smem, unsigned long long &configured) {
+cudaError_t configure(K kernel, int smem, std::atomic<unsigned long long> &configured) {
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
@@ -973,7 +974,7 @@ cudaError_t configure(K kernel, int smem, unsigned long long &configured) {
 template <class S, int CFG, bool ADJ>
 cudaError_t launch(const SimDesc *sims, const int4 *tiles, int n_tiles, const int *active, int it,
                    int parity, int store, int *err, cudaStream_t s) {
-  static unsigned long long configured = 0;
+  static std::atomic<unsigned long long> configured{0};
   cudaError_t e = configure(fused_step_tma_batch<S, CFG, ADJ>, S::SMEM, configured);
   if (e != cudaSuccess) return e;
   if (n_tiles <= 0) return cudaSuccess;
@@ -997,7 +998,7 @@ cudaError_t launch(const SimDesc *sims, const int4 *tiles, int n_tiles, const in
 template <class S, int CFG, bool ADJ>
 cudaError_t launch_persistent(const SimDesc &d, int it0, int n_steps, int parity0, int store,
                               int *err, unsigned *sched, cudaStream_t s) {
-  static unsigned long long configured = 0;
+  static std::atomic<unsigned long long> configured{0};
   cudaError_t e = configure(fused_steps_tma<S, CFG, ADJ>, S::SMEM, configured);
   if (e != cudaSuccess) return e;
   if (n_steps <= 0) return cudaSuccess;
@@ -1036,7 +1037,7 @@ cudaError_t launch_persistent(const SimDesc &d, int it0, int n_steps, int parity
 template <class S, int CFG, bool ADJ>
 cudaError_t launch_single(const SimDesc &d, int it, int parity, int store, int *err,
                           cudaStream_t s) {
-  static unsigned long long configured = 0;
+  static std::atomic<unsigned long long> configured{0};
   cudaError_t e = configure(fused_step_tma<S, CFG, ADJ>, S::SMEM, configured);
   if (e != cudaSuccess) return e;
   const int tiles_x = (d.nx + S::TX - 1) / S::TX, tiles_z = (d.nz + S::TZ - 1) / S::TZ;
@@ -1190,7 +1191,7 @@ size_t sched_words(int cfg, int nx, int nz) { return 1 + (size_t)tile_count(cfg,
 namespace {
 template <class S, int CFG, bool ADJ>
 int resident() {
-  static unsigned long long configured = 0;
+  static std::atomic<unsigned long long> configured{0};
   if (configure(fused_steps_tma<S, CFG, ADJ>, S::SMEM, configured) != cudaSuccess) return 0;
   int dev = 0, sms = 0, per_sm = 0;
   if (cudaGetDevice(&dev) != cudaSuccess ||
@@ -1206,7 +1207,7 @@ template <class S, int CFG>
 cudaError_t launch_persistent_batch(const SimDesc *sims, const int4 *tiles, int n_tiles,
                                     const int *active, int n_steps, int store, int *err,
                                     unsigned *sched, cudaStream_t s) {
-  static unsigned long long configured = 0;
+  static std::atomic<unsigned long long> configured{0};
   cudaError_t e = configure(fused_steps_tma_batch<S, CFG>, S::SMEM, configured);
   if (e != cudaSuccess) return e;
   if (n_steps <= 0 || n_tiles <= 0) return cudaSuccess;

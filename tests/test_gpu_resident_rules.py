@@ -196,3 +196,36 @@ def test_batch_autotune_times_every_scheme_on_a_graph_replay():
     for _ in range(3):
         b.autotune(16)
         assert b.cluster
+
+
+def test_models_that_take_the_whole_device_run_from_several_threads():
+    # Two of them spread over every SM by mailboxes (one in each precision), one
+    # on a cluster: a team starts only once all its CTAs are on the device, so
+    # none waits for a neighbour that another simulation keeps away.
+    import threading
+
+    ms = [model(1103, 497, [(200, 200)], [(230, 210)]),
+          model(400, 300, [(100, 100)], [(120, 110)], precision="fp64"),
+          model(700, 400, [(150, 100)], [(170, 110)]),
+          model(250, 151, [(100, 50)], [(120, 60)])]
+    ref = []
+    for m in ms:
+        m.forward_simulate(0, False)
+        ref.append([a.copy() for a in m.get_synthetic_data()])
+    wrong = []
+
+    def run(m, r):
+        try:
+            for _ in range(20):
+                m.forward_simulate(0, False)
+                if not all(np.array_equal(a, b) for a, b in zip(m.get_synthetic_data(), r)):
+                    wrong.append("results")
+        except Exception as e:
+            wrong.append(repr(e))
+
+    threads = [threading.Thread(target=run, args=x) for x in zip(ms, ref)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not wrong
