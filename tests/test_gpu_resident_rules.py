@@ -229,3 +229,25 @@ def test_models_that_take_the_whole_device_run_from_several_threads():
     for t in threads:
         t.join()
     assert not wrong
+
+
+@pytest.mark.parametrize("others", [0, 2])
+def test_batches_with_a_member_too_large_for_the_chip_refuse_the_resident_scheme(others):
+    ms = [model(2100, 900, [(200, 200)], [(230, 210)])]
+    ms += [model(68, 57, [(20, 20)], [(24, 24)]) for _ in range(others)]
+    b = psv.Batch()
+    for m in ms:
+        b.add(m, 0)
+    assert not b.cluster_fits
+    with pytest.raises(ValueError):
+        b.cluster = True
+    assert not b.cluster
+    b.autotune(4)
+    assert not b.cluster
+    b.forward()
+    for m in ms:
+        out = m.get_synthetic_data()
+        m.kernel_variant = "fused_tma_persistent"
+        m.forward_simulate(0, False)
+        for a, c in zip(out, m.get_synthetic_data()):
+            assert np.linalg.norm(a - c) <= 1e-4 * np.linalg.norm(c)
