@@ -462,7 +462,7 @@ void Batch::forward(bool store, int n_steps) {
   cuda_check(cudaMemcpy(&flag, err_flag_.get(), sizeof(int), cudaMemcpyDeviceToHost), "error flag");
   if (flag) {
     cudaMemsetAsync(err_flag_.get(), 0, sizeof(int), stream_);
-    throw Error(PSV_ERR_CUDA, "a CTA timed out waiting for its TMA tile copies");
+    throw Error(PSV_ERR_CUDA, tma::wait_error(flag));
   }
 }
 

@@ -1687,7 +1687,7 @@ void Model::check_device_error() {
   if (flag) {
     cudaMemsetAsync(err_flag_.get(), 0, sizeof(int), stream());
     cudaStreamSynchronize(stream());
-    throw Error(PSV_ERR_CUDA, "a CTA timed out waiting for its TMA tile copies");
+    throw Error(PSV_ERR_CUDA, tma::wait_error(flag));
   }
 }
 

@@ -28,6 +28,15 @@ struct Maps {
 enum TileCfg { kTile32x60 = 0, kTile16x28 = 1, kTile20x28 = 2, kTile16x60 = 3, kNumTileCfgs = 4 };
 void tile_dims(int cfg, int *tx, int *tz);
 
+// What a kernel's bounded wait that ran out raises in *err: 1 a tile's copies, 2
+// the neighbouring tiles of a persistent launch, 4 a neighbour's edges or kept
+// rates of a resident one.
+inline const char *wait_error(int flags) {
+  if (flags & 4) return "a CTA timed out waiting for its neighbours in a resident launch";
+  if (flags & 2) return "a CTA timed out waiting for neighbouring tiles in a persistent launch";
+  return "a CTA timed out waiting for its TMA tile copies";
+}
+
 // Everything a CTA needs about its simulation; lives in device memory.
 struct alignas(128) SimDesc {
   Maps maps[2];                // tensor maps for the descriptor's tile shape; parity p reads set p
