@@ -40,8 +40,13 @@
 //    step j.
 //
 // Points outside the updated region [2, n - 2) carry lm = mu = b = 0 and a
-// taper factor of 1: their update adds zero. Arithmetic is written with
-// explicit fused multiply-adds so that every instantiation rounds alike.
+// taper factor of 1: their update adds zero, or NaN where a diverging run has
+// infinities around them. That goes no further than the infinities do (such a
+// point is next to updated ones along one axis only, and reads and is read along
+// it), and leaves as the zero it replaced. (Points excepted from the update
+// one by one, by selects or predicated multiplications, cost 1 to 4 % of every
+// run.) Arithmetic is written with explicit fused multiply-adds so that every
+// instantiation rounds alike.
 //
 // Every wait is bounded: a thread whose wait runs out raises *err and stops
 // waiting for the rest of the launch, which then ends by itself.
@@ -680,11 +685,39 @@ __device__ __forceinline__ void member_steps(const tma::SimDesc &d, const Team &
     return;
   }
 
+  // Row k's fields as they leave the launch: NaN of points outside the updated
+  // region back to zero.
+  auto leave = [&](int k) {
+    const int x = x0 + r0 + k;
+    auto clear = [](float &v) { v = isnan(v) ? 0.f : v; };
+    if (!in_region(x, z)) {
+      clear(vx[k].x);
+      clear(vz[k].x);
+      clear(xx[k].x);
+      clear(zz[k].x);
+      clear(xz[k].x);
+    }
+    if (!in_region(x, z + 1)) {
+      clear(vx[k].y);
+      clear(vz[k].y);
+      clear(xx[k].y);
+      clear(zz[k].y);
+      clear(xz[k].y);
+    }
+  };
+  // kExact: the same for a pair of gradient sums.
+  auto leaves = [&](float2 v, int k) {
+    const int x = x0 + r0 + k;
+    if (isnan(v.x) && !in_region(x, z)) v.x = 0.f;
+    if (isnan(v.y) && !in_region(x, z + 1)) v.y = 0.f;
+    return v;
+  };
   auto save = [&](float *base) {
     const size_t gp = (size_t)nx * ps;
 #pragma unroll
     for (int k = 0; k < K; ++k) {
       if (k >= kn) continue;
+      leave(k);
       float *q = base + (size_t)(x0 + r0 + k) * ps + z;
       if (z + 1 < nz) {
         sts2(q, vx[k]);
@@ -815,6 +848,7 @@ __device__ __forceinline__ void member_steps(const tma::SimDesc &d, const Team &
 #pragma unroll
       for (int k = 0; k < K; ++k) {
         if (k >= kn) continue;
+        if (!ADJ) leave(k);
         const int x = x0 + r0 + k;
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
@@ -1016,7 +1050,7 @@ __device__ __forceinline__ void member_steps(const tma::SimDesc &d, const Team &
 #pragma unroll 1
         for (int k = 0; k < kn; ++k, to += ps, sum += 4 * (S - 4))
           for (int p = 0; p < 3; ++p) {
-            sts2(to + (size_t)p * nx * ps, lds2(sum + p * (S - 4)));
+            sts2(to + (size_t)p * nx * ps, leaves(lds2(sum + p * (S - 4)), k));
             sts2(sum + p * (S - 4), zero2);
           }
       }
@@ -1032,6 +1066,7 @@ __device__ __forceinline__ void member_steps(const tma::SimDesc &d, const Team &
 #pragma unroll
     for (int k = 0; k < K; ++k) {
       if (k >= kn) continue;
+      if (!EX) leave(k);
       const size_t o = (size_t)(x0 + r0 + k) * ps + z;
       const float2 v[5] = {vx[k], vz[k], xx[k], zz[k], xz[k]};
 #pragma unroll
@@ -1042,7 +1077,7 @@ __device__ __forceinline__ void member_steps(const tma::SimDesc &d, const Team &
       if (EX)
         for (int p = 0; p < 3; ++p)
           *reinterpret_cast<float2 *>(io.part + (size_t)p * nx * ps + o) =
-              lds2(G + ((r0 + k) * 4 + p) * (S - 4) + 2 * c);
+              leaves(lds2(G + ((r0 + k) * 4 + p) * (S - 4) + 2 * c), k);
     }
   }
   if (CLUSTER) cg::this_cluster().sync();

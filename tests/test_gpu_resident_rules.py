@@ -251,3 +251,32 @@ def test_batches_with_a_member_too_large_for_the_chip_refuse_the_resident_scheme
         m.forward_simulate(0, False)
         for a, c in zip(out, m.get_synthetic_data()):
             assert np.linalg.norm(a - c) <= 1e-4 * np.linalg.norm(c)
+
+
+@pytest.mark.parametrize("nx,nz", [(68, 57), (250, 151), (31, 700), (400, 300)])
+def test_points_outside_the_updated_region_stay_out_of_a_diverging_run(nx, nz):
+    # A time step ten times too long: infinities and NaN everywhere inside, the
+    # outermost two rows and columns as they were.
+    def rim(f):
+        g = np.array(f)
+        g[..., 2:-2, 2:-2] = 0.0
+        return g
+
+    for variant in (None, "fused_tma"):
+        m = model(nx, nz, [(nx // 3, nz // 3)], [(nx // 2, nz // 2)], dt=2.5e-3)
+        if variant:
+            m.kernel_variant = variant
+        m.forward_simulate(0, True)
+        fields = m.get_wavefields() + m.get_snapshots()
+        assert all(not np.isfinite(f).all() for f in fields[:5])
+        assert all(not rim(f).any() for f in fields)
+        m.calculate_l2_misfit()
+        m.calculate_l2_adjoint_sources()
+        m.reset_kernels()
+        m.adjoint_simulate(0)
+        fields = m.get_wavefields()
+        assert all(not np.isfinite(f).all() for f in fields)
+        assert all(not rim(f).any() for f in fields)
+        g = m.exact_gradient(50)[1]
+        assert all(not np.isfinite(f).all() for f in g)
+        assert all(not rim(f).any() for f in g)
