@@ -181,7 +181,7 @@ class SurrogateNet:
         n, dev = self.norm, torch.device("cuda", self.device)
         gs = n["gs"]
         if not (isinstance(gs, torch.Tensor) and gs.dtype == torch.float32 and gs.device == dev
-                and tuple(gs.shape) == (3, 20, 10) and gs.is_contiguous()
+                and tuple(gs.shape) == (3, 20, 10) and gs.is_contiguous() and not gs.requires_grad
                 and isinstance(n["m0"], float) and isinstance(n["ms"], float)):
             m, g = self.predict_features(self.features(z))
             return n["m0"] + n["ms"] * m.double(), gs * g
