@@ -516,6 +516,7 @@ void Model::build_descs() {
   descs_h_ = std::move(descs);
   resident_ = resident::plan(resident_grid());
   exact_plans_.clear();
+  shot_plans_.clear();
   const size_t mail = resident::mailbox_bytes(resident_);
   if (mail_.bytes() < mail) mail_.allocate(mail, false);
   tma_ok_ = true;
@@ -1022,14 +1023,16 @@ double Model::exact_gradient(int C, const std::vector<int> &shot_list) {
 }
 
 void Model::destroy_lanes() {
-  for (auto &l : lanes_) {
-    if (l->stream) {
-      cudaStreamSynchronize(l->stream);
-      cudaStreamDestroy(l->stream);
+  for (Lanes *lanes : {&lanes_, &shot_lanes_}) {
+    for (auto &l : *lanes) {
+      if (l->stream) {
+        cudaStreamSynchronize(l->stream);
+        cudaStreamDestroy(l->stream);
+      }
+      if (l->done) cudaEventDestroy(l->done);
     }
-    if (l->done) cudaEventDestroy(l->done);
+    lanes->clear();
   }
-  lanes_.clear();
   if (lanes_start_) {
     cudaEventDestroy(lanes_start_);
     lanes_start_ = nullptr;
@@ -1047,25 +1050,25 @@ void Model::destroy_lanes() {
 // same whatever C. Each shot's pipeline is captured once as a CUDA graph on
 // its lane's stream and replayed. At the end the shots' sums are added in
 // shot order, and the chain rule maps them to (vp, vs, rho).
-int Model::ensure_lanes(int K) {
+int Model::ensure_lanes(Lanes &lanes, int K) {
   int changed = 0;
   // Lanes beyond K give their memory back.
-  while (static_cast<int>(lanes_.size()) > K) {
-    auto &l = lanes_.back();
+  while (static_cast<int>(lanes.size()) > K) {
+    auto &l = lanes.back();
     if (l->stream) {
       cuda_check(cudaStreamSynchronize(l->stream), "lane sync");
       cudaStreamDestroy(l->stream);
     }
     if (l->done) cudaEventDestroy(l->done);
-    lanes_.pop_back();
+    lanes.pop_back();
     changed = 1;
   }
-  while (static_cast<int>(lanes_.size()) < K) {
+  while (static_cast<int>(lanes.size()) < K) {
     auto l = std::make_unique<ExactLane>();
-    if (!lanes_.empty())
+    if (!lanes.empty())
       cuda_check(cudaStreamCreateWithFlags(&l->stream, cudaStreamNonBlocking), "lane stream");
     cuda_check(cudaEventCreateWithFlags(&l->done, cudaEventDisableTiming), "lane event");
-    lanes_.push_back(std::move(l));
+    lanes.push_back(std::move(l));
     changed = 1;
   }
   if (!lanes_start_)
@@ -1110,7 +1113,7 @@ double Model::exact_gradient_lanes(int C, const std::vector<int> &shot_list) {
       grown = true;
     }
   };
-  if (ensure_lanes(K)) grown = true;
+  if (ensure_lanes(lanes_, K)) grown = true;
   for (auto &l : lanes_) {
     ensure(l->ckpt, n_ck * state_bytes);
     if (on_chip_lanes > 0) {
@@ -1434,29 +1437,55 @@ double Model::exact_gradient_lanes(int C, const std::vector<int> &shot_list) {
 }
 
 bool Model::run_model_lanes_ok() const {
-  const int shots = cfg_.n_shots;
-  if (prec_ != PSV_FP32 || !tma_ok_ || shots < 2 ||
-      (variant_ != kFusedTma && variant_ != kFusedTmaPersistent))
-    return false;
-  if (!use_resident()) return true;
-  // A grid resident on chip takes the whole device for one shot; per-step
-  // launches of up to kMaxLanes shots overlap. us per step and shot, forward and
-  // adjoint, resident | lanes: 400 x 260, 3 shots 5.5 | 5.4, 4 shots 5.5 | 4.3,
-  // 8 shots 5.4 | 2.6; 700 x 400, 3: 6.8 | 6.8, 4: 6.9 | 5.7, 8: 6.8 | 5.7;
-  // 850 x 420, 4: 7.6 | 6.7, 8: 7.5 | 7.3; 900 x 450, 4: 7.5 | 7.8, 8: 7.6 | 8.6.
-  // A last round of one to three shots costs the lanes most of a full one, at
-  // nine shots: 400 x 260 5.4 | 3.7, 700 x 400 6.8 | 6.9, 850 x 420 7.5 | 8.4.
-  const double cells = static_cast<double>(geo_.nx) * geo_.nz;
-  const int last = shots % kMaxLanes;
-  if (shots < 4 || cells > 3.8e5) return false;
-  return cells <= 2.5e5 || last == 0 || last >= 4;
+  if (prec_ != PSV_FP32 || !tma_ok_ || cfg_.n_shots < 2) return false;
+  if (use_resident()) {
+    resident::Plan plan;
+    return resident_shot_lanes(&plan) > 1;
+  }
+  return variant_ == kFusedTma || variant_ == kFusedTmaPersistent;
 }
 
-// run_model with the shots in concurrent lanes (FP32, per-step TMA
+// Lanes in which run_model takes the shots of a resident grid, each on its
+// share of the device, and their plan (0: one shot after another): the fewest
+// that take them in the fewest turns that fit. ms for 400 steps of eight shots,
+// one after another | concurrent per-step launches | these: 250 x 150 14.2 | 6.8 |
+// 3.7; 320 x 250 15.2 | 7.8 | 5.5; 400 x 260 17.6 | 8.8 | 7.9; 500 x 300 17.0 |
+// 10.7 | 11.3; 600 x 350 17.3 | 13.6 | 15.2; 700 x 400 21.4 | 18.3 | 16.9. Above
+// about 290 k points two lanes do not fit: 800 x 400 24.0 | 21.0 | 24.0, 900 x 450
+// 24.2 | 27.6 | 24.2. (Per-step launches give other bits than forward_simulate and
+// adjoint_simulate do on these grids, and larger rounding errors.) Up to three
+// shots one after another are as quick as per-step lanes were, and keep the
+// serial order of the kernels' FP64 sums.
+int Model::resident_shot_lanes(resident::Plan *plan) const {
+  *plan = resident::Plan();
+  const int shots = cfg_.n_shots;
+  if (!use_resident() || shots < 4) return 0;
+  DeviceGuard guard(device_);
+  for (int turns = 1; turns < shots; ++turns) {
+    const int lanes = (shots + turns - 1) / turns;
+    if (lanes > kMaxResidentLanes) continue;
+    if (lanes < 2) return 0;
+    auto it = shot_plans_.find(lanes);
+    if (it == shot_plans_.end())
+      it = shot_plans_
+               .emplace(lanes, resident_.cluster
+                                   ? resident_
+                                   : resident::plan_mailbox(resident_grid(),
+                                                            resident::resident_slots(1) / lanes, 1))
+               .first;
+    if (it->second.ctas() <= 0) continue;
+    *plan = it->second;
+    return lanes;
+  }
+  return 0;
+}
+
+// run_model with the shots in concurrent lanes (FP32: per-step TMA
 // launches; the persistent scheme's steps are the same tile arithmetic, so
-// the same states). Forward phase: each shot, in lane k % K, advances from
-// zero fields in the lane's two state slots (ping-pong), storing its
-// snapshots and recording its receivers into the lane's raw series, then
+// the same states; or one resident launch a shot, the same bits on any share
+// of the device). Forward phase: each shot, in lane k % K, advances from
+// zero fields in the lane's two state slots (ping-pong; resident: one), storing
+// its snapshots and recording its receivers into the lane's raw series, then
 // its seismograms. The misfit and adjoint sources follow on the model's
 // stream. Adjoint phase: each shot's adjoint in its lane, correlating into
 // the shot's own kernel sums, which are added to the kernels in shot order.
@@ -1466,22 +1495,27 @@ void Model::run_model_lanes(bool simulate_adjoint) {
   DeviceGuard guard(device_);
   ensure_snapshots();
   const int n_shots = cfg_.n_shots, nr = cfg_.nr, nt = cfg_.nt;
-  const int K = std::min(n_shots, kMaxLanes);
+  resident::Plan plan;
+  const int shares = resident_shot_lanes(&plan);
+  const bool on_chip = shares > 0;
+  const int K = on_chip ? shares : std::min(n_shots, kMaxLanes);
+  Lanes &lanes = on_chip ? shot_lanes_ : lanes_;
   const size_t gp = padded_size(), g = grid_size();
   const size_t field_bytes = gp * sizeof(float), state_bytes = 5 * field_bytes;
   cudaStream_t ms = stream();
-  bool grown = ensure_lanes(K) != 0;
+  bool grown = ensure_lanes(lanes, K) != 0;
   auto ensure = [&](DeviceBuffer &b, size_t bytes) {
     if (b.bytes() < bytes) {
       synchronize();
-      for (auto &l : lanes_)
+      for (auto &l : lanes)
         if (l->stream) cuda_check(cudaStreamSynchronize(l->stream), "lane sync");
       b.allocate(bytes);
       grown = true;
     }
   };
-  for (auto &l : lanes_) {
-    ensure(l->slots, 2 * state_bytes);
+  for (auto &l : lanes) {
+    ensure(l->slots, (on_chip ? 1 : 2) * state_bytes);
+    if (on_chip) ensure(l->mail, resident::mailbox_bytes(plan));
     ensure(l->raw, std::max<size_t>(2 * static_cast<size_t>(nr) * nt * sizeof(float), 16));
   }
   ensure(kshots_, static_cast<size_t>(n_shots) * 3 * g * sizeof(double));
@@ -1490,8 +1524,9 @@ void Model::run_model_lanes(bool simulate_adjoint) {
     float *b = reinterpret_cast<float *>(l.slots.as<unsigned char>() + j * state_bytes);
     return fast::Fields{b, b + gp, b + 2 * gp, b + 3 * gp, b + 4 * gp};
   };
-  for (auto &lp : lanes_) {
+  for (auto &lp : lanes) {
     ExactLane &l = *lp;
+    if (on_chip) break;
     if (l.rm_slots == l.slots.get() && l.rm_cfg == tile_cfg_) continue;
     for (int j = 0; j < 2; ++j)
       if (!tma::encode_input_maps(l.rm_maps[j], slot_fields(l, j), lm_.as<float>(),
@@ -1502,11 +1537,15 @@ void Model::run_model_lanes(bool simulate_adjoint) {
   }
   // One shot's forward (adjoint = false) or adjoint, in lane l on stream s.
   auto one = [&](ExactLane &l, int shot, bool adjoint, cudaStream_t s) {
-    cuda_check(cudaMemsetAsync(l.slots.get(), 0, 2 * state_bytes, s), "zero state");
     tma::SimDesc d = descs_h_[adjoint ? n_shots + shot : shot];
-    for (int j = 0; j < 2; ++j) {
-      d.set[j] = slot_fields(l, j);
-      d.maps[j] = l.rm_maps[j];
+    if (on_chip) {
+      d.set[0] = d.set[1] = slot_fields(l, 0);
+    } else {
+      cuda_check(cudaMemsetAsync(l.slots.get(), 0, 2 * state_bytes, s), "zero state");
+      for (int j = 0; j < 2; ++j) {
+        d.set[j] = slot_fields(l, j);
+        d.maps[j] = l.rm_maps[j];
+      }
     }
     float *raw = l.raw.as<float>();
     d.rec_vx = nr ? raw : nullptr;
@@ -1518,8 +1557,12 @@ void Model::run_model_lanes(bool simulate_adjoint) {
       d.kmu = k + g;
       d.krho = k + 2 * g;
     }
+    if (on_chip)
+      cuda_check(resident::steps(d, plan, adjoint, adjoint ? nt - 1 : 0, nt, 0, true, !adjoint,
+                                 resident::Dump(), l.mail.get(), err_flag_.as<int>(), s),
+                 adjoint ? "adjoint_simulate" : "forward_simulate");
     int cur = 0;
-    for (int n = 0; n < nt; ++n) {
+    for (int n = 0; n < nt && !on_chip; ++n) {
       const int it = adjoint ? nt - 1 - n : n;
       cuda_check(tma::step_single(d, tile_cfg_, adjoint, it, cur, !adjoint, err_flag_.as<int>(), s),
                  adjoint ? "adjoint_simulate" : "forward_simulate");
@@ -1536,17 +1579,17 @@ void Model::run_model_lanes(bool simulate_adjoint) {
   auto phase = [&](bool adjoint) {
     cuda_check(cudaEventRecord(lanes_start_, ms), "lane start");
     for (int k = 1; k < K; ++k)
-      cuda_check(cudaStreamWaitEvent(lanes_[k]->stream, lanes_start_, 0), "lane wait");
+      cuda_check(cudaStreamWaitEvent(lanes[k]->stream, lanes_start_, 0), "lane wait");
     for (int shot = 0; shot < n_shots; ++shot) {
       const int li = shot % K;
-      ExactLane &l = *lanes_[li];
+      ExactLane &l = *lanes[li];
       cudaStream_t s = li == 0 ? ms : l.stream;
       auto enqueue = [&] { one(l, shot, adjoint, s); };
       if (!use_graphs_) {
         enqueue();
         continue;
       }
-      GraphEntry &ge = graphs_[std::make_tuple(20 + li, shot, K, adjoint ? 1 : 0)];
+      GraphEntry &ge = graphs_[std::make_tuple((on_chip ? 60 : 20) + li, shot, K, adjoint ? 1 : 0)];
       if (ge.exec) {
         cuda_check(cudaGraphLaunch(ge.exec, s), "cudaGraphLaunch");
         continue;
@@ -1573,15 +1616,15 @@ void Model::run_model_lanes(bool simulate_adjoint) {
       cuda_check(cudaGraphLaunch(ge.exec, s), "cudaGraphLaunch");
     }
     for (int k = 1; k < K; ++k) {
-      cuda_check(cudaEventRecord(lanes_[k]->done, lanes_[k]->stream), "lane done");
-      cuda_check(cudaStreamWaitEvent(ms, lanes_[k]->done, 0), "lane join");
+      cuda_check(cudaEventRecord(lanes[k]->done, lanes[k]->stream), "lane done");
+      cuda_check(cudaStreamWaitEvent(ms, lanes[k]->done, 0), "lane join");
     }
     // The last shot's final state into the model's fields (nt steps from
-    // slot 0 end in slot nt % 2).
-    ExactLane &last = *lanes_[(n_shots - 1) % K];
+    // slot 0 end in slot nt % 2; resident: in the one there is).
+    ExactLane &last = *lanes[(n_shots - 1) % K];
     void *src[5], *dst[5];
     for (int f = 0; f < 5; ++f) {
-      src[f] = last.slots.as<unsigned char>() + (nt & 1) * state_bytes + f * field_bytes;
+      src[f] = last.slots.as<unsigned char>() + (on_chip ? 0 : nt & 1) * state_bytes + f * field_bytes;
       dst[f] = fields_[f].get();
     }
     cuda_check(copy_state(src, dst, nullptr, field_bytes, ms), "final state");

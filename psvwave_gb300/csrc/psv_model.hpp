@@ -319,14 +319,19 @@ class Model {
     const void *rm_slots = nullptr;
     int rm_cfg = -1;
   };
-  // run_model in lanes (FP32, TMA per-step launches): every shot's forward
-  // with snapshots, then every shot's adjoint with kernel correlation into
-  // per-shot sums (kshots_), added in shot order.
+  // run_model in lanes (FP32, TMA per-step launches or grids resident on their
+  // share of the device): every shot's forward with snapshots, then every
+  // shot's adjoint with kernel correlation into per-shot sums (kshots_), added
+  // in shot order.
   DeviceBuffer kshots_;
   bool run_model_lanes_ok() const;
   void run_model_lanes(bool simulate_adjoint);
-  int ensure_lanes(int K);  // makes exactly K lanes; returns 1 when lanes were (re)made
-  std::vector<std::unique_ptr<ExactLane>> lanes_;
+  using Lanes = std::vector<std::unique_ptr<ExactLane>>;
+  int ensure_lanes(Lanes &lanes, int K);  // makes exactly K lanes; returns 1 when lanes were (re)made
+  Lanes lanes_;
+  Lanes shot_lanes_;  // of run_model on resident grids: a state and mailboxes each
+  int resident_shot_lanes(resident::Plan *plan) const;
+  mutable std::map<int, resident::Plan> shot_plans_;  // by lanes
   DeviceBuffer gff_shots_;
   cudaEvent_t lanes_start_ = nullptr;
   static constexpr int kMaxLanes = 8;       // run_model lanes
