@@ -52,6 +52,8 @@ def parse():
     p.add_argument("--ncu-case-exact", type=int, default=0, metavar="NT",
                    help="run one exact gradient of one NT-step shot of the c3 workload, launch by "
                         "launch, and exit (for ncu captures)")
+    p.add_argument("--ncu-variant", default=None, metavar="NAME",
+                   help="kernel variant of --ncu-case-exact (default: the model's own scheme)")
     p.add_argument("--ncu-case-c4judge", type=int, default=0, metavar="SHAPE",
                    help="run one batched forward of the c4 judge (128 members) with the tile "
                         "shape given by index (0 32x60, 1 16x28, 2 20x28, 3 16x60; one launch "
@@ -269,21 +271,25 @@ def fwi_gradients_c3(steps, with_cpu=False):
             res["device_bytes"] = m.exact_bytes(kw["checkpoint_every"])
         out[name] = res
     out["value"] = out["checkpoint_100"]["value"]
-    # Algorithmic bytes of one checkpointed gradient: per shot and step two
-    # forward steps (checkpoint pass, recompute; 52 B per cell each) and one
-    # exact step (98.4 B per cell: 18 words of fields and medium, three FP32
-    # partial sums read and written, three float-float pairs on one step in
-    # 20).
+    # Bytes of one checkpointed gradient, for the scheme that ran. A gradient
+    # resident on chip moves the kept rates: 20 B per cell, shot and step out
+    # and 20 back in (bound by the exchange of edges and FP32 issue, not by
+    # HBM). Per-step launches move, per shot and step, two forward steps
+    # (checkpoint pass, recompute; 52 B per cell each) and one exact step
+    # (98.4 B per cell: 18 words of fields and medium, three FP32 partial sums
+    # read and written, three float-float pairs on one step in 20).
     cells = float(m.nx * m.nz)
-    per_grad = m.n_shots * m.nt * cells * (2 * 52.0 + 98.4)
+    resident = "resident_steps" in m.profile_forward(0, 10)[1]
+    per_cell = 40.0 if resident else 2 * 52.0 + 98.4
+    per_grad = m.n_shots * m.nt * cells * per_cell
     peak, kind = measured_peaks()
     t = out["checkpoint_100"]["ms_per_gradient"] / 1e3
-    out["roofline"] = {"bound": "hbm", "bytes_per_gradient": per_grad,
+    out["roofline"] = {"bound": "edge exchange, fp32" if resident else "hbm",
+                       "scheme": "resident" if resident else "per-step launches",
+                       "bytes_per_cell_and_step": per_cell, "bytes_per_gradient": per_grad,
                        "achieved": per_grad / t / 1e9, "peak": peak, "unit": "GB/s",
                        "frac": per_grad / t / 1e9 / peak, "peak_source": kind,
-                       "note": "whole checkpointed gradient, all kernels; bytes of steps that "
-                               "stream every field (a gradient resident on chip moves "
-                               "40 bytes per cell and step instead of 202)"}
+                       "note": "whole checkpointed gradient, all kernels"}
     if with_cpu:
         out["cpu_baseline"] = cpu_baseline_c3()
     return out
@@ -387,7 +393,9 @@ def batched(steps, warmup, rank=0, world=1, with_cpu=False):
            "workload": "c2: 256 seeded models, nx_inner U[200,800], nz_inner U[100,400], "
                        "25-cell boundary, 1-4 shots, Ricker 20-50 Hz, nt=1000, forward only",
            "members": info["members"], "cells_per_step": cells, "tiles": info["tiles"],
-           "tile_shape": shape, "persistent": b.persistent}
+           "tile_shape": shape, "persistent": b.persistent,
+           "scheme": "resident" if b.cluster else
+           "persistent tiles" if b.persistent else "per-step tiles"}
     if world > 1:
         out["parallelism"] = "models round-robin over %d ranks, no collective on the data path" % world
         return out
@@ -487,10 +495,10 @@ def ncu_case_small(nt):
                                                       m.get_synthetic_data()[0].sum()))
 
 
-def ncu_case_exact(nt):
+def ncu_case_exact(nt, variant=None):
     """One exact gradient (checkpoints every 100 steps) of a one-shot, NT-step
     version of the c3 workload, kernels launched one by one (no graph), for
-    ncu captures."""
+    ncu captures: resident on chip, or by the launches of `variant`."""
     import psvwave_gb300 as psv
     from psvwave_gb300 import workloads
 
@@ -501,6 +509,8 @@ def ncu_case_exact(nt):
     m.set_observed_data(*m.get_synthetic_data())
     m.set_parameter_fields(*start)
     m.set_graph_capture(False)
+    if variant:
+        m.kernel_variant = variant
     mis, _ = m.exact_gradient(100)
     print("ncu exact case: %s tiles, misfit %.9e" % (m.tile_shape, mis))
 
@@ -554,7 +564,7 @@ def main():
         ncu_case(args.ncu_case)
         return
     if args.ncu_case_exact:
-        ncu_case_exact(args.ncu_case_exact)
+        ncu_case_exact(args.ncu_case_exact, args.ncu_variant)
         return
     if args.ncu_case_small:
         ncu_case_small(args.ncu_case_small)

@@ -71,6 +71,15 @@ struct OnDevice {
   ~OnDevice() { cudaSetDevice(prev); }
 };
 
+// Cluster sizes of a batch. The smallest that holds a member fills the device
+// best, and more SMs speed up a single one; the sizes left out are slower than
+// the one below them, fewer of their clusters being resident at once (16 CTAs: 7,
+// 12: 8, 10: 13, 9 and 8: 15, 4: 36). ms for 1000 steps of 64 members, clusters of
+// 4 | 5 | 6 | 7 | 8 | 9 | 10 | 11 | 12 | 13 to 15 | 16 CTAs: 150 x 120 points 6.0 |
+// 6.6 | 6.2 | 8.9 | 8.5 | 7.9 | 8.1 | 11.1 | 11.1 | 12.6 to 13.5 | 12.2; 250 x 150 (9
+// hold it) 13.5 | 13.0 | 16.1 | 15.8 | 16.9 to 18.7 | 16.9.
+constexpr int kClusterSizes[] = {4, 5, 6, 8, 9, 10, 12, 16};
+
 // A member's plan under a layout; no CTAs: it does not fit.
 resident::Plan member_plan(const resident::Grid &g, int nc, int per_sm) {
   if (nc > 0) {
@@ -95,7 +104,7 @@ bool Batch::cluster_fits() {
     // Fewest CTAs that hold every member: clusters, else mailbox teams.
     fits_ = 0;
     std::vector<Layout> tries;
-    for (int nc : {4, 5, 6, 8, 9, 10, 12, 16}) {
+    for (int nc : kClusterSizes) {
       bool all = true;
       if (grids_.empty())
         for (const auto &mb : members_) grids_.push_back(mb.first->resident_grid());
@@ -565,7 +574,7 @@ int Batch::autotune(int n_steps) {
     // (The smallest clusters that hold a member fill the device best, the
     // largest are the quickest each.)
     std::vector<Layout> tries;
-    for (int nc : {4, 5, 6, 8, 9, 10, 12, 16}) {
+    for (int nc : kClusterSizes) {
       if (!tries.empty() && nc < 16) continue;
       bool any = false;
       for (const auto &g : grids_) any = any || resident::plan_cluster(g, nc).ctas() > 0;

@@ -1,14 +1,17 @@
 // FP32 time stepping of grids held on chip for every time step of a launch
-// (psv_resident_f32.cu).
+// (psv_resident_core.cuh).
 //
-// A simulation runs on a team of CTAs, one per SM, each owning a tile of at
-// most 64 columns. Every thread keeps its points' wave fields and medium in
-// registers for all steps, and the tile's fields lie in shared memory for
-// the neighbours' stencils. After each half-step the tile's edges go to the
-// neighbouring CTAs through mailboxes in global memory (L2) whose 64-bit
-// words carry a value and the step's number, so that the receiver needs no
-// flag, fence or barrier. Global memory otherwise carries only the initial
-// and final state, receivers, snapshots, correlations and injection.
+// A simulation runs on a team of CTAs, each owning a tile. Every thread keeps
+// its points' wave fields and medium in registers for all steps, and the tile's
+// fields lie in shared memory for the neighbours' stencils. After each half-step
+// the tile's edges go to the neighbouring CTAs, by one of two links. A team of up
+// to 16 CTAs is one thread-block cluster (tiles of up to 152 columns) and writes
+// straight into its neighbours' shared memory, counted on their mbarriers. Any
+// other (tiles of up to 64 columns, one or two CTAs on an SM) goes through
+// mailboxes in global memory (L2), whose 128-bit words carry three values and the
+// step's number, so that the receiver needs no flag, fence or barrier. Global
+// memory otherwise carries only the initial and final state, receivers,
+// snapshots, correlations and injection.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -20,8 +23,8 @@
 namespace psv {
 namespace resident {
 
-// A grid to split: its size, and the cells (ix nz + iz) of its receivers
-// of each shot's injection points, and of its injection terms (a cell per term).
+// A grid to split: its size, and the cells (ix nz + iz) of its receivers, of
+// each shot's injection points, and of its injection terms (a cell per term).
 struct Grid {
   int nx = 0, nz = 0;
   std::vector<int> receivers;
@@ -44,9 +47,11 @@ struct Plan {
 // The split of a grid for one simulation at a time: the largest cluster that
 // holds it, else mailboxes over the whole device. These calls set launch
 // attributes as a side effect (call outside stream capture). Measured, one
-// simulation: 250 x 150 points in one 16-CTA cluster 1.8 us a step, by
-// mailboxes 2.6 to 3.6 us (32 to 152 CTAs); 1103 x 497 points 3.9 us by
-// mailboxes.
+// simulation, us a step: 250 x 150 points in one cluster of 16 CTAs 1.7, by
+// mailboxes 2.6 to 3.6 (32 to 152 CTAs); 1103 x 497 points 3.9 by mailboxes.
+// Clusters of 16 | 8 | 4 | 2 | 1 CTAs, forward: 24 x 20 points 1.03 | 1.04 | 1.06 |
+// 0.97 | 0.99, 40 x 40 0.96 | 1.06 | 0.98 | 1.09 | 1.31, 68 x 56 0.99 | 1.04 | 1.24 |
+// 1.58 | 2.06, 100 x 80 1.03 | 1.21 | 1.61 | 2.5 | -.
 Plan plan(const Grid &g);
 // A cluster of exactly nc CTAs.
 Plan plan_cluster(const Grid &g, int nc);

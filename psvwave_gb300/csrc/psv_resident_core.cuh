@@ -80,7 +80,11 @@ __host__ __device__ __forceinline__ int split(int k, int parts, int n) {
   return (int)(((long long)k * n) / parts);
 }
 __host__ __device__ __forceinline__ int pairs(int nz) { return (nz + 1) / 2; }
-// Shared row strides: column pairs of a tile at most (S - 4) / 2.
+// Shared row strides: column pairs of a tile at most (S - 4) / 2. Mailbox tiles
+// have a warp a group, 32 pairs. A cluster keeps its tiles one column wide as
+// long as it can (152 columns: 76 pairs, six groups of them in a block), for the
+// rows of a group then stay in one CTA: 250 x 150 points 1.72 us a step in 16 x 1
+// tiles, 1.90 in 8 x 2; 100 x 80 1.03 and 1.12.
 constexpr int kNarrow = 68, kWide = 156;
 
 // Mailbox word: three values and the tag, one 16-byte access. The x stencils
