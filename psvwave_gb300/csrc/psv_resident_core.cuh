@@ -384,6 +384,7 @@ __device__ __forceinline__ void member_steps(const tma::SimDesc &d, const Team &
       xz[k] = load(in.txz, x, z);
     }
     const float2 l = load(d.lm, x, z), m = load(d.mu, x, z), b = load(d.b, x, z);
+    if (!EX) lm[k] = make_float2(-0.f, -0.f);
     if (in_region(x, z)) {
       inside |= 1u << (2 * k);
       lm[k].x = l.x;
@@ -689,27 +690,13 @@ __device__ __forceinline__ void member_steps(const tma::SimDesc &d, const Team &
     return;
   }
 
-  // Row k's fields as they leave the launch: NaN of points outside the updated
-  // region back to zero.
-  auto leave = [&](int k) {
-    const int x = x0 + r0 + k;
-    auto clear = [](float &v) { v = isnan(v) ? 0.f : v; };
-    if (!in_region(x, z)) {
-      clear(vx[k].x);
-      clear(vz[k].x);
-      clear(xx[k].x);
-      clear(zz[k].x);
-      clear(xz[k].x);
-    }
-    if (!in_region(x, z + 1)) {
-      clear(vx[k].y);
-      clear(vz[k].y);
-      clear(xx[k].y);
-      clear(zz[k].y);
-      clear(xz[k].y);
-    }
+  // A value at row k, column e as it leaves the launch: NaN of points outside
+  // the updated region (whose lm is -0) back to zero.
+  auto leave = [&](float v, int k, int e) {
+    return isnan(v) && __float_as_int(e ? lm[k].y : lm[k].x) < 0 ? 0.f : v;
   };
-  // kExact: the same for a pair of gradient sums.
+  auto leave2 = [&](float2 v, int k) { return make_float2(leave(v.x, k, 0), leave(v.y, k, 1)); };
+  // kExact: the same for gradient sums.
   auto leaves = [&](float2 v, int k) {
     const int x = x0 + r0 + k;
     if (isnan(v.x) && !in_region(x, z)) v.x = 0.f;
@@ -721,20 +708,19 @@ __device__ __forceinline__ void member_steps(const tma::SimDesc &d, const Team &
 #pragma unroll
     for (int k = 0; k < K; ++k) {
       if (k >= kn) continue;
-      leave(k);
       float *q = base + (size_t)(x0 + r0 + k) * ps + z;
       if (z + 1 < nz) {
-        sts2(q, vx[k]);
-        sts2(q + gp, vz[k]);
-        sts2(q + 2 * gp, xx[k]);
-        sts2(q + 3 * gp, zz[k]);
-        sts2(q + 4 * gp, xz[k]);
+        sts2(q, leave2(vx[k], k));
+        sts2(q + gp, leave2(vz[k], k));
+        sts2(q + 2 * gp, leave2(xx[k], k));
+        sts2(q + 3 * gp, leave2(zz[k], k));
+        sts2(q + 4 * gp, leave2(xz[k], k));
       } else {
-        q[0] = vx[k].x;
-        q[gp] = vz[k].x;
-        q[2 * gp] = xx[k].x;
-        q[3 * gp] = zz[k].x;
-        q[4 * gp] = xz[k].x;
+        q[0] = leave(vx[k].x, k, 0);
+        q[gp] = leave(vz[k].x, k, 0);
+        q[2 * gp] = leave(xx[k].x, k, 0);
+        q[3 * gp] = leave(zz[k].x, k, 0);
+        q[4 * gp] = leave(xz[k].x, k, 0);
       }
     }
   };
@@ -852,7 +838,6 @@ __device__ __forceinline__ void member_steps(const tma::SimDesc &d, const Team &
 #pragma unroll
       for (int k = 0; k < K; ++k) {
         if (k >= kn) continue;
-        if (!ADJ) leave(k);
         const int x = x0 + r0 + k;
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
@@ -863,11 +848,11 @@ __device__ __forceinline__ void member_steps(const tma::SimDesc &d, const Team &
                       sx = e ? xx[k].y : xx[k].x, sz = e ? zz[k].y : zz[k].x,
                       sh = e ? xz[k].y : xz[k].x;
           if (!ADJ) {
-            d.accu[0][soff + gi] = a;
-            d.accu[1][soff + gi] = b;
-            d.accu[2][soff + gi] = sx;
-            d.accu[3][soff + gi] = sz;
-            d.accu[4][soff + gi] = sh;
+            d.accu[0][soff + gi] = leave(a, k, e);
+            d.accu[1][soff + gi] = leave(b, k, e);
+            d.accu[2][soff + gi] = leave(sx, k, e);
+            d.accu[3][soff + gi] = leave(sz, k, e);
+            d.accu[4][soff + gi] = leave(sh, k, e);
           } else if (x >= d.fx0 && x < d.fx1 && iz >= d.fz0 && iz < d.fz1) {
             const float *as[5] = {d.accu[0] + soff, d.accu[1] + soff, d.accu[2] + soff,
                                   d.accu[3] + soff, d.accu[4] + soff};
@@ -1070,13 +1055,12 @@ __device__ __forceinline__ void member_steps(const tma::SimDesc &d, const Team &
 #pragma unroll
     for (int k = 0; k < K; ++k) {
       if (k >= kn) continue;
-      if (!EX) leave(k);
       const size_t o = (size_t)(x0 + r0 + k) * ps + z;
       const float2 v[5] = {vx[k], vz[k], xx[k], zz[k], xz[k]};
 #pragma unroll
       for (int f = 0; f < 5; ++f) {
-        dst[f][o] = v[f].x;
-        if (z + 1 < nz) dst[f][o + 1] = v[f].y;
+        dst[f][o] = EX ? v[f].x : leave(v[f].x, k, 0);
+        if (z + 1 < nz) dst[f][o + 1] = EX ? v[f].y : leave(v[f].y, k, 1);
       }
       if (EX)
         for (int p = 0; p < 3; ++p)
