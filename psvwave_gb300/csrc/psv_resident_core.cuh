@@ -693,7 +693,7 @@ __device__ __forceinline__ void member_steps(const tma::SimDesc &d, const Team &
   // A value at row k, column e as it leaves the launch: NaN of points outside
   // the updated region (whose lm is -0) back to zero.
   auto leave = [&](float v, int k, int e) {
-    return isnan(v) && __float_as_int(e ? lm[k].y : lm[k].x) < 0 ? 0.f : v;
+    return isnan(v) && __float_as_uint(e ? lm[k].y : lm[k].x) == 0x80000000u ? 0.f : v;
   };
   auto leave2 = [&](float2 v, int k) { return make_float2(leave(v.x, k, 0), leave(v.y, k, 1)); };
   // kExact: the same for gradient sums.

@@ -313,3 +313,19 @@ def test_points_outside_the_updated_region_stay_out_of_a_diverging_run(nx, nz):
         g = m.exact_gradient(50)[1]
         assert all(not np.isfinite(f).all() for f in g)
         assert all(not rim(f).any() for f in g)
+
+
+def test_a_medium_of_negative_density_keeps_its_nan():
+    # (Its lm is negative inside the updated region, where nothing is put back.)
+    out = []
+    for variant in (None, "fused_tma"):
+        m = model(68, 57, [(20, 20)], [(24, 24)])
+        if variant:
+            m.kernel_variant = variant
+        one = np.ones((m.nx, m.nz))
+        m.set_parameter_fields(2e5 * one, 8e4 * one, -1500.0 * one)
+        m.forward_simulate(0, False)
+        out.append(m.get_wavefields())
+    for a, b in zip(*out):
+        assert np.isnan(b[2:-2, 2:-2]).any()
+        assert np.isnan(a[2:-2, 2:-2]).sum() >= 0.9 * np.isnan(b[2:-2, 2:-2]).sum()
