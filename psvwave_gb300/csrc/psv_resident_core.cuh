@@ -384,7 +384,6 @@ __device__ __forceinline__ void member_steps(const tma::SimDesc &d, const Team &
       xz[k] = load(in.txz, x, z);
     }
     const float2 l = load(d.lm, x, z), m = load(d.mu, x, z), b = load(d.b, x, z);
-    if (!EX) lm[k] = make_float2(-0.f, -0.f);
     if (in_region(x, z)) {
       inside |= 1u << (2 * k);
       lm[k].x = l.x;
@@ -691,18 +690,14 @@ __device__ __forceinline__ void member_steps(const tma::SimDesc &d, const Team &
   }
 
   // A value at row k, column e as it leaves the launch: NaN of points outside
-  // the updated region (whose lm is -0) back to zero.
+  // the updated region back to zero. (b = 0 tells them, which no finite density
+  // has; a test by position in the loop of steps cost the tallest tiles of a batch
+  // registers, a mark in lm's sign the forward steps.)
   auto leave = [&](float v, int k, int e) {
-    return isnan(v) && __float_as_uint(e ? lm[k].y : lm[k].x) == 0x80000000u ? 0.f : v;
+    if (EX) return isnan(v) && !in_region(x0 + r0 + k, z + e) ? 0.f : v;
+    return isnan(v) && (e ? bb[k].y : bb[k].x) == 0.f ? 0.f : v;
   };
   auto leave2 = [&](float2 v, int k) { return make_float2(leave(v.x, k, 0), leave(v.y, k, 1)); };
-  // kExact: the same for gradient sums.
-  auto leaves = [&](float2 v, int k) {
-    const int x = x0 + r0 + k;
-    if (isnan(v.x) && !in_region(x, z)) v.x = 0.f;
-    if (isnan(v.y) && !in_region(x, z + 1)) v.y = 0.f;
-    return v;
-  };
   auto save = [&](float *base) {
     const size_t gp = (size_t)nx * ps;
 #pragma unroll
@@ -1039,7 +1034,7 @@ __device__ __forceinline__ void member_steps(const tma::SimDesc &d, const Team &
 #pragma unroll 1
         for (int k = 0; k < kn; ++k, to += ps, sum += 4 * (S - 4))
           for (int p = 0; p < 3; ++p) {
-            sts2(to + (size_t)p * nx * ps, leaves(lds2(sum + p * (S - 4)), k));
+            sts2(to + (size_t)p * nx * ps, leave2(lds2(sum + p * (S - 4)), k));
             sts2(sum + p * (S - 4), zero2);
           }
       }
@@ -1065,7 +1060,7 @@ __device__ __forceinline__ void member_steps(const tma::SimDesc &d, const Team &
       if (EX)
         for (int p = 0; p < 3; ++p)
           *reinterpret_cast<float2 *>(io.part + (size_t)p * nx * ps + o) =
-              leaves(lds2(G + ((r0 + k) * 4 + p) * (S - 4) + 2 * c), k);
+              leave2(lds2(G + ((r0 + k) * 4 + p) * (S - 4) + 2 * c), k);
     }
   }
   if (CLUSTER) cg::this_cluster().sync();
