@@ -1453,9 +1453,10 @@ bool Model::run_model_lanes_ok() const {
 // 10.7 | 11.3; 600 x 350 17.3 | 13.6 | 15.2; 700 x 400 21.4 | 18.3 | 16.9. Above
 // about 290 k points two lanes do not fit: 800 x 400 24.0 | 21.0 | 24.0, 900 x 450
 // 24.2 | 27.6 | 24.2. (Per-step launches give other bits than forward_simulate and
-// adjoint_simulate do on these grids, and larger rounding errors.) Up to three
-// shots one after another are as quick as per-step lanes were, and keep the
-// serial order of the kernels' FP64 sums.
+// adjoint_simulate do on these grids, with errors against 64 bits of 0.7 to 2.5
+// times these, over two surveys and three sizes.) Up to three shots one after
+// another are as quick as per-step lanes were, and keep the serial order of the
+// kernels' FP64 sums.
 int Model::resident_shot_lanes(resident::Plan *plan) const {
   *plan = resident::Plan();
   const int shots = cfg_.n_shots;
