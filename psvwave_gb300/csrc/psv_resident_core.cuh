@@ -210,7 +210,8 @@ __device__ __forceinline__ float2 mul2(float2 a, float2 b) {
   return make_float2(__fmul_rn(a.x, b.x), __fmul_rn(a.y, b.y));
 }
 
-template <int MODE, int K, int S, bool CLUSTER>
+// (BATCH: the final state is nobody's output.)
+template <int MODE, int K, int S, bool CLUSTER, bool BATCH = false>
 __device__ __forceinline__ void member_steps(const tma::SimDesc &d, const Team &tm, int it0,
                                              int n_steps, int parity, bool zero, int store,
                                              const Dump &dump, const RateIo &io, int *err) {
@@ -689,33 +690,50 @@ __device__ __forceinline__ void member_steps(const tma::SimDesc &d, const Team &
     return;
   }
 
-  // A value at row k, column e as it leaves the launch: NaN of points outside
-  // the updated region back to zero. (b = 0 tells them, which no finite density
-  // has; a test by position in the loop of steps cost the tallest tiles of a batch
-  // registers, a mark in lm's sign the forward steps.)
-  auto leave = [&](float v, int k, int e) {
-    if (EX) return isnan(v) && !in_region(x0 + r0 + k, z + e) ? 0.f : v;
-    return isnan(v) && (e ? bb[k].y : bb[k].x) == 0.f ? 0.f : v;
+  // Before a thread's fields leave the launch: NaN of points outside the updated
+  // region (b = 0 tells them, which no finite density has) back to zero. Threads
+  // without such points pass by.
+  auto put_back = [&] {
+    if (x0 + r0 >= 2 && x0 + r0 + kn <= nx - 2 && z >= 2 && z + 2 <= nz - 2) return;
+    auto clear = [](float2 &v, float2 b) {
+      if (isnan(v.x) && b.x == 0.f) v.x = 0.f;
+      if (isnan(v.y) && b.y == 0.f) v.y = 0.f;
+    };
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      clear(vx[k], bb[k]);
+      clear(vz[k], bb[k]);
+      clear(xx[k], bb[k]);
+      clear(zz[k], bb[k]);
+      clear(xz[k], bb[k]);
+    }
   };
-  auto leave2 = [&](float2 v, int k) { return make_float2(leave(v.x, k, 0), leave(v.y, k, 1)); };
+  // kExact: the same for gradient sums of row k.
+  auto sums_back = [&](float2 v, int k) {
+    const int x = x0 + r0 + k;
+    if (isnan(v.x) && !in_region(x, z)) v.x = 0.f;
+    if (isnan(v.y) && !in_region(x, z + 1)) v.y = 0.f;
+    return v;
+  };
   auto save = [&](float *base) {
     const size_t gp = (size_t)nx * ps;
+    put_back();
 #pragma unroll
     for (int k = 0; k < K; ++k) {
       if (k >= kn) continue;
       float *q = base + (size_t)(x0 + r0 + k) * ps + z;
       if (z + 1 < nz) {
-        sts2(q, leave2(vx[k], k));
-        sts2(q + gp, leave2(vz[k], k));
-        sts2(q + 2 * gp, leave2(xx[k], k));
-        sts2(q + 3 * gp, leave2(zz[k], k));
-        sts2(q + 4 * gp, leave2(xz[k], k));
+        sts2(q, vx[k]);
+        sts2(q + gp, vz[k]);
+        sts2(q + 2 * gp, xx[k]);
+        sts2(q + 3 * gp, zz[k]);
+        sts2(q + 4 * gp, xz[k]);
       } else {
-        q[0] = leave(vx[k].x, k, 0);
-        q[gp] = leave(vz[k].x, k, 0);
-        q[2 * gp] = leave(xx[k].x, k, 0);
-        q[3 * gp] = leave(zz[k].x, k, 0);
-        q[4 * gp] = leave(xz[k].x, k, 0);
+        q[0] = vx[k].x;
+        q[gp] = vz[k].x;
+        q[2 * gp] = xx[k].x;
+        q[3 * gp] = zz[k].x;
+        q[4 * gp] = xz[k].x;
       }
     }
   };
@@ -830,6 +848,7 @@ __device__ __forceinline__ void member_steps(const tma::SimDesc &d, const Team &
     }
     if (snap && mine) {
       const size_t soff = (size_t)(it / d.si) * nx * nz;
+      if (!ADJ) put_back();
 #pragma unroll
       for (int k = 0; k < K; ++k) {
         if (k >= kn) continue;
@@ -843,11 +862,11 @@ __device__ __forceinline__ void member_steps(const tma::SimDesc &d, const Team &
                       sx = e ? xx[k].y : xx[k].x, sz = e ? zz[k].y : zz[k].x,
                       sh = e ? xz[k].y : xz[k].x;
           if (!ADJ) {
-            d.accu[0][soff + gi] = leave(a, k, e);
-            d.accu[1][soff + gi] = leave(b, k, e);
-            d.accu[2][soff + gi] = leave(sx, k, e);
-            d.accu[3][soff + gi] = leave(sz, k, e);
-            d.accu[4][soff + gi] = leave(sh, k, e);
+            d.accu[0][soff + gi] = a;
+            d.accu[1][soff + gi] = b;
+            d.accu[2][soff + gi] = sx;
+            d.accu[3][soff + gi] = sz;
+            d.accu[4][soff + gi] = sh;
           } else if (x >= d.fx0 && x < d.fx1 && iz >= d.fz0 && iz < d.fz1) {
             const float *as[5] = {d.accu[0] + soff, d.accu[1] + soff, d.accu[2] + soff,
                                   d.accu[3] + soff, d.accu[4] + soff};
@@ -1034,7 +1053,7 @@ __device__ __forceinline__ void member_steps(const tma::SimDesc &d, const Team &
 #pragma unroll 1
         for (int k = 0; k < kn; ++k, to += ps, sum += 4 * (S - 4))
           for (int p = 0; p < 3; ++p) {
-            sts2(to + (size_t)p * nx * ps, leave2(lds2(sum + p * (S - 4)), k));
+            sts2(to + (size_t)p * nx * ps, sums_back(lds2(sum + p * (S - 4)), k));
             sts2(sum + p * (S - 4), zero2);
           }
       }
@@ -1046,6 +1065,7 @@ __device__ __forceinline__ void member_steps(const tma::SimDesc &d, const Team &
 
   if (mine) {
     const fast::Fields out = d.set[parity ^ (n_steps & 1)];
+    if (!EX && !BATCH) put_back();
     float *const dst[5] = {out.vx, out.vz, out.txx, out.tzz, out.txz};
 #pragma unroll
     for (int k = 0; k < K; ++k) {
@@ -1054,13 +1074,13 @@ __device__ __forceinline__ void member_steps(const tma::SimDesc &d, const Team &
       const float2 v[5] = {vx[k], vz[k], xx[k], zz[k], xz[k]};
 #pragma unroll
       for (int f = 0; f < 5; ++f) {
-        dst[f][o] = EX ? v[f].x : leave(v[f].x, k, 0);
-        if (z + 1 < nz) dst[f][o + 1] = EX ? v[f].y : leave(v[f].y, k, 1);
+        dst[f][o] = v[f].x;
+        if (z + 1 < nz) dst[f][o + 1] = v[f].y;
       }
       if (EX)
         for (int p = 0; p < 3; ++p)
           *reinterpret_cast<float2 *>(io.part + (size_t)p * nx * ps + o) =
-              leave2(lds2(G + ((r0 + k) * 4 + p) * (S - 4) + 2 * c), k);
+              sums_back(lds2(G + ((r0 + k) * 4 + p) * (S - 4) + 2 * c), k);
     }
   }
   if (CLUSTER) cg::this_cluster().sync();

@@ -26,8 +26,8 @@ __global__ void __launch_bounds__(kMaxThreads, 1)
   const Member m = members[cta_member[blockIdx.x]];
   const Team t{(int)blockIdx.x - m.first, m.tiles_x, m.tiles_z, m.groups, m.n_rec, m.n_inj,
                0, m.n_term, mail + (size_t)m.first * kBox};
-  member_steps<kForward, K, S, CLUSTER>(sims[m.sim], t, 0, n_steps, 0, true, store, Dump(),
-                                        RateIo(), err);
+  member_steps<kForward, K, S, CLUSTER, true>(sims[m.sim], t, 0, n_steps, 0, true, store, Dump(),
+                                              RateIo(), err);
 }
 
 size_t smem_bytes(int Rm, int S, int nr, int n_points, int n_terms) {

@@ -329,3 +329,18 @@ def test_a_medium_of_negative_density_keeps_its_nan():
     for a, b in zip(*out):
         assert np.isnan(b[2:-2, 2:-2]).any()
         assert np.isnan(a[2:-2, 2:-2]).sum() >= 0.9 * np.isnan(b[2:-2, 2:-2]).sum()
+
+
+def test_snapshots_of_a_diverging_batch_keep_their_rim():
+    ms = [model(nx, nz, [(20, 20)], [(24, 24)], dt=2.5e-3) for nx, nz in ((68, 57), (250, 151))]
+    b = psv.Batch()
+    for m in ms:
+        b.add(m, 0)
+    b.cluster = True
+    b.forward(True)
+    for m in ms:
+        for f in m.get_snapshots():
+            f = np.array(f)
+            assert not np.isfinite(f).all()
+            f[..., 2:-2, 2:-2] = 0.0
+            assert not f.any()
